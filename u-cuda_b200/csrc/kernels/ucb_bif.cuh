@@ -237,10 +237,8 @@ extern "C" __global__ void UCB_LAUNCH_BOUNDS ucb_bif_kernel(const UcbBifParams p
 // recorded series, the peaks, the intervals and a helper array per cell in HBM and runs
 // three kernels. Here a warp integrates its 32 cells (one per lane) with the peaks
 // streaming into the warp's own scratch slot (one contiguous row of `cap` peaks per
-// lane), then runs the dbscan of each of the 32 cells in turn with all 32 lanes: the
-// dbscan's control flow (seeds, stack pops) is the same for the whole warp and each scan
-// over the peaks is split across the lanes, so no lane waits on another cell's pops.
-// Scratch is per resident warp, not per cell.
+// lane), then finds their periods (ucb_dbscan1d.cuh). Scratch is per resident warp, not per
+// cell.
 struct UcbBif2dParams {
     long long total;           // cells
     int n_pts;
@@ -256,8 +254,8 @@ struct UcbBif2dParams {
     numb vals[UCB_NV];
     const numb* axis0;
     const numb* axis1;
-    numb* peaks;               // per warp slot: 32 x cap
-    int* work;                 // per warp slot: cap labels + cap stack slots
+    char* rows;                // per warp slot: 32 rows of cap 8-byte entries
+    char* work;                // per warp slot: bif2d_work_bytes(cap)
     double* out_values;        // period (-1 where the dbscan result is negative)
     int* out_flags;            // -1 / 1
     unsigned long long* counter;
@@ -274,64 +272,49 @@ struct Bif2dSink {
     }
 };
 
-// The reference's dbscan step for step, one warp per cell: labels (helpful[0, P)) and the
-// stack slots (helpful[P, 2P)) as integers — they only ever hold cluster numbers and
-// indices below 2,500, exact in numb — with the slots written at P + k and popped at
-// P + NumNeibor - 1, inner bound P - 1, result cluster - 1. Peaks enter times mult_peak (1)
-// and intervals times mult_interval (0) (configCUDA.h), so the distance is that of the
-// peak values. Within one scan each k touches only its own label and slot and NumNeibor
-// only counts, so the lanes take k = lane, lane + 32, ... and the hits are summed with a
-// ballot.
-__device__ __forceinline__ int dbscan_warp(const numb* peaks, int P, int* lab, int* stk, numb eps, int lane) {
-    if (P == -1) return -1;
-    if (P == 0) return 0;
-    if (P == 1) return 1;
-    for (int k = lane; k < P; k += 32) {
-        lab[k] = 0;
-        stk[k] = 0;
-    }
-    __syncwarp();
-    int cluster = 0, nn = 0;
-    for (unsigned long long i = 0; i < (unsigned long long)P; i++) {
-        if (nn >= 1) {
-            const int v = stk[nn - 1];
-            __syncwarp();
-            if (lane == 0) stk[nn - 1] = 0;
-            i = (unsigned long long)v;
-            nn = nn - 1;
-        } else if (lab[i] == 0) {
-            nn = 0;
-            ++cluster;
-            __syncwarp();
-            if (lane == 0) lab[i] = cluster;
-        } else {
-            continue;
+// Scratch of one warp besides its 32 peak rows (the host sizes it by the same rule): the
+// sort's two key and two index buffers of one cell, then the bit sets of the 32 replays,
+// interleaved by lane.
+__device__ __forceinline__ long long bif2d_sort_bytes(int cap) { return ((long long)cap * 20 + 127) & ~127LL; }
+__device__ __forceinline__ long long bif2d_work_bytes(int cap) {
+    return bif2d_sort_bytes(cap) + (long long)((cap + 31) / 32) * 3 * 32 * 4;
+}
+
+// Periods of a warp's 32 cells from their peak rows: the rows are sorted one after the other
+// by the whole warp, each giving way to its cell's ranges and order (6 bytes a peak in rows
+// of 8), then every lane replays its own cell's dbscan.
+__device__ __noinline__ int bif2d_periods(char* rows, char* work, int cap, int count, numb eps, int lane) {
+    PeakKey* keys = reinterpret_cast<PeakKey*>(work);
+    unsigned short* idx = reinterpret_cast<unsigned short*>(work + (long long)cap * 16);
+    for (int c = 0; c < 32; ++c) {
+        const int P = __shfl_sync(0xFFFFFFFFu, count, c);
+        if (P < 2) continue;
+        char* row = rows + (long long)c * cap * 8;
+        PeakKey *ka = keys, *kb = keys + cap;
+        unsigned short *ia = idx, *ib = idx + cap;
+        for (int e = lane; e < P; e += 32) {
+            ka[e] = peak_key(reinterpret_cast<const numb*>(row)[e]);
+            ia[e] = (unsigned short)e;
         }
         __syncwarp();
-        const numb xi = peaks[i];
-        int hits = 0;
-        // chunks of 32 are independent (each k touches only its own label and slot): both
-        // loads of a lane are issued unconditionally and four chunks are in flight at once
-#pragma unroll 4
-        for (int k0 = 0; k0 < P - 1; k0 += 32) {
-            const int k = k0 + lane;
-            const bool in = k < P - 1;
-            const int lk = in ? lab[k] : 1;
-            const numb pk = in ? peaks[k] : xi;
-            // the reference's distance sqrt(dx * dx + 0 * 0) = sqrt(fl(dx * dx)) is exactly
-            // |dx| in binary floating point (correctly rounded product and square root; an
-            // overflowing or underflowing dx * dx still compares the same against eps)
-            const bool hit = in && i != (unsigned long long)k && lk == 0 && fabs(pk - xi) < eps;
-            if (hit) {
-                lab[k] = cluster;
-                stk[k] = k;
-            }
-            hits += __popc(__ballot_sync(0xFFFFFFFFu, hit));
+        for (int run = 1; run < P; run *= 2) {
+            merge_level(ka, ia, kb, ib, P, run, lane);
+            __syncwarp();
+            PeakKey* tk = ka;
+            ka = kb;
+            kb = tk;
+            unsigned short* ti = ia;
+            ia = ib;
+            ib = ti;
         }
-        nn += hits;
+        peak_ranges(ka, ia, P, eps, reinterpret_cast<unsigned int*>(row),
+                    reinterpret_cast<unsigned short*>(row + (long long)cap * 4), lane);
         __syncwarp();
     }
-    return cluster - 1;
+    const char* row = rows + (long long)lane * cap * 8;
+    return dbscan_replay(count, reinterpret_cast<const unsigned int*>(row),
+                         reinterpret_cast<const unsigned short*>(row + (long long)cap * 4),
+                         reinterpret_cast<unsigned int*>(work + bif2d_sort_bytes(cap)) + lane, 32);
 }
 
 // Trajectory and peaks of one cell of a 2-D period map: the peak count (or the -1 / 0
@@ -387,23 +370,17 @@ __device__ __forceinline__ int bif2d_peaks(const UcbBif2dParams& p, long long ki
 extern "C" __global__ void UCB_LAUNCH_BOUNDS ucb_bif2d_kernel(const UcbBif2dParams p) {
     const int lane = threadIdx.x & 31;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    numb* slot = p.peaks + warp * 32 * (long long)p.cap;
-    int* lab = p.work + warp * 2 * (long long)p.cap;
-    int* stk = lab + p.cap;
+    char* rows = p.rows + warp * 32 * (long long)p.cap * 8;
+    char* work = p.work + warp * ucbdev::bif2d_work_bytes(p.cap);
     long long ns = 0;
     for (;;) {
         const long long base = ucbdev::warp_fetch(p.counter, lane);
         if (base >= p.total) break;
         const long long i = base + lane;
-        const int count = i < p.total ? ucbdev::bif2d_peaks(p, i, slot + (long long)lane * p.cap, ns) : 0;
+        numb* row = reinterpret_cast<numb*>(rows + (long long)lane * p.cap * 8);
+        const int count = i < p.total ? ucbdev::bif2d_peaks(p, i, row, ns) : 0;
         __syncwarp();
-        int mine = 0;
-        for (int c = 0; c < 32; ++c) {
-            if (base + c >= p.total) break;
-            const int P = __shfl_sync(0xFFFFFFFFu, count, c);
-            const int period = ucbdev::dbscan_warp(slot + (long long)c * p.cap, P, lab, stk, p.eps, lane);
-            if (lane == c) mine = period;
-        }
+        const int mine = ucbdev::bif2d_periods(rows, work, p.cap, count, p.eps, lane);
         if (i < p.total) {
             long long out = i;
             if (p.swap_xy) out = (i % p.n_pts) * p.n_pts + i / p.n_pts;

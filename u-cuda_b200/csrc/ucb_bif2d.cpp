@@ -94,7 +94,7 @@ CompileRequest bif2d_compile_request(const ucb_bif2d_request& q, const SweepMap&
     std::vector<std::string> defs = clock_defines(sys);
     defs.push_back("UCB_BIF2D 1");
     rq.source = make_prelude(q.opt.precision, q.amount_of_x, q.n_values, m, true, sys, defs) +
-                "#include \"ucb_device.cuh\"\n#include \"ucb_bif.cuh\"\n";
+                "#include \"ucb_device.cuh\"\n#include \"ucb_dbscan1d.cuh\"\n#include \"ucb_bif.cuh\"\n";
     rq.headers = device_headers();
     rq.options.push_back(sys.exact ? "--fmad=false" : "--fmad=true");
     rq.kernels = {"ucb_bif2d_kernel"};
@@ -163,17 +163,20 @@ extern "C" int ucb_run_bif2d(ucb_engine* e, const ucb_bif2d_request* req, ucb_bi
     const long long total = (long long)n * n;
     // A peak needs a rise and a fall: at most one per two recorded samples.
     const int cap = (int)std::min<long long>(kMaxAmountOfPeaks, pointsInBlock / 2 + 2);
-    // Scratch per resident warp: 32 rows of peaks + dbscan labels and stack slots. The
-    // persistent grid is trimmed if the slots would exceed 40 % of the free memory.
+    // Scratch per resident warp: 32 rows of peaks, and the sort buffers and bit sets of the
+    // period count (bif2d_work_bytes of ucb_bif.cuh). The persistent grid is trimmed if the
+    // slots would exceed 40 % of the free memory.
     const int block = shape.block, warps_per_block = block / 32;
-    const size_t per_warp = (size_t)cap * (32 * esz + 2 * sizeof(int32_t));
+    const size_t row_bytes = (size_t)32 * cap * 8;
+    const size_t warp_work = (((size_t)cap * 20 + 127) & ~(size_t)127) + (size_t)((cap + 31) / 32) * 3 * 32 * 4;
+    const size_t per_warp = row_bytes + warp_work;
     int grid = persistent_grid(e, fn, block, total);
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
     const size_t budget = std::max<size_t>((size_t)(0.4 * (double)free_b), (size_t)64 << 20);
     grid = (int)std::max<long long>(1, std::min<long long>(grid, (long long)(budget / (per_warp * warps_per_block))));
-    const size_t slot_bytes = (size_t)grid * warps_per_block * 32 * cap * esz;
-    const size_t work_bytes = (size_t)grid * warps_per_block * 2 * cap * sizeof(int32_t);
+    const size_t slot_bytes = (size_t)grid * warps_per_block * row_bytes;
+    const size_t work_bytes = (size_t)grid * warps_per_block * warp_work;
 
     std::vector<double> t0d, t1d;
     std::vector<float> t0f, t1f;
