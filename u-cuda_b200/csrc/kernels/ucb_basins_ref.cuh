@@ -108,14 +108,13 @@ __device__ __forceinline__ void basins_ref_cell(const UcbBasinsRefParams& p, lon
     sums.sp = sums.sp2 = sums.si = sums.si2 = 0;
     PeakScan scan;
     scan.init();
-    scan.d1 = scan.d2 = 0;
     if (flag == 1 || flag == -1) flag = loop_record(st, x, a, p.h, p.points, p.pre_scaller, p.writable_var, p.maxv,
                                                      scan, sums, ns);
     if (flag == 0) {
         f1 = 999;
         f2 = 999;
     } else if (flag == -1) {
-        f1 = scan.d2;  // the last recorded sample
+        f1 = scan.last;  // the last recorded sample
         f2 = (numb)-1.0;
     } else {
         int n = (scan.found > 1) ? scan.found - 1 : 0;

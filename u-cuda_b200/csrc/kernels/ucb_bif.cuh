@@ -31,15 +31,17 @@ struct UcbBifParams {
 
 namespace ucbdev {
 
-// Streaming peakFinder. Position p is decided when sample p+1 arrives, as in the
-// reference loop that looks one sample ahead; positions p >= n-2 are never candidates.
+// State of the streaming peakFinder between chunks of samples. A position is decided once
+// the sample after it is there, as in the reference loop that looks one sample ahead;
+// positions >= n-2 are never candidates.
 struct PeakScan {
-    numb d0, d1, d2;           // samples p-1, p, p+1
+    numb last;                 // the last sample
     long long next_i;          // first index allowed as a new candidate (outer loop i)
     bool plateau;              // inside the inner loop (j) of a candidate
     int found;                 // peaks found so far (before dropping the first)
     numb prev_t;               // raw time of the previous peak
     __device__ __forceinline__ void init() {
+        last = 0;
         next_i = 2;
         plateau = false;
         found = 0;
@@ -81,46 +83,88 @@ struct Bif1dSink {
     }
 };
 
-// Emits a peak at position j with the reference's interpolation.
+// Emits a peak at position j (samples d0, d1, d2 at j - 1, j, j + 1) with the reference's
+// interpolation.
 template <class Sink>
-__device__ __forceinline__ void emit_peak(PeakScan& s, long long j, const Sink& sink) {
-    numb denom = s.d0 - (numb)2.0 * s.d1 + s.d2;
+__device__ __forceinline__ void emit_peak(PeakScan& s, long long j, numb d0, numb d1, numb d2, const Sink& sink) {
+    numb denom = d0 - (numb)2.0 * d1 + d2;
     numb delta = 0.0;
-    if (fabs(denom) > 1e-12) delta = 0.5 * (s.d0 - s.d2) / denom;
-    const numb value = s.d1 - 0.25 * (s.d0 - s.d2) * delta;
+    if (fabs(denom) > 1e-12) delta = 0.5 * (d0 - d2) / denom;
+    const numb value = d1 - 0.25 * (d0 - d2) * delta;
     const numb t = (numb)(j - 1) + delta;
     if (s.found > 0) sink.put(s.found - 1, value, t - s.prev_t);
     s.prev_t = t;
     s.found += 1;
 }
 
-// Feeds sample index q (value v). Decides position q-1.
+// Samples are searched for peaks a chunk at a time. Searched one by one inside the step
+// loop, every sample waited for the finder's comparisons and branches, and whenever one of
+// the warp's 32 lanes had a peak all of them waited for its division (about every second
+// sample of a chaotic map). Collected first (one local-memory store a sample), a chunk's
+// comparisons are independent of each other and give a bit mask of candidates, and the lanes
+// work through their few peaks of the chunk together. A divisor of kCheckInterval.
+// B200, native FP64: Lorenz diagram of 1,024 values 6.12 -> 3.60 ms, period map 256^2
+// 17.7 -> 14.7 ms; Duffing features 256^2 (FP32) 75.0 -> 73.1 ms.
+constexpr int kScanChunk = 20;
+// Samples in flight in the comparison loop. A diagram runs about one warp per scheduler, so it
+// takes the whole chunk at once (113 registers; 3.6 against 4.3 ms with 5); the maps keep
+// their resident warps (256^2 period map: 64 against 120 registers, 14.7 against 15.1 ms).
+#if defined(UCB_BIF2D) || defined(UCB_BIF_NO_KERNELS)
+#define UCB_SCAN_UNROLL 5
+#else
+#define UCB_SCAN_UNROLL 20
+#endif
+
+// Decides the positions q0 - 1 .. q0 + m - 2 of a series of n samples, w[2 .. m + 1] holding
+// the samples q0 .. q0 + m - 1 and w[0], w[1] the two before them.
 template <class Sink>
-__device__ __forceinline__ void scan_push(PeakScan& s, long long q, numb v, long long n, const Sink& sink) {
-    s.d0 = s.d1;
-    s.d1 = s.d2;
-    s.d2 = v;
-    const long long pos = q - 1;  // window is (pos-1, pos, pos+1)
-    if (q < 3 || pos > n - 3) return;
-    if (s.plateau) {
-        if (s.d1 < s.d2) {
-            s.plateau = false;
-            s.next_i = pos + 2;
-        } else if (s.d1 - s.d2 > (numb)kEpsPeakDelta) {
-            emit_peak(s, pos, sink);
-            s.plateau = false;
-            s.next_i = pos + 2;
-        }
-        return;
+__device__ __forceinline__ void scan_chunk(PeakScan& s, const numb* w, long long q0, int m, long long n,
+                                           const Sink& sink) {
+    // bit c: position q0 + c - 1 is above its predecessor and not below its successor (also
+    // set beside a NaN); w beyond the chunk's samples is stale and masked out
+    unsigned int cand = 0;
+    numb prev = w[1];
+    bool up = prev > w[0];
+    UCB_PRAGMA_(unroll UCB_SCAN_UNROLL)
+    for (int c = 0; c < kScanChunk; ++c) {
+        const numb v = w[c + 2];
+        const bool next_up = v > prev;
+        if (up && !next_up) cand |= 1u << c;
+        up = next_up;
+        prev = v;
     }
-    if (pos < s.next_i) return;
-    if (s.d1 - s.d0 > (numb)kEpsPeakDelta && s.d1 > (numb)kPeakThreshold && s.d1 >= s.d2) {
-        // inner loop starts at j = i with the same window
-        if (s.d1 - s.d2 > (numb)kEpsPeakDelta) {
-            emit_peak(s, pos, sink);
-            s.next_i = pos + 2;
-        } else {
-            s.plateau = true;
+    int c = q0 < 3 ? (int)(3 - q0) : 0;                     // positions from 2
+    const int end = n - 1 - q0 < m ? (int)(n - 1 - q0) : m;  // to n - 3
+    while (c < end) {
+        if (s.plateau) {
+            const numb d1 = w[c + 1], d2 = w[c + 2];
+            if (d1 < d2) {
+                s.plateau = false;
+                s.next_i = q0 + c + 1;
+            } else if (d1 - d2 > (numb)kEpsPeakDelta) {
+                emit_peak(s, q0 + c - 1, w[c], d1, d2, sink);
+                s.plateau = false;
+                s.next_i = q0 + c + 1;
+            }
+            ++c;
+            continue;
+        }
+        const unsigned int left = cand & (~0u << c);
+        if (!left) break;
+        c = __ffs((int)left) - 1;
+        if (c >= end) break;
+        const long long pos = q0 + c - 1;
+        const numb d0 = w[c], d1 = w[c + 1], d2 = w[c + 2];
+        ++c;
+        if (pos < s.next_i) continue;
+        if (d1 - d0 > (numb)kEpsPeakDelta && d1 > (numb)kPeakThreshold && d1 >= d2) {
+            // inner loop starts at j = i with the same window
+            if (d1 - d2 > (numb)kEpsPeakDelta) {
+                emit_peak(s, pos, d0, d1, d2, sink);
+                s.next_i = pos + 2;
+            } else {
+                s.plateau = true;
+            }
         }
     }
 }
@@ -128,23 +172,34 @@ __device__ __forceinline__ void scan_push(PeakScan& s, long long q, numb v, long
 template <class S, class Sink>
 __device__ __forceinline__ int loop_record(const S& st, numb* x, const numb* a, numb h, long long iters, int pre,
                                            int wv, numb maxv, PeakScan& scan, const Sink& sink, long long& ns) {
-    // Chunks of kCheckInterval samples, the divergence test after the first one's steps
-    // (i % kCheckInterval == 0), so the per-sample loop carries no 64-bit modulo: these
-    // launches run a warp or so per SM, where every instruction of a sample is latency.
-    for (long long i0 = 0; i0 < iters; i0 += kCheckInterval) {
-        scan_push(scan, i0, recorded_value(x, wv), iters, sink);
-        st.step(x, a, h);
-        for (int j = 1; j < pre; ++j) st.step(x, a, h);
-        ns += pre;
-        if (diverged(x, maxv)) return 0;
-        const int n = (iters - i0 < kCheckInterval) ? (int)(iters - i0) : kCheckInterval;
-        for (int c = 1; c < n; ++c) {
-            scan_push(scan, i0 + c, recorded_value(x, wv), iters, sink);
+    numb w[kScanChunk + 2];
+#pragma unroll
+    for (int k = 0; k < kScanChunk + 2; ++k) w[k] = 0;
+    // The divergence test comes after the steps of samples 0, kCheckInterval, ...
+    for (long long q0 = 0; q0 < iters; q0 += kScanChunk) {
+        const int m = (iters - q0 < kScanChunk) ? (int)(iters - q0) : kScanChunk;
+        int c = 0;
+        if (q0 % kCheckInterval == 0) {
+            w[2] = recorded_value(x, wv);
+            st.step(x, a, h);
+            for (int j = 1; j < pre; ++j) st.step(x, a, h);
+            if (diverged(x, maxv)) {
+                ns += pre;
+                return 0;
+            }
+            c = 1;
+        }
+        for (; c < m; ++c) {
+            w[c + 2] = recorded_value(x, wv);
             st.step(x, a, h);
             for (int j = 1; j < pre; ++j) st.step(x, a, h);
         }
-        ns += (long long)pre * (n - 1);
+        ns += (long long)pre * m;
+        scan_chunk(scan, w, q0, m, iters, sink);
+        w[0] = w[m];
+        w[1] = w[m + 1];
     }
+    scan.last = w[1];
     numb xPrev[UCB_NX];
 #pragma unroll
     for (int j = 0; j < UCB_NX; ++j) xPrev[j] = x[j];
@@ -208,7 +263,6 @@ extern "C" __global__ void UCB_LAUNCH_BOUNDS ucb_bif_kernel(const UcbBifParams p
             if (flag == 1 || flag == -1) {
                 ucbdev::PeakScan scan;
                 scan.init();
-                scan.d1 = scan.d2 = 0;
                 const ucbdev::Bif1dSink sink{p.out_peaks + cell * p.max_out, p.out_intervals + cell * p.max_out,
                                              p.max_out, p.time_step};
                 flag = ucbdev::loop_record(st, x, a, h, iters, p.pre_scaller, p.writable_var, p.maxv, scan, sink, ns);
@@ -348,7 +402,6 @@ __device__ __forceinline__ int bif2d_peaks(const UcbBif2dParams& p, long long ki
         if (flag == 1 || flag == -1) {
             ucbdev::PeakScan scan;
             scan.init();
-            scan.d1 = scan.d2 = 0;
             const ucbdev::Bif2dSink sink{row, p.cap};
             flag = ucbdev::loop_record(st, x, a, h, iters, p.pre_scaller, p.writable_var, p.maxv, scan, sink, ns);
             if (flag == 1) {
