@@ -116,8 +116,7 @@ __device__ __forceinline__ void basins_cell(const UcbBasinsParams& p, long long 
         } else
 #endif
         {
-            UCB_STEP_LOOP
-            for (int s = 0; s < p.steps_per_period; ++s) st.step(x, a, p.h);
+            run_single<false>(st, x, a, p.h, p.steps_per_period, p.maxv);
         }
         ns += p.steps_per_period;
 #if UCB_PHASE >= 0

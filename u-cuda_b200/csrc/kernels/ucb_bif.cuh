@@ -169,6 +169,53 @@ __device__ __forceinline__ void scan_chunk(PeakScan& s, const numb* w, long long
     }
 }
 
+// The next m samples of a series to w[2 ..], each with its `pre` steps; with check the
+// divergence test after the first sample's steps. 0: diverged there.
+template <class S>
+__device__ __forceinline__ int sample_chunk(const S& st, numb* x, const numb* a, numb h, numb* w, int m, bool check,
+                                            int pre, int wv, numb maxv) {
+    int c = 0;
+    if (check) {
+        w[2] = recorded_value(x, wv);
+        st.step(x, a, h);
+        for (int j = 1; j < pre; ++j) st.step(x, a, h);
+        if (diverged(x, maxv)) return 0;
+        c = 1;
+    }
+    for (; c < m; ++c) {
+        w[c + 2] = recorded_value(x, wv);
+        st.step(x, a, h);
+        for (int j = 1; j < pre; ++j) st.step(x, a, h);
+    }
+    return 1;
+}
+
+#ifdef UCB_SIXTH
+__device__ __noinline__ int redo_samples(numb* x, const numb* a, numb h, numb* w, int m, bool check, int pre, int wv,
+                                         numb maxv) {
+    return sample_chunk(VerbatimStepper(), x, a, h, w, m, check, pre, wv, maxv);
+}
+__device__ __forceinline__ int run_samples(const Stepper& st, numb* x, const numb* a, numb h, numb* w, int m,
+                                           bool check, int pre, int wv, numb maxv) {
+    numb keep[UCB_NX];
+    copy_state<UCB_NX>(x, keep);
+    int r = st.verbatim ? 0 : sample_chunk(st, x, a, h, w, m, check, pre, wv, maxv);
+    if (st.failed()) {
+        numb av[UCB_NV];
+        copy_values(a, av);
+        r = redo_samples(keep, av, h, w, m, check, pre, wv, maxv);
+        copy_state<UCB_NX>(keep, x);
+    }
+    return r;
+}
+#else
+template <class S>
+__device__ __forceinline__ int run_samples(const S& st, numb* x, const numb* a, numb h, numb* w, int m, bool check,
+                                           int pre, int wv, numb maxv) {
+    return sample_chunk(st, x, a, h, w, m, check, pre, wv, maxv);
+}
+#endif
+
 template <class S, class Sink>
 __device__ __forceinline__ int loop_record(const S& st, numb* x, const numb* a, numb h, long long iters, int pre,
                                            int wv, numb maxv, PeakScan& scan, const Sink& sink, long long& ns) {
@@ -178,21 +225,9 @@ __device__ __forceinline__ int loop_record(const S& st, numb* x, const numb* a, 
     // The divergence test comes after the steps of samples 0, kCheckInterval, ...
     for (long long q0 = 0; q0 < iters; q0 += kScanChunk) {
         const int m = (iters - q0 < kScanChunk) ? (int)(iters - q0) : kScanChunk;
-        int c = 0;
-        if (q0 % kCheckInterval == 0) {
-            w[2] = recorded_value(x, wv);
-            st.step(x, a, h);
-            for (int j = 1; j < pre; ++j) st.step(x, a, h);
-            if (diverged(x, maxv)) {
-                ns += pre;
-                return 0;
-            }
-            c = 1;
-        }
-        for (; c < m; ++c) {
-            w[c + 2] = recorded_value(x, wv);
-            st.step(x, a, h);
-            for (int j = 1; j < pre; ++j) st.step(x, a, h);
+        if (run_samples(st, x, a, h, w, m, q0 % kCheckInterval == 0, pre, wv, maxv) == 0) {
+            ns += pre;
+            return 0;
         }
         ns += (long long)pre * m;
         scan_chunk(scan, w, q0, m, iters, sink);
@@ -203,7 +238,7 @@ __device__ __forceinline__ int loop_record(const S& st, numb* x, const numb* a, 
     numb xPrev[UCB_NX];
 #pragma unroll
     for (int j = 0; j < UCB_NX; ++j) xPrev[j] = x[j];
-    for (int j = 0; j < pre; ++j) st.step(x, a, h);
+    run_single<false>(st, x, a, h, pre, maxv);
     ns += pre;
     return fixed_point_flag(x, xPrev);
 }
@@ -213,18 +248,17 @@ template <class S>
 __device__ __forceinline__ int loop_transient(const S& st, numb* x, const numb* a, numb h, long long iters, int pre,
                                               numb maxv, long long& ns) {
     for (long long i0 = 0; i0 < iters; i0 += kCheckInterval) {
-        st.step(x, a, h);
-        ns += 1;
-        if (diverged(x, maxv)) return 0;
-        const long long n = (iters - i0 < kCheckInterval) ? iters - i0 : kCheckInterval;
-        UCB_STEP_LOOP
-        for (long long i = 1; i < n; ++i) st.step(x, a, h);
-        ns += n - 1;
+        const int n = (iters - i0 < kCheckInterval) ? (int)(iters - i0) : kCheckInterval;
+        if (run_single<true>(st, x, a, h, n, maxv) == 0) {
+            ns += 1;
+            return 0;
+        }
+        ns += n;
     }
     numb xPrev[UCB_NX];
 #pragma unroll
     for (int j = 0; j < UCB_NX; ++j) xPrev[j] = x[j];
-    for (int j = 0; j < pre; ++j) st.step(x, a, h);
+    run_single<false>(st, x, a, h, pre, maxv);
     ns += pre;
     return fixed_point_flag(x, xPrev);
 }

@@ -120,12 +120,35 @@ __device__ __forceinline__ void probe_direction(unsigned long long seq, numb* z)
 // ---------------------------------------------------------------------------
 #ifdef UCB_EXACT
 // The KRS body verbatim (the reference's calculateDiscreteModel slot).
-struct Stepper {
-    __device__ __forceinline__ explicit Stepper(numb) {}
+struct VerbatimStepper {
     __device__ __forceinline__ void step(numb* x, const numb* a, numb h) const {
         calculateDiscreteModel(x, a, h);
     }
 };
+#ifdef UCB_SIXTH
+// The body with its division by six replaced (ucb_exact.cuh). The bits are the division's
+// while `range` stays within kSixthRange; run_single / run_pair / run_probes and the
+// sampling of ucb_bif.cuh take a block of steps again with VerbatimStepper otherwise, and the
+// trajectory's later blocks with it from the start.
+struct Stepper {
+    mutable unsigned int range;
+    mutable bool verbatim;
+    __device__ __forceinline__ explicit Stepper(numb) : range(0), verbatim(false) {}
+    __device__ __forceinline__ void step(numb* x, const numb* a, numb h) const {
+        calculateDiscreteModelFast(x, a, h, range);
+    }
+    // After a block of steps: whether it has to be taken again.
+    __device__ __forceinline__ bool failed() const {
+        if (range > kSixthRange) verbatim = true;
+        range = 0;
+        return verbatim;
+    }
+};
+#else
+struct Stepper : VerbatimStepper {
+    __device__ __forceinline__ explicit Stepper(numb) {}
+};
+#endif
 #else
 #ifdef UCB_TRIG_PHASE
 __device__ __forceinline__ void ucb_sincos(double v, double* s, double* c) { sincos(v, s, c); }
@@ -431,23 +454,154 @@ __device__ __forceinline__ bool diverged2(const float2* x, float maxValue, int c
 // `iters` steps, the divergence test after iterations 0, 100, 200, ... of this call,
 // then one extra step and the fixed-point test. 1 ok / -1 fixed point / 0 diverged.
 // ---------------------------------------------------------------------------
+// `n` steps of x; with Check the divergence test after the first of them. 0: diverged there.
+template <bool Check, class S>
+__device__ __forceinline__ int block_single(const S& s, numb* x, const numb* a, numb h, int n, numb maxValue) {
+    s.step(x, a, h);
+    if (Check && diverged(x, maxValue)) return 0;
+    UCB_STEP_LOOP
+    for (int i = 1; i < n; ++i) s.step(x, a, h);
+    return 1;
+}
+
+// The same for two trajectories in lock step.
+template <class S>
+__device__ __forceinline__ int block_pair(const S& s, numb* x, numb* y, const numb* a, numb h, int n, numb maxValue) {
+    s.step(x, a, h);
+    s.step(y, a, h);
+    if (diverged(x, maxValue) || diverged(y, maxValue)) return 0;
+    UCB_STEP_LOOP
+    for (int i = 1; i < n; ++i) {
+        s.step(x, a, h);
+        s.step(y, a, h);
+    }
+    return 1;
+}
+
+#ifdef UCB_NT
+// Steps of a block unrolled. The verbatim bodies are long: ten of them for two trajectories
+// run out of the instruction cache at one warp a scheduler (200-point curve, FP64: 5.4 ms
+// unrolled, 4.7 ms as a loop; FP32 6.8 and 6.5 ms by twos); the native ones fit.
+#if !defined(UCB_EXACT)
+#define UCB_NT_UNROLL UCB_NT
+#elif defined(UCB_NUMB_F32)
+#define UCB_NT_UNROLL 2
+#else
+#define UCB_NT_UNROLL 1
+#endif
+// A whole block of two trajectories whose length is known at compile time
+// (UCB_NT <= kCheckInterval steps and the extra step).
+template <class S>
+__device__ __forceinline__ int block_pair_nt(const S& s, numb* x, numb* y, const numb* a, numb h, numb maxValue) {
+    s.step(x, a, h);
+    s.step(y, a, h);
+    if (diverged(x, maxValue) || diverged(y, maxValue)) return 0;
+    UCB_PRAGMA_(unroll UCB_NT_UNROLL)
+    for (int i = 1; i < UCB_NT + UCB_EXTRA_STEP; ++i) {
+        s.step(x, a, h);
+        s.step(y, a, h);
+    }
+    return 1;
+}
+#endif
+
+#ifdef UCB_SIXTH
+// Blocks taken again with the division. The state at the start of the block waits in local
+// memory (the arrays these calls take), not in registers.
+template <bool Check>
+__device__ __noinline__ int redo_single(numb* x, const numb* a, numb h, int n, numb maxValue) {
+    return block_single<Check>(VerbatimStepper(), x, a, h, n, maxValue);
+}
+__device__ __noinline__ int redo_pair(numb* xy, const numb* a, numb h, int n, numb maxValue, bool whole_nt) {
+#ifdef UCB_NT
+    if (whole_nt) return block_pair_nt(VerbatimStepper(), xy, xy + UCB_NX, a, h, maxValue);
+#endif
+    return block_pair(VerbatimStepper(), xy, xy + UCB_NX, a, h, n, maxValue);
+}
+__device__ __forceinline__ void copy_values(const numb* a, numb* out) {
+#pragma unroll
+    for (int i = 0; i < UCB_NV; ++i) out[i] = a[i];
+}
+template <int N>
+__device__ __forceinline__ void copy_state(const numb* x, numb* out) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) out[i] = x[i];
+}
+
+template <bool Check>
+__device__ __forceinline__ int run_single(const Stepper& s, numb* x, const numb* a, numb h, int n, numb maxValue) {
+    numb keep[UCB_NX];
+    copy_state<UCB_NX>(x, keep);
+    int r = s.verbatim ? 0 : block_single<Check>(s, x, a, h, n, maxValue);
+    if (s.failed()) {
+        numb av[UCB_NV];
+        copy_values(a, av);
+        r = redo_single<Check>(keep, av, h, n, maxValue);
+        copy_state<UCB_NX>(keep, x);
+    }
+    return r;
+}
+__device__ __forceinline__ int finish_pair(const Stepper& s, int r, numb* keep, numb* x, numb* y, const numb* a,
+                                           numb h, int n, numb maxValue, bool whole_nt) {
+    if (s.failed()) {
+        numb av[UCB_NV];
+        copy_values(a, av);
+        r = redo_pair(keep, av, h, n, maxValue, whole_nt);
+        copy_state<UCB_NX>(keep, x);
+        copy_state<UCB_NX>(keep + UCB_NX, y);
+    }
+    return r;
+}
+__device__ __forceinline__ int run_pair(const Stepper& s, numb* x, numb* y, const numb* a, numb h, int n,
+                                        numb maxValue) {
+    numb keep[2 * UCB_NX];
+    copy_state<UCB_NX>(x, keep);
+    copy_state<UCB_NX>(y, keep + UCB_NX);
+    const int r = s.verbatim ? 0 : block_pair(s, x, y, a, h, n, maxValue);
+    return finish_pair(s, r, keep, x, y, a, h, n, maxValue, false);
+}
+#ifdef UCB_NT
+__device__ __forceinline__ int run_pair_nt(const Stepper& s, numb* x, numb* y, const numb* a, numb h, numb maxValue) {
+    numb keep[2 * UCB_NX];
+    copy_state<UCB_NX>(x, keep);
+    copy_state<UCB_NX>(y, keep + UCB_NX);
+    const int r = s.verbatim ? 0 : block_pair_nt(s, x, y, a, h, maxValue);
+    return finish_pair(s, r, keep, x, y, a, h, UCB_NT, maxValue, true);
+}
+#endif
+#else
+template <bool Check, class S>
+__device__ __forceinline__ int run_single(const S& s, numb* x, const numb* a, numb h, int n, numb maxValue) {
+    return block_single<Check>(s, x, a, h, n, maxValue);
+}
+template <class S>
+__device__ __forceinline__ int run_pair(const S& s, numb* x, numb* y, const numb* a, numb h, int n, numb maxValue) {
+    return block_pair(s, x, y, a, h, n, maxValue);
+}
+#ifdef UCB_NT
+template <class S>
+__device__ __forceinline__ int run_pair_nt(const S& s, numb* x, numb* y, const numb* a, numb h, numb maxValue) {
+    return block_pair_nt(s, x, y, a, h, maxValue);
+}
+#endif
+#endif
+
 template <class S>
 __device__ __forceinline__ int loop_single(const S& s, numb* x, const numb* a, numb h, long long iters,
                                            numb maxValue, long long& ns) {
     for (long long i0 = 0; i0 < iters; i0 += kCheckInterval) {
-        s.step(x, a, h);
-        ns += 1;
-        if (diverged(x, maxValue)) return 0;
         const int n = (iters - i0 < kCheckInterval) ? (int)(iters - i0) : kCheckInterval;
-        UCB_STEP_LOOP
-        for (int i = 1; i < n; ++i) s.step(x, a, h);
-        ns += n - 1;
+        if (run_single<true>(s, x, a, h, n, maxValue) == 0) {
+            ns += 1;
+            return 0;
+        }
+        ns += n;
     }
 #if UCB_EXTRA_STEP
     numb xPrev[UCB_NX];
 #pragma unroll
     for (int j = 0; j < UCB_NX; ++j) xPrev[j] = x[j];
-    s.step(x, a, h);
+    run_single<false>(s, x, a, h, 1, maxValue);
     ns += 1;
     return fixed_point_flag(x, xPrev);
 #else
@@ -463,51 +617,32 @@ template <class S>
 __device__ __forceinline__ int loop_pair(const S& s, numb* x, numb* y, const numb* a, numb h,
                                          long long iters, numb maxValue, long long& ns) {
     for (long long i0 = 0; i0 < iters; i0 += kCheckInterval) {
-        s.step(x, a, h);
-        s.step(y, a, h);
-        ns += 2;
-        if (diverged(x, maxValue) || diverged(y, maxValue)) return 0;
         const int n = (iters - i0 < kCheckInterval) ? (int)(iters - i0) : kCheckInterval;
-        UCB_STEP_LOOP
-        for (int i = 1; i < n; ++i) {
-            s.step(x, a, h);
-            s.step(y, a, h);
+        if (run_pair(s, x, y, a, h, n, maxValue) == 0) {
+            ns += 2;
+            return 0;
         }
-        ns += 2 * (n - 1);
+        ns += 2 * n;
     }
 #if UCB_EXTRA_STEP
-    s.step(x, a, h);
-    s.step(y, a, h);
+    run_single<false>(s, x, a, h, 1, maxValue);
+    run_single<false>(s, y, a, h, 1, maxValue);
     ns += 2;
 #endif
     return 1;
 }
 
 #ifdef UCB_NT
-// loop_pair for a block length known at compile time (UCB_NT <= kCheckInterval steps):
-// the same sequence — first step of both, divergence test, the remaining UCB_NT - 1
-// steps, the extra step — fully unrolled, without loop control.
+// loop_pair for a block length known at compile time: the same sequence — first step of
+// both, divergence test, the remaining UCB_NT - 1 steps, the extra step.
 template <class S>
 __device__ __forceinline__ int loop_pair_nt(const S& s, numb* x, numb* y, const numb* a, numb h, numb maxValue,
                                             long long& ns) {
-    s.step(x, a, h);
-    s.step(y, a, h);
-    if (diverged(x, maxValue) || diverged(y, maxValue)) {
+    if (run_pair_nt(s, x, y, a, h, maxValue) == 0) {
         ns += 2;
         return 0;
     }
-#pragma unroll
-    for (int i = 1; i < UCB_NT; ++i) {
-        s.step(x, a, h);
-        s.step(y, a, h);
-    }
-#if UCB_EXTRA_STEP
-    s.step(x, a, h);
-    s.step(y, a, h);
-    ns += 2 * (UCB_NT + 1);
-#else
-    ns += 2 * UCB_NT;
-#endif
+    ns += 2 * (UCB_NT + UCB_EXTRA_STEP);
     return 1;
 }
 #endif

@@ -374,7 +374,10 @@ extern "C" __global__ void UCB_LAUNCH_BOUNDS ucb_state_kernel(const UcbLleParams
     for (int k = 0; k < UCB_NV; ++k) a[k] = p.vals[k];
     ucbdev::apply_sweep(c, p.axis0, p.axis1, x, a);
     const ucbdev::Stepper st(cs.h);
-    for (long long s = 0; s < p.skip; ++s) st.step(x, a, cs.h);
+    for (long long s = 0; s < p.skip; s += ucbdev::kCheckInterval) {
+        const int n = p.skip - s < ucbdev::kCheckInterval ? (int)(p.skip - s) : ucbdev::kCheckInterval;
+        ucbdev::run_single<false>(st, x, a, cs.h, n, p.maxv);
+    }
 #pragma unroll
     for (int k = 0; k < UCB_NX; ++k) p.out_values[i * UCB_NX + k] = (double)x[k];
 }

@@ -101,32 +101,75 @@ __device__ __forceinline__ void gram_schmidt_classical(const numb (*a)[UCB_NX], 
     }
 }
 
-// x and the N probes advanced in lock step (the reference advances them one after the
-// other; they never interact inside a block). 0 if any diverged.
-template <class S>
-__device__ __forceinline__ int loop_probes(const S& s, numb* x, numb (*y)[UCB_NX], const numb* a, numb h,
-                                           long long iters, numb maxValue, long long& ns) {
-    for (long long i0 = 0; i0 < iters; i0 += kCheckInterval) {
-        s.step(x, a, h);
+// `n` steps of x and the N probes in lock step (the reference advances them one after the
+// other; they never interact inside a block); with Check the divergence test after the first
+// of them. 0 if any diverged there.
+template <bool Check, class S>
+__device__ __forceinline__ int block_probes(const S& s, numb* x, numb (*y)[UCB_NX], const numb* a, numb h, int n,
+                                            numb maxValue) {
+    s.step(x, a, h);
 #pragma unroll
-        for (int j = 0; j < UCB_NX; ++j) s.step(y[j], a, h);
-        ns += UCB_NX + 1;
+    for (int j = 0; j < UCB_NX; ++j) s.step(y[j], a, h);
+    if (Check) {
         bool bad = diverged(x, maxValue);
 #pragma unroll
         for (int j = 0; j < UCB_NX; ++j) bad = bad || diverged(y[j], maxValue);
         if (bad) return 0;
-        const long long n = (iters - i0 < kCheckInterval) ? iters - i0 : kCheckInterval;
-        for (long long i = 1; i < n; ++i) {
-            s.step(x, a, h);
+    }
+    for (int i = 1; i < n; ++i) {
+        s.step(x, a, h);
 #pragma unroll
-            for (int j = 0; j < UCB_NX; ++j) s.step(y[j], a, h);
+        for (int j = 0; j < UCB_NX; ++j) s.step(y[j], a, h);
+    }
+    return 1;
+}
+
+#ifdef UCB_SIXTH
+template <bool Check>
+__device__ __noinline__ int redo_probes(numb* xy, const numb* a, numb h, int n, numb maxValue) {
+    return block_probes<Check>(VerbatimStepper(), xy, reinterpret_cast<numb(*)[UCB_NX]>(xy + UCB_NX), a, h, n,
+                               maxValue);
+}
+template <bool Check>
+__device__ __forceinline__ int run_probes(const Stepper& s, numb* x, numb (*y)[UCB_NX], const numb* a, numb h, int n,
+                                          numb maxValue) {
+    numb keep[UCB_NX + UCB_NX * UCB_NX];
+    copy_state<UCB_NX>(x, keep);
+#pragma unroll
+    for (int j = 0; j < UCB_NX; ++j) copy_state<UCB_NX>(y[j], keep + UCB_NX + j * UCB_NX);
+    int r = s.verbatim ? 0 : block_probes<Check>(s, x, y, a, h, n, maxValue);
+    if (s.failed()) {
+        numb av[UCB_NV];
+        copy_values(a, av);
+        r = redo_probes<Check>(keep, av, h, n, maxValue);
+        copy_state<UCB_NX>(keep, x);
+#pragma unroll
+        for (int j = 0; j < UCB_NX; ++j) copy_state<UCB_NX>(keep + UCB_NX + j * UCB_NX, y[j]);
+    }
+    return r;
+}
+#else
+template <bool Check, class S>
+__device__ __forceinline__ int run_probes(const S& s, numb* x, numb (*y)[UCB_NX], const numb* a, numb h, int n,
+                                          numb maxValue) {
+    return block_probes<Check>(s, x, y, a, h, n, maxValue);
+}
+#endif
+
+// A whole loop call of x and the probes. 0 if any diverged.
+template <class S>
+__device__ __forceinline__ int loop_probes(const S& s, numb* x, numb (*y)[UCB_NX], const numb* a, numb h,
+                                           long long iters, numb maxValue, long long& ns) {
+    for (long long i0 = 0; i0 < iters; i0 += kCheckInterval) {
+        const int n = (iters - i0 < kCheckInterval) ? (int)(iters - i0) : kCheckInterval;
+        if (run_probes<true>(s, x, y, a, h, n, maxValue) == 0) {
+            ns += UCB_NX + 1;
+            return 0;
         }
-        ns += (long long)(UCB_NX + 1) * (n - 1);
+        ns += (long long)(UCB_NX + 1) * n;
     }
 #if UCB_EXTRA_STEP
-    s.step(x, a, h);
-#pragma unroll
-    for (int j = 0; j < UCB_NX; ++j) s.step(y[j], a, h);
+    run_probes<false>(s, x, y, a, h, 1, maxValue);
     ns += UCB_NX + 1;
 #endif
     return 1;

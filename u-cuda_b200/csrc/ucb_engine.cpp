@@ -278,19 +278,34 @@ SystemCode make_system_code(const std::string& krs_body, int nx, int nv, int pre
         s.note = "native form unavailable (" + why + "); using the exact form";
     }
     (void)nv;
+    std::string fast;
     {
         // Algorithmic FLOPs of the exact form: the same RK4 count when the body is the
         // template, unknown (0) for other bodies.
         fe::Rhs r;
         std::string why;
         try {
-            if (fe::recognize_rk4(krs_body, nx, r, why)) s.flops_step = fe::rk4_step_flops(r);
+            if (fe::recognize_rk4(krs_body, nx, r, why)) {
+                s.flops_step = fe::rk4_step_flops(r);
+                // the template with its division by six replaced, same bits (ucb_exact.cuh)
+                const std::string sum = "h * (k[i][0] + 2 * k[i][1] + 2 * k[i][2] + k[i][3])";
+                const size_t at = krs_body.find(sum + " / 6;");
+                if (at != std::string::npos) {
+                    fast = krs_body;
+                    fast.replace(at, sum.size() + 5, "ucb_sixth(" + sum + ", sixth_range);");
+                }
+            }
         } catch (...) {
         }
     }
     std::ostringstream o;
     o << "__device__ __forceinline__ void calculateDiscreteModel(numb* X, const numb* a, const numb h) {\n"
       << krs_body << "\n}\n";
+    if (!fast.empty())
+        o << "#define UCB_SIXTH 1\n#include \"ucb_exact.cuh\"\n"
+          << "__device__ __forceinline__ void calculateDiscreteModelFast(numb* X, const numb* a, const numb h, "
+             "unsigned int& sixth_range) {\n"
+          << fast << "\n}\n";
     s.exact = true;
     s.code = o.str();
     return s;
