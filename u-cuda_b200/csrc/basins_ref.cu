@@ -15,11 +15,12 @@
 // space: cells are binned into squares of side 0.7 eps (two cells of one square are
 // within eps of each other, so a square is connected by construction), squares are sorted,
 // neighbouring squares up to two apart are joined (atomic union-find) when any pair of
-// their cells is within eps, and the components are ranked by their lowest fixed-point /
+// their cells is within eps (the squares next to each other first), and the components are ranked by their lowest fixed-point /
 // oscillating cell with a radix sort.
 #include <cuda_runtime.h>
 
 #include <cub/cub.cuh>
+#include <math_constants.h>
 
 #include <algorithm>
 #include <cmath>
@@ -38,7 +39,7 @@ constexpr long long kExcluded = 0x7FFFFFFFFFFFFFFFLL;   // unbound cells (last s
 constexpr long long kSingleton = 0x7FFFFFFFFFFFFFFELL;  // cells that join nothing: own square
 constexpr double kMaxSquare = 2305843009213693952.0;     // 2^61 squares from the origin
 constexpr unsigned int kNone = 0xFFFFFFFFu;
-constexpr int kPairInline = 1024;  // pair products searched by the square's own thread
+constexpr int kPairInline = 256;  // pair products searched by one thread
 
 // Feature bounding box of a square as order-preserving integer keys (dkey).
 struct Box {
@@ -214,93 +215,229 @@ __device__ __forceinline__ void unite(unsigned int* parent, unsigned int a, unsi
 }
 
 // The reference's neighbour test, sqrt(dx^2 + dy^2) <= eps, in numb (float when single),
-// rounded operation by operation (no contraction into FMA).
-__device__ __forceinline__ bool within(double ax, double ay, double bx, double by, double eps, int single) {
-    if (single) {
-        const float dx = __fsub_rn((float)ax, (float)bx), dy = __fsub_rn((float)ay, (float)by);
-        return sqrtf(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy))) <= (float)eps;
+// rounded operation by operation (no contraction into FMA). The square root only decides
+// within a few ulp of eps: outside that band (in2, out2: eps^2 less / more the margin) the
+// rounded square does, where eps^2 is well inside the range of numb.
+struct Within {
+    double eps, in2, out2;
+    int single;
+    bool plain;
+    __device__ __forceinline__ Within(double e, int s) : eps(e), single(s) {
+        const double margin = s ? 1e-5 : 1e-9;
+        plain = s ? (e > 1e-15 && e < 1e15) : (e > 1e-140 && e < 1e140);
+        in2 = plain ? e * e * (1.0 - margin) : -1.0;
+        out2 = plain ? e * e * (1.0 + margin) : CUDART_INF;
     }
-    const double dx = __dsub_rn(ax, bx), dy = __dsub_rn(ay, by);
-    return sqrt(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy))) <= eps;
-}
+    __device__ __forceinline__ bool operator()(double ax, double ay, double bx, double by) const {
+        const double dx = __dsub_rn(ax, bx), dy = __dsub_rn(ay, by);
+        const double d2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
+        if (d2 > out2) return false;
+        if (d2 < in2) return true;
+        if (single) {
+            const float fx = __fsub_rn((float)ax, (float)bx), fy = __fsub_rn((float)ay, (float)by);
+            return sqrtf(__fadd_rn(__fmul_rn(fx, fx), __fmul_rn(fy, fy))) <= (float)eps;
+        }
+        return sqrt(d2) <= eps;
+    }
+};
 
-// Every square is joined with the squares up to two steps ahead of it (the other half of
-// its 5 x 5 neighbourhood joins it from the other side): skipped when the boxes are
-// surely more than eps apart, joined outright when every pair is surely within eps,
-// otherwise searched pair by pair — here for small squares, by a whole CTA later
-// (heavy list) for large ones. The margins cover the rounding of the reference's test
-// (a few ulp of numb).
+// Offsets of the squares ahead of a square in its 5 x 5 neighbourhood (the other half joins
+// it from its own side): the 4 next to it, then the 8 two steps away.
+__constant__ signed char kAheadX[12] = {0, 1, 1, 1, 0, 1, 1, 2, 2, 2, 2, 2};
+__constant__ signed char kAheadY[12] = {1, -1, 0, 1, 2, -2, 2, -2, -1, 0, 1, 2};
+
+// Joins every square with `count` of the squares ahead of it, from offset `first`, one thread
+// per pair: skipped when the boxes are surely more than eps apart, joined outright when every
+// pair of cells is surely within eps, otherwise searched cell by cell — here for small
+// squares, by a whole CTA (heavy list) for large ones. The margins cover the rounding of
+// the reference's test (a few ulp of numb).
 __global__ void join_kernel(const double* sf1, const double* sf2, const unsigned int* start, const long long* sx,
-                            const long long* sy, const Box* box, unsigned int nsq, double eps, int single,
-                            unsigned int* parent, uint2* heavy, unsigned int* n_heavy) {
-    const unsigned int s = blockIdx.x * blockDim.x + threadIdx.x;
+                            const long long* sy, const Box* box, unsigned int nsq, double eps, int single, int first,
+                            int count, unsigned int* parent, uint2* heavy, unsigned int* n_heavy) {
+    const unsigned long long w = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned int s = (unsigned int)(w / count);
     if (s >= nsq || sx[s] == kExcluded || sx[s] == kSingleton) return;
+    const int k = first + (int)(w % count);
+    const Within within(eps, single);
     const double margin = single ? 1e-5 : 1e-9;
     const double lo2 = eps * eps * (1.0 - margin), hi2 = eps * eps * (1.0 + margin);
-    const unsigned int a0 = start[s], a1 = start[s + 1];
-    const Box ka = box[s];
-    const double ax0 = dval(ka.x0), ax1 = dval(ka.x1), ay0 = dval(ka.y0), ay1 = dval(ka.y1);
-    for (int dx = 0; dx <= 2; ++dx) {
-        for (int dy = -2; dy <= 2; ++dy) {
-            if (dx == 0 && dy <= 0) continue;
-            const long long tx = sx[s] + dx, ty = sy[s] + dy;
-            unsigned int lo = 0, hi = nsq;  // binary search of (tx, ty) among the sorted squares
-            while (lo < hi) {
-                const unsigned int mid = (lo + hi) >> 1;
-                if (sx[mid] < tx || (sx[mid] == tx && sy[mid] < ty)) lo = mid + 1;
-                else hi = mid;
-            }
-            if (lo >= nsq || sx[lo] != tx || sy[lo] != ty) continue;
-            const unsigned int t = lo;
-            const Box kb = box[t];
-            const double bx0 = dval(kb.x0), bx1 = dval(kb.x1), by0 = dval(kb.y0), by1 = dval(kb.y1);
-            const double gx = fmax(0.0, fmax(bx0 - ax1, ax0 - bx1)), gy = fmax(0.0, fmax(by0 - ay1, ay0 - by1));
-            if (gx * gx + gy * gy > hi2) continue;
-            const double fx = fmax(ax1, bx1) - fmin(ax0, bx0), fy = fmax(ay1, by1) - fmin(ay0, by0);
-            if (fx * fx + fy * fy < lo2) {
-                unite(parent, s, t);
-                continue;
-            }
-            if (find_root(parent, s) == find_root(parent, t)) continue;
-            const unsigned int b0 = start[t], b1 = start[t + 1];
-            if ((unsigned long long)(a1 - a0) * (b1 - b0) > (unsigned long long)kPairInline) {
-                heavy[atomicAdd(n_heavy, 1u)] = make_uint2(s, t);
-                continue;
-            }
-            bool hit = false;
-            for (unsigned int i = a0; i < a1 && !hit; ++i)
-                for (unsigned int j = b0; j < b1 && !hit; ++j) hit = within(sf1[i], sf2[i], sf1[j], sf2[j], eps, single);
-            if (hit) unite(parent, s, t);
-        }
+    const long long tx = sx[s] + kAheadX[k], ty = sy[s] + kAheadY[k];
+    unsigned int lo = s + 1, hi = nsq;  // binary search of (tx, ty) among the sorted squares
+    while (lo < hi) {
+        const unsigned int mid = (lo + hi) >> 1;
+        if (sx[mid] < tx || (sx[mid] == tx && sy[mid] < ty)) lo = mid + 1;
+        else hi = mid;
     }
+    if (lo >= nsq || sx[lo] != tx || sy[lo] != ty) return;
+    const unsigned int t = lo;
+    const Box ka = box[s], kb = box[t];
+    const double ax0 = dval(ka.x0), ax1 = dval(ka.x1), ay0 = dval(ka.y0), ay1 = dval(ka.y1);
+    const double bx0 = dval(kb.x0), bx1 = dval(kb.x1), by0 = dval(kb.y0), by1 = dval(kb.y1);
+    const double gx = fmax(0.0, fmax(bx0 - ax1, ax0 - bx1)), gy = fmax(0.0, fmax(by0 - ay1, ay0 - by1));
+    if (gx * gx + gy * gy > hi2) return;
+    const double fx = fmax(ax1, bx1) - fmin(ax0, bx0), fy = fmax(ay1, by1) - fmin(ay0, by0);
+    if (fx * fx + fy * fy < lo2) {
+        unite(parent, s, t);
+        return;
+    }
+    if (find_root(parent, s) == find_root(parent, t)) return;
+    const unsigned int a0 = start[s], a1 = start[s + 1], b0 = start[t], b1 = start[t + 1];
+    if ((unsigned long long)(a1 - a0) * (b1 - b0) > (unsigned long long)kPairInline) {
+        heavy[atomicAdd(n_heavy, 1u)] = make_uint2(s, t);
+        return;
+    }
+    bool hit = false;
+    for (unsigned int i = a0; i < a1 && !hit; ++i)
+        for (unsigned int j = b0; j < b1 && !hit; ++j) hit = within(sf1[i], sf2[i], sf1[j], sf2[j]);
+    if (hit) unite(parent, s, t);
 }
 
-// Pair search of the heavy square pairs: one CTA per pair, threads striding over the
-// first square's cells, stopping as soon as any thread finds a pair within eps.
-__global__ void __launch_bounds__(256) heavy_join_kernel(const double* sf1, const double* sf2,
-                                                         const unsigned int* start, const uint2* heavy,
-                                                         const unsigned int* n_heavy, double eps, int single,
-                                                         unsigned int* parent) {
+// Bounding boxes of a square's cells by kSub x kSub parts of its box, as floats relative to
+// the box's lower corner and rounded outwards (non-negative, so ordered as integers).
+constexpr int kSub = 16, kParts = kSub * kSub;
+struct PartBoxes {
+    float x0[kParts], x1[kParts], y0[kParts], y1[kParts];
+};
+
+struct Frame {  // a square's box
+    double x0, y0, ix, iy;
+    __device__ __forceinline__ explicit Frame(const Box& b) : x0(dval(b.x0)), y0(dval(b.y0)) {
+        const double wx = dval(b.x1) - x0, wy = dval(b.y1) - y0;
+        ix = wx > 0 ? kSub / wx : 0;
+        iy = wy > 0 ? kSub / wy : 0;
+    }
+    __device__ __forceinline__ int part(double x, double y) const {
+        const int i = min(kSub - 1, (int)((x - x0) * ix)), j = min(kSub - 1, (int)((y - y0) * iy));
+        return j * kSub + i;
+    }
+};
+
+__device__ __forceinline__ void lower(float* at, float v) {
+    if (v < *(volatile float*)at) atomicMin(reinterpret_cast<int*>(at), __float_as_int(v));
+}
+__device__ __forceinline__ void raise(float* at, float v) {
+    if (v > *(volatile float*)at) atomicMax(reinterpret_cast<int*>(at), __float_as_int(v));
+}
+
+// Search of the heavy square pairs for cells within eps of each other, one CTA per pair:
+//   1. pairs joined meanwhile are skipped, and a few thousand cell pairs are tried (dense
+//      neighbouring squares are joined here);
+//   2. the squares' parts: a pair of part boxes surely within eps joins the squares, one surely
+//      farther apart is out; only the cells of the parts in between (boxes about eps apart)
+//   3. are compared, a tile of the second square's at a time.
+// Trying every pair of cells took (cells of a)(cells of b) square roots where no pair is
+// within eps — two squares of a dense attractor's rim, or of two attractors side by side — and
+// most of the time of the clustering. B200, whole calls, 1,048,576 cells of four attractors,
+// eps 0.25: 41 -> 3.1 ms (mean of three inputs; 3.0 ms where every heavy pair had a hit, as
+// before); of two attractors, eps 0.5, FP32: 696 -> 3.3 ms.
+constexpr int kHeavyThreads = 256, kTile = 512;
+constexpr unsigned long long kDirect = 1 << 15;  // pair products compared without the parts
+__global__ void __launch_bounds__(kHeavyThreads) heavy_join_kernel(const double* sf1, const double* sf2,
+                                                                   const unsigned int* start, const Box* box,
+                                                                   const uint2* heavy, const unsigned int* n_heavy,
+                                                                   double eps, int single, unsigned int* parent) {
     __shared__ int found;
+    __shared__ PartBoxes part[2];
+    __shared__ unsigned char live[2][kParts];
+    __shared__ double tx[kTile], ty[kTile];
+    __shared__ int n_tile;
+    const Within within(eps, single);
     const unsigned int count = *n_heavy;
+    const int tid = threadIdx.x;
     for (unsigned int w = blockIdx.x; w < count; w += gridDim.x) {
         const unsigned int s = heavy[w].x, t = heavy[w].y;
-        if (threadIdx.x == 0) found = find_root(parent, s) == find_root(parent, t) ? 1 : 0;
+        if (tid == 0) found = find_root(parent, s) == find_root(parent, t) ? 1 : 0;
         __syncthreads();
-        const unsigned int a0 = start[s], a1 = start[s + 1], b0 = start[t], b1 = start[t + 1];
-        for (unsigned int i = a0 + threadIdx.x; i < a1; i += blockDim.x) {
-            if (*(volatile int*)&found) break;
-            const double x = sf1[i], y = sf2[i];
-            for (unsigned int j = b0; j < b1; ++j) {
-                if (within(x, y, sf1[j], sf2[j], eps, single)) {
+        const unsigned int a0 = start[s], b0 = start[t];
+        const unsigned int na = start[s + 1] - a0, nb = start[t + 1] - b0;
+        const Box ba = box[s], bb = box[t];
+        const unsigned long long product = (unsigned long long)na * nb;
+        if (!found) {
+            unsigned int r = (unsigned int)tid * 2654435761u + 12345u;
+            for (int k = 0; k < 16; ++k) {
+                r = r * 1664525u + 1013904223u;
+                const unsigned int i = a0 + (unsigned int)(((unsigned long long)r * na) >> 32);
+                r = r * 1664525u + 1013904223u;
+                const unsigned int j = b0 + (unsigned int)(((unsigned long long)r * nb) >> 32);
+                if (within(sf1[i], sf2[i], sf1[j], sf2[j])) found = 2;
+            }
+        }
+        __syncthreads();
+        // the boxes' coordinates resolve eps: else every part is compared
+        const double reach = fmax(fmax(fabs(dval(ba.x0)), fabs(dval(ba.x1))), fmax(fabs(dval(ba.y0)), fabs(dval(ba.y1))));
+        const bool parts = product > kDirect && within.plain && reach < 1e7 * eps;
+        const Frame fa(ba), fb(bb);
+        if (!found && parts) {
+            for (int k = tid; k < 2 * kParts; k += kHeavyThreads) {
+                PartBoxes& p = part[k / kParts];
+                const int c = k % kParts;
+                p.x0[c] = p.y0[c] = CUDART_INF_F;
+                p.x1[c] = p.y1[c] = -1.0f;  // empty
+                live[k / kParts][c] = 0;
+            }
+            __syncthreads();
+            for (int side = 0; side < 2; ++side) {
+                const Frame& f = side ? fb : fa;
+                const unsigned int c0 = side ? b0 : a0, n = side ? nb : na;
+                PartBoxes& p = part[side];
+                for (unsigned int i = tid; i < n; i += kHeavyThreads) {
+                    const double x = sf1[c0 + i], y = sf2[c0 + i];
+                    const int c = f.part(x, y);
+                    lower(&p.x0[c], __double2float_rd(x - f.x0));
+                    raise(&p.x1[c], __double2float_ru(x - f.x0));
+                    lower(&p.y0[c], __double2float_rd(y - f.y0));
+                    raise(&p.y1[c], __double2float_ru(y - f.y0));
+                }
+            }
+            __syncthreads();
+            const double ox = fb.x0 - fa.x0, oy = fb.y0 - fa.y0;  // the second frame in the first
+            const double near2 = eps * eps * (1.0 - 2e-5), far2 = eps * eps * (1.0 + 2e-5);
+            for (int k = tid; k < kParts * kParts; k += kHeavyThreads) {
+                const int i = k % kParts, j = k / kParts;
+                if (part[0].x1[i] < 0 || part[1].x1[j] < 0) continue;
+                const double px0 = part[0].x0[i], px1 = part[0].x1[i], py0 = part[0].y0[i], py1 = part[0].y1[i];
+                const double qx0 = part[1].x0[j] + ox, qx1 = part[1].x1[j] + ox;
+                const double qy0 = part[1].y0[j] + oy, qy1 = part[1].y1[j] + oy;
+                const double gx = fmax(0.0, fmax(qx0 - px1, px0 - qx1)), gy = fmax(0.0, fmax(qy0 - py1, py0 - qy1));
+                if (gx * gx + gy * gy > far2) continue;
+                const double fx = fmax(px1, qx1) - fmin(px0, qx0), fy = fmax(py1, qy1) - fmin(py0, qy0);
+                if (fx * fx + fy * fy < near2) {
                     found = 2;
                     break;
                 }
-                if (((j - b0) & 63) == 63 && *(volatile int*)&found) break;
+                live[0][i] = live[1][j] = 1;
             }
         }
         __syncthreads();
-        if (threadIdx.x == 0 && found == 2) unite(parent, s, t);
+        if (!found) {
+            for (unsigned int j0 = 0; j0 < nb; j0 += kTile) {
+                if (tid == 0) n_tile = 0;
+                __syncthreads();
+                for (unsigned int j = j0 + tid; j < min(nb, j0 + kTile); j += kHeavyThreads) {
+                    const double x = sf1[b0 + j], y = sf2[b0 + j];
+                    if (parts && !live[1][fb.part(x, y)]) continue;
+                    const int at = atomicAdd(&n_tile, 1);
+                    tx[at] = x;
+                    ty[at] = y;
+                }
+                __syncthreads();
+                if (n_tile) {
+                    for (unsigned int i = tid; i < na; i += kHeavyThreads) {
+                        if (*(volatile int*)&found) break;
+                        const double x = sf1[a0 + i], y = sf2[a0 + i];
+                        if (parts && !live[0][fa.part(x, y)]) continue;
+                        bool hit = false;
+#pragma unroll 4
+                        for (int j = 0; j < n_tile; ++j) hit = hit || within(x, y, tx[j], ty[j]);
+                        if (hit) found = 2;
+                    }
+                }
+                __syncthreads();
+                if (found) break;
+            }
+        }
+        __syncthreads();
+        if (tid == 0 && found == 2) unite(parent, s, t);
         __syncthreads();
     }
 }
@@ -410,7 +547,7 @@ int cluster_features(ucb_engine* e, cudaStream_t st, DeviceArena& mem, double* d
     unsigned int* sq_of = mem.get<unsigned int>(N);
     double* sf1 = mem.get<double>(N);
     double* sf2 = mem.get<double>(N);
-    unsigned int* counts = mem.get<unsigned int>(4);  // [2]: heavy square pairs
+    unsigned int* counts = mem.get<unsigned int>(2);  // heavy pairs of squares next to / two steps from each other
     if (!bx || !by || !k_in || !k_out || !v_in || !order || !head || !sq_of || !sf1 || !sf2 || !counts) {
         err = mem.err;
         return -1;
@@ -450,7 +587,7 @@ int cluster_features(ucb_engine* e, cudaStream_t st, DeviceArena& mem, double* d
     unsigned int* root_fp = mem.get<unsigned int>(nsq);
     unsigned int* root_osc = mem.get<unsigned int>(nsq);
     int* comp_label = mem.get<int>(nsq);
-    uint2* heavy = mem.get<uint2>((size_t)nsq * 12);
+    uint2* heavy = mem.get<uint2>((size_t)nsq * 8);
     if (!start || !sx || !sy || !box || !parent || !min_fp || !min_osc || !root_fp || !root_osc || !comp_label ||
         !heavy) {
         err = mem.err;
@@ -460,10 +597,17 @@ int cluster_features(ucb_engine* e, cudaStream_t st, DeviceArena& mem, double* d
     ucbbr::init_squares_kernel<<<GS, B, 0, st>>>(nsq, N, start, parent, box, min_fp, min_osc, comp_label);
     ucbbr::squares_kernel<<<G, B, 0, st>>>(bx, by, order, head, sq_of, N, start, sx, sy);
     ucbbr::square_stats_kernel<<<G, B, 0, st>>>(sf1, sf2, order, sq_of, d_cls, sx, N, box, min_fp, min_osc);
-    cudaMemsetAsync(counts + 2, 0, 4, st);
-    ucbbr::join_kernel<<<GS, B, 0, st>>>(sf1, sf2, start, sx, sy, box, nsq, eps, single, parent, heavy, counts + 2);
-    ucbbr::heavy_join_kernel<<<e->sm_count * 4, 256, 0, st>>>(sf1, sf2, start, heavy, counts + 2, eps, single,
-                                                                parent);
+    // Squares next to each other first: two steps apart, most pairs of a dense attractor are
+    // then joined through the square between them and drop out.
+    cudaMemsetAsync(counts, 0, 8, st);
+    for (int far = 0; far < 2; ++far) {
+        const int first = far ? 4 : 0, count = far ? 8 : 4;
+        const unsigned int GJ = (unsigned int)(((unsigned long long)nsq * count + B - 1) / B);
+        ucbbr::join_kernel<<<GJ, B, 0, st>>>(sf1, sf2, start, sx, sy, box, nsq, eps, single, first, count, parent, heavy,
+                                             counts + far);
+        ucbbr::heavy_join_kernel<<<e->sm_count * 4, ucbbr::kHeavyThreads, 0, st>>>(sf1, sf2, start, box, heavy,
+                                                                                   counts + far, eps, single, parent);
+    }
     cudaMemsetAsync(root_fp, 0xFF, (size_t)nsq * 4, st);
     cudaMemsetAsync(root_osc, 0xFF, (size_t)nsq * 4, st);
     ucbbr::root_stats_kernel<<<GS, B, 0, st>>>(parent, min_fp, min_osc, nsq, root_fp, root_osc);
@@ -490,7 +634,7 @@ int cluster_features(ucb_engine* e, cudaStream_t st, DeviceArena& mem, double* d
         err = std::string("CUDA basins clustering: ") + cudaGetErrorString(ce);
         return -1;
     }
-    return 13;  // own kernels (the radix sorts and the scan are CUB's)
+    return 15;  // own kernels (the radix sorts and the scan are CUB's)
 }
 
 void label_extremes(const int* labels, long long n, int& mx, int& mn) {
