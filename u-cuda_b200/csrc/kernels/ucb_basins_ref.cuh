@@ -85,7 +85,8 @@ struct BasinSums {
     }
 };
 
-__device__ __forceinline__ void basins_ref_cell(const UcbBasinsRefParams& p, long long cell, long long& ns) {
+__device__ __forceinline__ void basins_ref_cell(const UcbBasinsRefParams& p, long long cell, bool live,
+                                                long long& ns) {
     const CellAxes c = cell_axes(cell, p.n_pts);
     numb x[UCB_NX], a[UCB_NV];
 #pragma unroll
@@ -93,9 +94,9 @@ __device__ __forceinline__ void basins_ref_cell(const UcbBasinsRefParams& p, lon
 #pragma unroll
     for (int k = 0; k < UCB_NV; ++k) a[k] = p.vals[k];
     apply_sweep(c, p.axis0, p.axis1, x, a);
-    const Stepper st(p.h);
+    UCB_CELL_STEPPER(p.h, x);
     numb f1, f2;
-    int flag = loop_transient(st, x, a, p.h, p.skip, p.pre_scaller, p.maxv, ns);
+    int flag = loop_transient(st, x, a, p.h, p.skip, p.pre_scaller, p.maxv, ns, live);
     BasinSums sums;
     bool a1, a2, a3, a4, b1, b2, b3, b4;
     basin_needs(p.feature1, a1, a2, a3, a4);
@@ -108,8 +109,9 @@ __device__ __forceinline__ void basins_ref_cell(const UcbBasinsRefParams& p, lon
     sums.sp = sums.sp2 = sums.si = sums.si2 = 0;
     PeakScan scan;
     scan.init();
-    if (flag == 1 || flag == -1) flag = loop_record(st, x, a, p.h, p.points, p.pre_scaller, p.writable_var, p.maxv,
-                                                     scan, sums, ns);
+    if (UCB_RECORDS(flag)) flag = loop_record(st, x, a, p.h, p.points, p.pre_scaller, p.writable_var, p.maxv, scan,
+                                              sums, ns, flag != 0);
+    if (!live) return;
     if (flag == 0) {
         f1 = 999;
         f2 = 999;
@@ -156,7 +158,11 @@ extern "C" __global__ void UCB_LAUNCH_BOUNDS ucb_basins_ref_kernel(const UcbBasi
         const long long base = ucbdev::warp_fetch(p.counter, lane);
         if (base >= p.total) break;
         const long long i = base + lane;
-        if (i < p.total) ucbdev::basins_ref_cell(p, i, ns);
+#ifdef UCB_FORCED
+        ucbdev::basins_ref_cell(p, i < p.total ? i : p.total - 1, i < p.total, ns);
+#else
+        if (i < p.total) ucbdev::basins_ref_cell(p, i, true, ns);
+#endif
     }
     ucbdev::warp_add_steps(p.steps, ns, lane);
 }

@@ -216,9 +216,91 @@ __device__ __forceinline__ int run_samples(const S& st, numb* x, const numb* a, 
 }
 #endif
 
+#ifdef UCB_FORCED
+// The loops of a build whose warp shares its forcing: every lane takes every step, and a lane
+// without a live cell (past the grid, or diverged) only does not count.
+template <class Sink>
+__device__ __forceinline__ int loop_record(const ForcedStepper& st, numb* x, const numb* a, numb h, long long iters,
+                                           int pre, int wv, numb maxv, PeakScan& scan, const Sink& sink,
+                                           long long& ns, bool live) {
+    if (!__any_sync(0xFFFFFFFFu, live)) return 0;
+    numb w[kScanChunk + 2];
+#pragma unroll
+    for (int k = 0; k < kScanChunk + 2; ++k) w[k] = 0;
+    for (long long q0 = 0; q0 < iters; q0 += kScanChunk) {
+        const int m = (iters - q0 < kScanChunk) ? (int)(iters - q0) : kScanChunk;
+        int c = 0;
+        if (q0 % kCheckInterval == 0) {
+            st.set_phase(x);
+            w[2] = recorded_value(x, wv);
+            st.steps(x, a, h, pre);
+            if (live && diverged(x, maxv)) {
+                ns += pre;
+                live = false;
+            }
+            if (!__any_sync(0xFFFFFFFFu, live)) return 0;
+            c = 1;
+        }
+        if (pre == 1 && wv >= 0 && wv != UCB_TRIG_PHASE) {
+            numb* at = w + c + 2;
+            st.steps(x, a, h, m - c, [&](int i) { at[i] = recorded_value(x, wv); });
+        } else {
+            for (; c < m; ++c) {
+                st.set_phase(x);
+                w[c + 2] = recorded_value(x, wv);
+                st.steps(x, a, h, pre);
+            }
+        }
+        if (live) {
+            ns += (long long)pre * m;
+            scan_chunk(scan, w, q0, m, iters, sink);
+        }
+        w[0] = w[m];
+        w[1] = w[m + 1];
+    }
+    scan.last = w[1];
+    st.set_phase(x);
+    numb xPrev[UCB_NX];
+#pragma unroll
+    for (int j = 0; j < UCB_NX; ++j) xPrev[j] = x[j];
+    st.steps(x, a, h, pre);
+    if (!live) return 0;
+    ns += pre;
+    return fixed_point_flag(x, xPrev);
+}
+
+__device__ __forceinline__ int loop_transient(const ForcedStepper& st, numb* x, const numb* a, numb h, long long iters,
+                                              int pre, numb maxv, long long& ns, bool live) {
+    for (long long i0 = 0; i0 < iters; i0 += kCheckInterval) {
+        st.steps(x, a, h, 1);
+        if (live) {
+            ns += 1;
+            if (diverged(x, maxv)) live = false;
+        }
+        if (!__any_sync(0xFFFFFFFFu, live)) return 0;
+        const int n = (iters - i0 < kCheckInterval) ? (int)(iters - i0) : kCheckInterval;
+        st.steps(x, a, h, n - 1);
+        if (live) ns += n - 1;
+    }
+    numb xPrev[UCB_NX];
+#pragma unroll
+    for (int j = 0; j < UCB_NX; ++j) xPrev[j] = x[j];
+    st.steps(x, a, h, pre);
+    if (!live) return 0;
+    ns += pre;
+    return fixed_point_flag(x, xPrev);
+}
+#define UCB_CELL_STEPPER(h, x) \
+    __shared__ numb forced_tab[UCB_BLOCK / 32][kForced * kForcedEntry]; \
+    const ForcedStepper st(h, forced_tab[threadIdx.x >> 5], (x)[UCB_TRIG_PHASE], threadIdx.x & 31)
+#define UCB_RECORDS(flag) true  // the warp together
+#else
+#define UCB_CELL_STEPPER(h, x) const Stepper st(h)
+#define UCB_RECORDS(flag) ((flag) == 1 || (flag) == -1)
 template <class S, class Sink>
 __device__ __forceinline__ int loop_record(const S& st, numb* x, const numb* a, numb h, long long iters, int pre,
-                                           int wv, numb maxv, PeakScan& scan, const Sink& sink, long long& ns) {
+                                           int wv, numb maxv, PeakScan& scan, const Sink& sink, long long& ns,
+                                           bool /*live*/) {
     numb w[kScanChunk + 2];
 #pragma unroll
     for (int k = 0; k < kScanChunk + 2; ++k) w[k] = 0;
@@ -246,7 +328,7 @@ __device__ __forceinline__ int loop_record(const S& st, numb* x, const numb* a, 
 // Transient of calculateDiscreteModelCUDA: one step per iteration, preScaller extra steps.
 template <class S>
 __device__ __forceinline__ int loop_transient(const S& st, numb* x, const numb* a, numb h, long long iters, int pre,
-                                              numb maxv, long long& ns) {
+                                              numb maxv, long long& ns, bool /*live*/) {
     for (long long i0 = 0; i0 < iters; i0 += kCheckInterval) {
         const int n = (iters - i0 < kCheckInterval) ? (int)(iters - i0) : kCheckInterval;
         if (run_single<true>(st, x, a, h, n, maxv) == 0) {
@@ -262,15 +344,22 @@ __device__ __forceinline__ int loop_transient(const S& st, numb* x, const numb* 
     ns += pre;
     return fixed_point_flag(x, xPrev);
 }
+#endif
 
 }  // namespace ucbdev
 
 #if !defined(UCB_BIF2D) && !defined(UCB_BIF_NO_KERNELS)
 extern "C" __global__ void UCB_LAUNCH_BOUNDS ucb_bif_kernel(const UcbBifParams p) {
-    const long long cell = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    long long cell = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     long long ns = 0;
-    if (cell < p.n_pts) {
+    const bool live = cell < p.n_pts;
+#ifdef UCB_FORCED
+    if (!live) cell = p.n_pts - 1;  // its lane steps with the warp
+    {
+#else
+    if (live) {
+#endif
         numb x[UCB_NX], a[UCB_NV];
 #pragma unroll
         for (int i = 0; i < UCB_NX; ++i) x[i] = p.ic[i];
@@ -292,14 +381,16 @@ extern "C" __global__ void UCB_LAUNCH_BOUNDS ucb_bif_kernel(const UcbBifParams p
         if (!(h > 0)) {
             count = -1;
         } else {
-            const ucbdev::Stepper st(h);
-            int flag = ucbdev::loop_transient(st, x, a, h, skip, p.pre_scaller, p.maxv, ns);
-            if (flag == 1 || flag == -1) {
+            using namespace ucbdev;
+            UCB_CELL_STEPPER(h, x);
+            int flag = ucbdev::loop_transient(st, x, a, h, skip, p.pre_scaller, p.maxv, ns, live);
+            if (UCB_RECORDS(flag)) {
                 ucbdev::PeakScan scan;
                 scan.init();
                 const ucbdev::Bif1dSink sink{p.out_peaks + cell * p.max_out, p.out_intervals + cell * p.max_out,
                                              p.max_out, p.time_step};
-                flag = ucbdev::loop_record(st, x, a, h, iters, p.pre_scaller, p.writable_var, p.maxv, scan, sink, ns);
+                flag = ucbdev::loop_record(st, x, a, h, iters, p.pre_scaller, p.writable_var, p.maxv, scan, sink,
+                                           ns, flag != 0);
                 if (flag == 1) {
                     int n = (scan.found > 1) ? scan.found - 1 : 0;
                     if (n >= ucbdev::kMaxAmountOfPeaks) n = ucbdev::kMaxAmountOfPeaks;
@@ -311,7 +402,7 @@ extern "C" __global__ void UCB_LAUNCH_BOUNDS ucb_bif_kernel(const UcbBifParams p
                 count = flag;
             }
         }
-        p.out_counts[cell] = count;
+        if (live) p.out_counts[cell] = count;
     }
     ucbdev::warp_add_steps(p.steps, ns, lane);
 }
@@ -407,7 +498,8 @@ __device__ __noinline__ int bif2d_periods(char* rows, char* work, int cap, int c
 
 // Trajectory and peaks of one cell of a 2-D period map: the peak count (or the -1 / 0
 // trajectory flag), peaks in row[0, min(count, cap)).
-__device__ __forceinline__ int bif2d_peaks(const UcbBif2dParams& p, long long kidx, numb* row, long long& ns) {
+__device__ __forceinline__ int bif2d_peaks(const UcbBif2dParams& p, long long kidx, numb* row, long long& ns,
+                                           bool live) {
     const ucbdev::CellAxes c = ucbdev::cell_axes(kidx, p.n_pts);
     numb x[UCB_NX], a[UCB_NV];
 #pragma unroll
@@ -431,13 +523,14 @@ __device__ __forceinline__ int bif2d_peaks(const UcbBif2dParams& p, long long ki
     if (!(h > 0)) {
         count = -1;
     } else {
-        const ucbdev::Stepper st(h);
-        int flag = ucbdev::loop_transient(st, x, a, h, skip, p.pre_scaller, p.maxv, ns);
-        if (flag == 1 || flag == -1) {
+        UCB_CELL_STEPPER(h, x);
+        int flag = ucbdev::loop_transient(st, x, a, h, skip, p.pre_scaller, p.maxv, ns, live);
+        if (UCB_RECORDS(flag)) {
             ucbdev::PeakScan scan;
             scan.init();
             const ucbdev::Bif2dSink sink{row, p.cap};
-            flag = ucbdev::loop_record(st, x, a, h, iters, p.pre_scaller, p.writable_var, p.maxv, scan, sink, ns);
+            flag = ucbdev::loop_record(st, x, a, h, iters, p.pre_scaller, p.writable_var, p.maxv, scan, sink,
+                                       ns, flag != 0);
             if (flag == 1) {
                 int n = (scan.found > 1) ? scan.found - 1 : 0;
                 if (n >= ucbdev::kMaxAmountOfPeaks) n = ucbdev::kMaxAmountOfPeaks;
@@ -465,7 +558,12 @@ extern "C" __global__ void UCB_LAUNCH_BOUNDS ucb_bif2d_kernel(const UcbBif2dPara
         if (base >= p.total) break;
         const long long i = base + lane;
         numb* row = reinterpret_cast<numb*>(rows + (long long)lane * p.cap * 8);
-        const int count = i < p.total ? ucbdev::bif2d_peaks(p, i, row, ns) : 0;
+#ifdef UCB_FORCED
+        int count = ucbdev::bif2d_peaks(p, i < p.total ? i : p.total - 1, row, ns, i < p.total);
+        if (i >= p.total) count = 0;
+#else
+        const int count = i < p.total ? ucbdev::bif2d_peaks(p, i, row, ns, true) : 0;
+#endif
         __syncwarp();
         const int mine = ucbdev::bif2d_periods(rows, work, p.cap, count, p.eps, lane);
         if (i < p.total) {

@@ -241,27 +241,44 @@ struct Stepper {
 #endif
     }
 #ifdef UCB_KAHAN_CLOCK
-    // The clock after one step from xc (Kahan's compensated sum).
-    __device__ __forceinline__ numb clock_next(numb xc) const {
-        const numb y = hr - kc;
+    // The clock after one step from xc (Kahan's compensated sum, error c).
+    __device__ __forceinline__ numb clock_next(numb xc, numb& c) const {
+        const numb y = hr - c;
         const numb t = xc + y;
-        kc = (t - xc) - y;
+        c = (t - xc) - y;
         return t;
+    }
+    __device__ __forceinline__ numb clock_next(numb xc) const { return clock_next(xc, kc); }
+#endif
+#ifdef UCB_TRIG_PHASE
+    // (cos, sin) of the forcing at the three stage phases of a step that starts at phase ph
+    // (clock error kc).
+    __device__ __forceinline__ void stage_phases(numb ph, numb kc_, numb* tc) const {
+        numb s0, c0;
+        ucb_sincos(ph, &s0, &c0);
+#if defined(UCB_KAHAN_CLOCK) && UCB_CLOCK_VAR == UCB_TRIG_PHASE
+        {  // the forcing at the compensated phase x - kc (first order in kc <= half an ulp)
+            const numb cc = fma(kc_, s0, c0);
+            s0 = fma(-kc_, c0, s0);
+            c0 = cc;
+        }
+#endif
+        tc[0] = c0;
+        tc[1] = s0;
+        tc[2] = fma(c0, ch, -s0 * sh);
+        tc[3] = fma(s0, ch, c0 * sh);
+        tc[4] = fma(c0, cf, -s0 * sf);
+        tc[5] = fma(s0, cf, c0 * sf);
     }
 #endif
     __device__ __forceinline__ void step(numb* x, const numb* a, numb h) const {
 #ifdef UCB_TRIG_PHASE
-        numb s0, c0;
-        ucb_sincos(x[UCB_TRIG_PHASE], &s0, &c0);
-#if defined(UCB_KAHAN_CLOCK) && UCB_CLOCK_VAR == UCB_TRIG_PHASE
-        {  // the forcing at the compensated phase x - kc (first order in kc <= half an ulp)
-            const numb cc = fma(kc, s0, c0);
-            s0 = fma(-kc, c0, s0);
-            c0 = cc;
-        }
+        numb tc[6];
+#ifdef UCB_KAHAN_CLOCK
+        stage_phases(x[UCB_TRIG_PHASE], kc, tc);
+#else
+        stage_phases(x[UCB_TRIG_PHASE], (numb)0, tc);
 #endif
-        const numb tc[6] = {c0, s0, fma(c0, ch, -s0 * sh), fma(s0, ch, c0 * sh), fma(c0, cf, -s0 * sf),
-                            fma(s0, cf, c0 * sf)};
         step_trig(x, a, h, tc);
 #else
         numb k1[UCB_NX], k2[UCB_NX], k3[UCB_NX], k4[UCB_NX], xt[UCB_NX];
@@ -702,6 +719,88 @@ __device__ __forceinline__ void apply_sweep(const CellAxes& c, const numb* ax0, 
     a[UCB_IDX1] = ax1[c.i1];
 #endif
 }
+
+// A forcing phase that no axis sweeps runs through the same values in every cell.
+#if defined(UCB_TRIG_PHASE) && !defined(UCB_EXACT) && UCB_HAXIS == -1 &&                                      \
+    (UCB_POV == 1 || (UCB_IDX0 != UCB_TRIG_PHASE && (UCB_POV == 2 || UCB_DIM == 1 || UCB_IDX1 != UCB_TRIG_PHASE)))
+#define UCB_FORCED 1
+// Stepper whose warp evaluates that phase once for all its cells: lane l takes the phase l
+// steps ahead and writes the stage phases' (cos, sin) to the warp's table, so a step reads
+// three pairs (one broadcast) where it evaluated a sincos and two rotations, with the same
+// bits. Every lane of the warp has to take every step: the loops of ucb_bif.cuh keep a
+// finished cell's lane going until the whole warp is done. The component of the state
+// itself is not advanced (set_phase() gives it), unless the system reads it elsewhere.
+// B200, reference-method Duffing features 256^2, whole calls: FP32 73.1 -> 49.2 ms (350,000
+// steps a cell), FP64 23.9 -> 13.8 ms (47,700 steps a cell); FP64 100^2 14.3 -> 7.7 ms.
+#if UCB_UNROLL > 1
+#define UCB_FORCED_UNROLL UCB_UNROLL
+#else
+#define UCB_FORCED_UNROLL 4  // the next steps' loads ahead of this one's chain: 57.2 -> 54.7 ms
+#endif
+constexpr int kForced = 20;  // steps of a table; a divisor of kCheckInterval
+constexpr int kForcedEntry = 8;  // cos, sin of three stages, the phase, padding
+struct ForcedStepper : Stepper {
+    numb* tab;
+    int lane;
+    mutable int pos;
+    mutable numb ph, err;  // phase at the table's end and its clock error
+    __device__ __forceinline__ ForcedStepper(numb h, numb* tab_, numb ph0, int lane_)
+        : Stepper(h), tab(tab_), lane(lane_), pos(kForced), ph(ph0), err(0) {}
+    __device__ __forceinline__ void advance(const numb* x, const numb* a, numb& v, numb& e) const {
+#if defined(UCB_KAHAN_CLOCK) && UCB_CLOCK_VAR == UCB_TRIG_PHASE
+        v = clock_next(v, e);
+#else
+        numb k[UCB_NX];  // (its phase component is a constant)
+        ucb_rhs_trig(x, a, k, (numb)1, (numb)0);
+        const numb r = k[UCB_TRIG_PHASE];
+        v = fma(h6, (r + r) + (numb)2 * (r + r), v);
+#endif
+    }
+    __device__ __forceinline__ void fill(const numb* x, const numb* a) const {
+        numb v = ph, e = err;
+#pragma unroll
+        for (int l = 0; l < kForced - 1; ++l)
+            if (l < lane) advance(x, a, v, e);
+        numb tc[6];
+        stage_phases(v, e, tc);
+        __syncwarp();
+        if (lane < kForced) {
+            numb* t = tab + lane * kForcedEntry;
+#pragma unroll
+            for (int j = 0; j < 6; ++j) t[j] = tc[j];
+            t[6] = v;
+        }
+        advance(x, a, v, e);
+        ph = __shfl_sync(0xFFFFFFFFu, v, kForced - 1);
+        err = __shfl_sync(0xFFFFFFFFu, e, kForced - 1);
+        __syncwarp();
+        pos = 0;
+    }
+    __device__ __forceinline__ void set_phase(numb* x) const {
+        x[UCB_TRIG_PHASE] = pos < kForced ? tab[pos * kForcedEntry + 6] : ph;
+    }
+    // n steps, before(i) ahead of step i; the state's phase component is left stale.
+    template <class F>
+    __device__ __forceinline__ void steps(numb* x, const numb* a, numb h, int n, const F& before) const {
+        for (int done = 0; done < n;) {
+            if (pos == kForced) fill(x, a);
+            const int m = n - done < kForced - pos ? n - done : kForced - pos;
+            const numb* t = tab + pos * kForcedEntry;
+            UCB_PRAGMA_(unroll UCB_FORCED_UNROLL)
+            for (int i = 0; i < m; ++i) {
+                before(done + i);
+                step_trig(x, a, h, t + i * kForcedEntry);
+            }
+            pos += m;
+            done += m;
+        }
+    }
+    __device__ __forceinline__ void steps(numb* x, const numb* a, numb h, int n) const {
+        steps(x, a, h, n, [](int) {});
+        set_phase(x);
+    }
+};
+#endif
 
 // Adds the per-thread work counts of a warp into a global counter (one atomic per warp).
 __device__ __forceinline__ void warp_add_steps(unsigned long long* counter, long long ns, int lane) {
