@@ -182,10 +182,19 @@ __device__ __forceinline__ int sample_chunk(const S& st, numb* x, const numb* a,
         if (diverged(x, maxv)) return 0;
         c = 1;
     }
+    if (pre == 1) {
+        // by fours, so that the next samples' selects and stores fall into the steps' latencies
+        // (Lorenz diagram, kernel: FP64 3.11 -> 2.66 ms, FP32 2.59 -> 2.13 ms; period maps 1-5 %)
+#pragma unroll 4
+        for (; c < m; ++c) {
+            w[c + 2] = recorded_value(x, wv);
+            st.step(x, a, h);
+        }
+        return 1;
+    }
     for (; c < m; ++c) {
         w[c + 2] = recorded_value(x, wv);
-        st.step(x, a, h);
-        for (int j = 1; j < pre; ++j) st.step(x, a, h);
+        for (int j = 0; j < pre; ++j) st.step(x, a, h);
     }
     return 1;
 }
