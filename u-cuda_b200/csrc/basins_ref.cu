@@ -802,7 +802,6 @@ extern "C" int ucb_run_basins_dbscan(ucb_engine* e, const ucb_basins_dbscan_requ
     pk.put<void*>(ws);
     pk.put<void*>(ws + 8);
     EventPair cev;
-    begin_run(e);
     cudaEventRecord(e->ev0, st);
     if (!launch_packed(e, fn, persistent_grid(e, fn, shape.block, total), shape.block, st, pk, err))
         return fail(e, res, UCB_E_CUDA, err);

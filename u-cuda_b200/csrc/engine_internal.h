@@ -27,12 +27,12 @@ struct TuneConfig {
 };
 }  // namespace ucb
 
-// Host view of the run-control block the kernels poll (kernels/ucb_device.cuh UcbControl):
-// page-locked host memory mapped into the device's address space.
+// Page-locked staging of the run control (kernels/ucb_device.cuh UcbControl lives in device
+// memory): the cancel word on its way to the device, the queue position on its way back.
 struct ucb_run_control {
-    volatile int32_t cancel;
+    int32_t cancel;
     int32_t pad;
-    volatile unsigned long long fetched;
+    unsigned long long fetched;
 };
 
 struct ucb_engine {
@@ -61,8 +61,12 @@ struct ucb_engine {
     // and launch shape as resolved at prepare time, by kernel-build key (an autotune after
     // the prepare does not change what the allocation-free call launches).
     std::map<std::string, std::shared_ptr<void>> pinned_lle;
-    // Run control of the host-buffer entry points (null when mapped memory is unavailable).
+    // Run control of the host-buffer entry points (null when it could not be set up): the
+    // staging, the block the kernels poll, and the stream that moves words between the two
+    // while a kernel runs.
     ucb_run_control* control = nullptr;
+    void* control_dev = nullptr;
+    cudaStream_t control_stream = nullptr;
 };
 
 namespace ucb {
@@ -196,14 +200,13 @@ ucb_lle2d_request as_lle2d(const ucb_lle1d_request& q);
 // Launch helper: persistent grid size for a kernel.
 int persistent_grid(ucb_engine* e, CUfunction f, int block, long long work_items);
 
-// Run control of the host-buffer entry points (ucb_run_*). begin_run resets the queue
-// position before a launch. wait_run waits for `done` (an event recorded after the run's
-// main kernel); while it waits it mirrors the caller's *cancel into the control block (the
-// kernels' warps then take no more cells and an adaptive cell abandons its steps) and
-// writes the queue position / work_items to *progress. Without cancel and progress words
-// it simply synchronises. Returns UCB_OK, UCB_E_CANCELLED (the control block is clear
-// again once the kernel has ended) or UCB_E_CUDA.
-void begin_run(ucb_engine* e);
+// Run control of the host-buffer entry points (ucb_run_*). wait_run waits for `done` (an
+// event recorded after the run's main kernel, whose work counter is the workspace's first
+// word); while it waits it mirrors the caller's *cancel into the control block (the kernels'
+// warps then take no more cells and an adaptive cell abandons its steps) and writes the
+// queue position / work_items to *progress. Without cancel and progress words it simply
+// synchronises. Returns UCB_OK, UCB_E_CANCELLED (the control block is clear again once the
+// kernel has ended) or UCB_E_CUDA.
 int wait_run(ucb_engine* e, cudaEvent_t done, const volatile int32_t* cancel, volatile float* progress,
              long long work_items, std::string& err);
 

@@ -229,7 +229,6 @@ extern "C" int ucb_run_bif2d(ucb_engine* e, const ucb_bif2d_request* req, ucb_bi
     pk.put<void*>(d_flags);
     pk.put<void*>(ws);
     pk.put<void*>(ws + 8);
-    begin_run(e);
     cudaEventRecord(e->ev0, e->stream);
     if (!launch_packed(e, fn, grid, block, e->stream, pk, err)) rc = UCB_E_CUDA;
     cudaEventRecord(e->ev1, e->stream);

@@ -81,16 +81,20 @@ bool ensure_init(ucb_engine* e, std::string& err) {
         return false;
     }
     {
-        // run control: cancel word and queue position shared with the kernels
+        // run control: the cancel word the kernels poll, in device memory (a poll of mapped
+        // host memory crossed PCIe at every fetch of the work queue)
         void* h = nullptr;
         void* dptr = nullptr;
-        if (cudaHostAlloc(&h, sizeof(ucb_run_control), cudaHostAllocMapped) == cudaSuccess &&
-            cudaHostGetDevicePointer(&dptr, h, 0) == cudaSuccess) {
+        if (cudaHostAlloc(&h, sizeof(ucb_run_control), cudaHostAllocDefault) == cudaSuccess &&
+            cudaMalloc(&dptr, 256) == cudaSuccess && cudaMemset(dptr, 0, 256) == cudaSuccess &&
+            cudaStreamCreateWithFlags(&e->control_stream, cudaStreamNonBlocking) == cudaSuccess) {
             std::memset(h, 0, sizeof(ucb_run_control));
             e->control = static_cast<ucb_run_control*>(h);
+            e->control_dev = dptr;
             e->modules.set_control(dptr);
         } else {
             if (h) cudaFreeHost(h);
+            if (dptr) cudaFree(dptr);
             cudaGetLastError();
         }
     }
@@ -98,8 +102,11 @@ bool ensure_init(ucb_engine* e, std::string& err) {
     return true;
 }
 
-void begin_run(ucb_engine* e) {
-    if (e->control) e->control->fetched = 0;
+// Writes the cancel word the kernels poll.
+static void set_cancel(ucb_engine* e, int32_t v) {
+    e->control->cancel = v;
+    cudaMemcpyAsync(e->control_dev, &e->control->cancel, sizeof(int32_t), cudaMemcpyHostToDevice, e->control_stream);
+    cudaStreamSynchronize(e->control_stream);
 }
 
 int wait_run(ucb_engine* e, cudaEvent_t done, const volatile int32_t* cancel, volatile float* progress,
@@ -120,14 +127,17 @@ int wait_run(ucb_engine* e, cudaEvent_t done, const volatile int32_t* cancel, vo
         if (ce == cudaSuccess) break;
         if (ce != cudaErrorNotReady) {
             err = std::string("CUDA: ") + cudaGetErrorString(ce);
-            if (cancelled) c->cancel = 0;
+            if (cancelled) set_cancel(e, 0);
             return UCB_E_CUDA;
         }
         if (cancel && *cancel && !cancelled) {
-            c->cancel = 1;
+            set_cancel(e, 1);
             cancelled = true;
         }
-        if (progress && work_items > 0) {
+        if (progress && work_items > 0 &&
+            cudaMemcpyAsync(&c->fetched, e->ws, sizeof(c->fetched), cudaMemcpyDeviceToHost, e->control_stream) ==
+                cudaSuccess &&
+            cudaStreamSynchronize(e->control_stream) == cudaSuccess) {
             const double f = (double)c->fetched / (double)work_items;
             *progress = (float)std::min(f, 0.999);
         }
@@ -137,7 +147,7 @@ int wait_run(ucb_engine* e, cudaEvent_t done, const volatile int32_t* cancel, vo
             std::this_thread::sleep_for(std::chrono::microseconds(200));
     }
     if (cancelled) {
-        c->cancel = 0;
+        set_cancel(e, 0);
         err = "Cancelled by user";
         return UCB_E_CANCELLED;
     }
@@ -836,6 +846,8 @@ void ucb_destroy(ucb_engine* e) {
         if (e->pool) cudaMemPoolDestroy(e->pool);
         e->pinned_lle.clear();
         if (e->control) cudaFreeHost(e->control);
+        if (e->control_dev) cudaFree(e->control_dev);
+        if (e->control_stream) cudaStreamDestroy(e->control_stream);
     }
     delete e;
 }
@@ -889,7 +901,6 @@ int ucb_run_lle2d(ucb_engine* e, const ucb_lle2d_request* req, ucb_lle2d_result*
     if ((ce = dev_alloc(e, (void**)&d_values, total * sizeof(double), e->stream)) != cudaSuccess ||
         (ce = dev_alloc(e, (void**)&d_flags, total * sizeof(int32_t), e->stream)) != cudaSuccess)
         return fail(e, res->error, &res->ok, UCB_E_CUDA, std::string("cudaMallocAsync: ") + cudaGetErrorString(ce));
-    begin_run(e);
     cudaEventRecord(e->ev0, e->stream);
     int rc = enqueue_lle(e, q, plan, L, d_values, d_flags, e->stream, err);
     cudaEventRecord(e->ev1, e->stream);
@@ -977,7 +988,6 @@ int ucb_run_lle1d(ucb_engine* e, const ucb_lle1d_request* req, ucb_lle1d_result*
     if ((ce = dev_alloc(e, (void**)&d_values, (size_t)n * sizeof(double), e->stream)) != cudaSuccess ||
         (ce = dev_alloc(e, (void**)&d_flags, (size_t)n * sizeof(int32_t), e->stream)) != cudaSuccess)
         return fail(e, res->error, &res->ok, UCB_E_CUDA, std::string("cudaMallocAsync: ") + cudaGetErrorString(ce));
-    begin_run(e);
     cudaEventRecord(e->ev0, e->stream);
     int rc = enqueue_lle(e, q, plan, L, d_values, d_flags, e->stream, err);
     cudaEventRecord(e->ev1, e->stream);
