@@ -522,6 +522,23 @@ __device__ __forceinline__ int block_pair_nt(const S& s, numb* x, numb* y, const
 }
 #endif
 
+#ifdef UCB_NT
+// The same block of one trajectory (the other one in another lane): half the code.
+#if !defined(UCB_EXACT)
+#define UCB_NT_SPLIT_UNROLL UCB_NT
+#else
+#define UCB_NT_SPLIT_UNROLL 2
+#endif
+template <class S>
+__device__ __forceinline__ int block_nt(const S& s, numb* x, const numb* a, numb h, numb maxValue) {
+    s.step(x, a, h);
+    if (diverged(x, maxValue)) return 0;
+    UCB_PRAGMA_(unroll UCB_NT_SPLIT_UNROLL)
+    for (int i = 1; i < UCB_NT + UCB_EXTRA_STEP; ++i) s.step(x, a, h);
+    return 1;
+}
+#endif
+
 #ifdef UCB_SIXTH
 // Blocks taken again with the division. The state at the start of the block waits in local
 // memory (the arrays these calls take), not in registers.
@@ -558,6 +575,20 @@ __device__ __forceinline__ int run_single(const Stepper& s, numb* x, const numb*
     }
     return r;
 }
+#ifdef UCB_NT
+__device__ __forceinline__ int run_nt(const Stepper& s, numb* x, const numb* a, numb h, numb maxValue) {
+    numb keep[UCB_NX];
+    copy_state<UCB_NX>(x, keep);
+    int r = s.verbatim ? 0 : block_nt(s, x, a, h, maxValue);
+    if (s.failed()) {
+        numb av[UCB_NV];
+        copy_values(a, av);
+        r = redo_single<true>(keep, av, h, UCB_NT + UCB_EXTRA_STEP, maxValue);
+        copy_state<UCB_NX>(keep, x);
+    }
+    return r;
+}
+#endif
 __device__ __forceinline__ int finish_pair(const Stepper& s, int r, numb* keep, numb* x, numb* y, const numb* a,
                                            numb h, int n, numb maxValue, bool whole_nt) {
     if (s.failed()) {
@@ -596,6 +627,10 @@ __device__ __forceinline__ int run_pair(const S& s, numb* x, numb* y, const numb
     return block_pair(s, x, y, a, h, n, maxValue);
 }
 #ifdef UCB_NT
+template <class S>
+__device__ __forceinline__ int run_nt(const S& s, numb* x, const numb* a, numb h, numb maxValue) {
+    return block_nt(s, x, a, h, maxValue);
+}
 template <class S>
 __device__ __forceinline__ int run_pair_nt(const S& s, numb* x, numb* y, const numb* a, numb h, numb maxValue) {
     return block_pair_nt(s, x, y, a, h, maxValue);

@@ -500,6 +500,7 @@ std::vector<char> pack_lle_params(const LleParamsT<T>& head, const double* ic, i
 struct LleLaunch {
     std::shared_ptr<Module> mod;
     CUfunction fn = nullptr;
+    CUfunction split = nullptr;  // shadow form, two lanes a cell (null: not in this build)
     SystemCode sys;
     bool tangent = false;
     TuneConfig shape;  // launch shape (block size used by the launch)
@@ -534,6 +535,7 @@ CompileRequest lle_compile_request(const ucb_lle2d_request& q, const LlePlan& pl
     rq.headers = device_headers();
     rq.options.push_back(L.sys.exact ? "--fmad=false" : "--fmad=true");
     rq.kernels = {"ucb_lle_kernel", "ucb_state_kernel"};
+    if (!tangent && plan.map.h_axis == -1) rq.kernels.insert(rq.kernels.begin(), "ucb_lle_split_kernel");
     return rq;
 }
 
@@ -545,13 +547,32 @@ bool lle_tuned_request(ucb_engine* e, const ucb_lle2d_request& q, const LlePlan&
     return tune_request(e, q.opt, 128, rq, L.shape, err);
 }
 
+// The kernels of a loaded LLE module.
+void bind_lle(LleLaunch& L) {
+    L.fn = L.mod->functions["ucb_lle_kernel"];
+    const auto it = L.mod->functions.find("ucb_lle_split_kernel");
+    L.split = it != L.mod->functions.end() ? it->second : nullptr;
+}
+
 bool prepare_lle(ucb_engine* e, const ucb_lle2d_request& q, const LlePlan& plan, LleLaunch& L, std::string& err) {
     CompileRequest rq;
     if (!lle_tuned_request(e, q, plan, L, rq, err)) return false;
     L.mod = e->modules.get(rq, err);
     if (!L.mod) return false;
-    L.fn = L.mod->functions["ucb_lle_kernel"];
+    bind_lle(L);
     return true;
+}
+
+// Whether a shadow map of `cells` cells runs with a trajectory a lane (ucb_lle_split_kernel):
+// while its warps (16 cells each) have a scheduler of their own. A step then waits for one
+// trajectory's chain; with a second warp on a scheduler the two forms issue the same
+// instructions, and the pair form takes the transient and the renormalisation once a cell.
+// The verbatim step waits longer for its chain, which two warps still share.
+// B200, pair / split, Chen maps: native FP64 96^2 0.87 / 0.63 ms, 100^2 (two warps on some
+// schedulers) 0.87 / 0.90, 300^2 3.6 / 4.2; exact FP64 90^2 1.69 / 0.97, 137^2 1.70 / 1.53,
+// 170^2 2.71 / 2.95; exact FP32 137^2 1.75 / 1.36, 170^2 2.37 / 2.60.
+bool split_pays(const ucb_engine* e, const LleLaunch& L, long long cells) {
+    return cells <= 16LL * (L.sys.exact ? 2 : 1) * 4 * e->sm_count;
 }
 
 // Enqueues the LLE kernel. Workspace layout: [0] work counter, [8] step counter,
@@ -610,11 +631,14 @@ int enqueue_lle_fn(ucb_engine* e, const ucb_lle2d_request& q, const LlePlan& pla
                                          list_compact ? 1 : 0);
     }
     const int block = L.shape.block;
-    const int grid = persistent ? persistent_grid(e, L.fn, block, total) : (int)((total + block - 1) / block);
+    const bool split = persistent && L.split && split_pays(e, L, total);
+    const CUfunction fn = split ? L.split : L.fn;
+    const int grid = persistent ? persistent_grid(e, fn, block, split ? 2 * total : total)
+                                : (int)((total + block - 1) / block);
     size_t psize = params.size();
     void* cfg[] = {CU_LAUNCH_PARAM_BUFFER_POINTER, params.data(), CU_LAUNCH_PARAM_BUFFER_SIZE, &psize,
                    CU_LAUNCH_PARAM_END};
-    CUresult r = driver().cuLaunchKernel(L.fn, grid, 1, 1, block, 1, 1, 0, (CUstream)stream, nullptr, cfg);
+    CUresult r = driver().cuLaunchKernel(fn, grid, 1, 1, block, 1, 1, 0, (CUstream)stream, nullptr, cfg);
     if (r != CUDA_SUCCESS) {
         err = "cuLaunchKernel(lle2d): " + cu_error_string(r);
         return UCB_E_CUDA;
@@ -746,7 +770,7 @@ int lle2d_plan_and_find(ucb_engine* e, const ucb_lle2d_request& q, bool load_if_
         delete L;
         return load_if_missing ? UCB_E_COMPILE : UCB_E_INVALID;
     }
-    L->fn = L->mod->functions["ucb_lle_kernel"];
+    bind_lle(*L);
     *plan_out = plan;
     *launch_out = L;
     return UCB_OK;
@@ -762,7 +786,7 @@ int lle2d_pin(ucb_engine* e, const ucb_lle2d_request& q, std::string& err) {
     if (!tune_request(e, q.opt, 128, rq, L->shape, err)) return UCB_E_INVALID;
     L->mod = e->modules.get(rq, err);
     if (!L->mod) return UCB_E_COMPILE;
-    L->fn = L->mod->functions["ucb_lle_kernel"];
+    bind_lle(*L);
     e->pinned_lle[key] = L;
     return UCB_OK;
 }
