@@ -43,6 +43,7 @@ struct UcbLsParams {
     unsigned long long* counter;
     unsigned long long* steps;
     long long* out_cell_steps;  // per cell: steps (fixed) / step attempts (DP5); may be null
+    int groups;                 // cells a warp at a time (UCB_LS_GROUP)
 };
 
 namespace ucbdev {
@@ -710,6 +711,220 @@ __device__ __forceinline__ void ls_cell_dp5(const UcbLsParams& p, long long kidx
     for (int k = 0; k < UCB_NX; ++k) outv[k] = ok ? acc[k] / p.t_end : 999.0;
     ls_store(p, kidx, outv);
 }
+
+#if defined(UCB_LS_GROUP)
+// ls_cell_dp5 with a cell on UCB_NX lanes, one tangent vector each (the same values and order of
+// operations): every lane of a group takes the state's step and its own vector's, the error
+// sums and Gram-Schmidt rows are exchanged by shuffles. An attempt is then two chains of
+// stages instead of N + 1 and its registers fall from 254 to 204 (FP64), so a map of few cells,
+// which lasts as long as its slowest ones, ends sooner; a group takes its next cell as soon as
+// it is done. The exchanges are taken by the whole warp; what a group does between them
+// depends on values that all its lanes hold. (The tangent's stages beside the state's, before
+// its step is accepted, gave the same times.) B200, 96^2 hyper-chaotic Rossler, t_end 50, FP64:
+// 68 -> 46 ms; where each form runs and its times: dp5_groups of ucb_ls.cpp.
+// mgs() over the group's rows (lane k holds row k), for groups with `act`; the log of the
+// norms added to acc. False if the group's rows are not independent and finite.
+__device__ __forceinline__ bool group_mgs(numb* v, double& acc, bool act, int k, int base, unsigned int group) {
+    double norm = 1.0;
+    bool good = true;
+#pragma unroll
+    for (int j = 0; j < UCB_NX; ++j) {
+        if (act && k == j) {
+            double n2 = 0;
+#pragma unroll
+            for (int l = 0; l < UCB_NX; ++l) n2 = fma((double)v[l], (double)v[l], n2);
+            norm = sqrt(n2);
+            good = norm > 0 && isfinite(norm);
+            const numb inv = (numb)(1.0 / norm);
+#pragma unroll
+            for (int l = 0; l < UCB_NX; ++l) v[l] *= inv;
+        }
+        __syncwarp();
+        numb w[UCB_NX];
+#pragma unroll
+        for (int l = 0; l < UCB_NX; ++l) w[l] = __shfl_sync(0xFFFFFFFFu, v[l], base + j);
+        if (act && k > j) {
+            double d = 0;
+#pragma unroll
+            for (int l = 0; l < UCB_NX; ++l) d = fma((double)v[l], (double)w[l], d);
+            const numb dn = (numb)d;
+#pragma unroll
+            for (int l = 0; l < UCB_NX; ++l) v[l] = fma(-dn, w[l], v[l]);
+        }
+    }
+    const unsigned int ok = __ballot_sync(0xFFFFFFFFu, good);
+    if (act) acc += log(norm);
+    return (ok & group) == group;
+}
+
+__device__ __forceinline__ void ls_groups_dp5(const UcbLsParams& p, long long& ns) {
+    const unsigned int full = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    const bool member = lane < p.groups * UCB_NX;
+    const int k = member ? lane % UCB_NX : 0, base = lane - k;
+    const unsigned int group = member ? ((1u << UCB_NX) - 1u) << base : 0u;
+    // the group's cell, the same in all its lanes but for the vector and its log sum
+    Dp5State S;
+    numb a[UCB_NV], v[UCB_NX];
+    double acc = 0, t = 0, h = 0, facmax = 5.0, t_gs = 0, t_meas = 0, spread = 0, clock0 = 0;
+    long long kidx = 0, attempts = 0, accepted = 0, cell_ns = 0;
+    int since_gs = 0;
+    bool busy = false, drained = !member, measuring = false, ok = true;
+    const double t_stop = (double)p.transient + p.t_end;
+#pragma unroll
+    for (int i = 0; i < UCB_NX; ++i) v[i] = 0;
+    for (;;) {
+        const bool need = !busy && !drained;
+        const unsigned int asking = __ballot_sync(full, need && k == 0);
+        if (asking) {
+            unsigned long long first = 0;
+            if (lane == 0) {
+                const bool stop = run_cancelled();
+                first = atomicAdd(p.counter, (unsigned long long)__popc(asking));
+                if (stop) first = 0x7fffffffffffffffULL;
+            }
+            first = __shfl_sync(full, first, 0);
+            const unsigned long long i = first + __popc(asking & ((1u << base) - 1u));
+            bool fresh = false;
+            if (need) {
+                if (i >= (unsigned long long)p.total) {
+                    drained = true;
+                } else {
+                    fresh = busy = true;
+                    kidx = p.cell_offset + (long long)i;
+                    const CellAxes c = cell_axes(kidx, p.n_pts);
+#pragma unroll
+                    for (int j = 0; j < UCB_NX; ++j) S.X[0][j] = p.ic[j];
+#pragma unroll
+                    for (int j = 0; j < UCB_NV; ++j) a[j] = p.vals[j];
+                    apply_sweep(c, p.axis0, p.axis1, S.X[0], a);
+#ifdef UCB_KAHAN_CLOCK
+                    clock0 = (double)S.X[0][UCB_CLOCK_VAR];
+#endif
+                    Rng st;
+                    rng_init(1234567891ULL, (unsigned long long)kidx, 0ULL, &st);
+#pragma unroll
+                    for (int j = 0; j < UCB_NX; ++j)
+#pragma unroll
+                        for (int l = 0; l < UCB_NX; ++l) {
+                            const numb u = rng_uniform(&st) - 0.5;
+                            if (j == k) v[l] = u;
+                        }
+                    acc = t = t_gs = t_meas = 0.0;
+                    spread = 1e300;
+                    h = p.h0;
+                    facmax = 5.0;
+                    attempts = accepted = cell_ns = 0;
+                    since_gs = 0;
+                    measuring = !((double)p.transient > 0);
+                    ucb_rhs(S.X[0], a, S.k1);
+                }
+            }
+            double junk = 0;
+            const bool good = group_mgs(v, junk, fresh, k, base, group);
+            if (fresh) ok = good;
+        }
+        if (!__any_sync(full, busy)) break;
+        // a cell can take millions of attempts: a cancelled run abandons it
+        if (__any_sync(full, busy && (attempts & 4095) == 4095)) {
+            const int stop = __shfl_sync(full, (int)run_cancelled(), 0);
+            if (stop && (attempts & 4095) == 4095) ok = false;
+        }
+        // one attempt of every group that goes on
+        bool tried = false, tangent = false, last = false;
+        double ex2 = 0, err2 = 0, e_own = 0, t_target = 0;
+        numb vn[UCB_NX];
+        if (busy && ok && t < t_stop) {
+            if (++attempts > p.max_steps) {
+                ok = false;
+            } else {
+                tried = true;
+                t_target = measuring ? t_stop : (double)p.transient;
+                if (t + h >= t_target) { h = t_target - t; last = true; }
+                const Dp5Coef cf = dp5_coef((numb)h, h);
+                ex2 = dp5_state_step(S, a, cf, p.rtol, p.atol);
+                cell_ns += 1;
+                // err^2: the mean of the squared scaled errors (the RMS norm, squared)
+                err2 = ex2 * (1.0 / UCB_NX);
+                tangent = err2 <= 1.0 && measuring;
+                if (tangent) e_own = dp5_tangent_step(S, a, cf, p.rtol, p.atol, v, vn);
+            }
+        }
+        if (__any_sync(full, tangent)) {
+            double ev2 = 0;
+#pragma unroll
+            for (int j = 0; j < UCB_NX; ++j) ev2 += __shfl_sync(full, e_own, base + j);
+            if (tangent) err2 = (ex2 + ev2) * (1.0 / (UCB_NX + UCB_NX * UCB_NX));
+        }
+        bool gs = false;
+        if (tried) {
+            if (!isfinite(err2)) {
+                ok = false;
+            } else if (err2 <= 1.0) {
+                if (measuring) {
+#pragma unroll
+                    for (int i = 0; i < UCB_NX; ++i) v[i] = vn[i];
+                }
+                const double t_new = last ? t_target : t + h;
+                if (measuring) t_gs += t_new - t;
+                t = t_new;
+#pragma unroll
+                for (int i = 0; i < UCB_NX; ++i) { S.X[0][i] = S.xn[i]; S.k1[i] = S.k7[i]; }
+#ifdef UCB_KAHAN_CLOCK
+                S.X[0][UCB_CLOCK_VAR] = (numb)fma((double)UCB_CLOCK_RATE, t, clock0);
+#endif
+                if (diverged(S.X[0], p.maxv)) {
+                    ok = false;
+                } else if ((++accepted & 15) == 0 &&
+                           t_stop - t > kEscapeFactor * h * (double)(p.max_steps - attempts)) {
+                    ok = false;  // the escape test of ls_cell_dp5
+                } else {
+                    gs = measuring && (++since_gs >= p.gs_every || last || t_gs * spread > UCB_GS_BUDGET);
+                    if (last && !measuring) measuring = true;
+                    const double fac = (err2 > 0) ? dp5_factor(err2) : facmax;
+                    h *= fmin(facmax, fmax(0.2, fac));
+                    facmax = 5.0;
+                }
+            } else {
+                h *= fmax(0.2, dp5_factor(err2));
+                facmax = 2.0;
+                if (!(h > 1e-14)) ok = false;
+            }
+        }
+        if (__any_sync(full, gs)) {
+            const bool good = group_mgs(v, acc, gs, k, base, group);
+            const double a0 = __shfl_sync(full, acc, base), an = __shfl_sync(full, acc, base + UCB_NX - 1);
+            if (gs) {
+                ok = good;
+                since_gs = 0;
+                t_meas += t_gs;
+                t_gs = 0.0;
+                spread = fmax(0.0, (a0 - an) / t_meas);
+            }
+        }
+        const bool done = busy && (!ok || !(t < t_stop));
+        if (__any_sync(full, done)) {
+            const double out = ok ? acc / p.t_end : 999.0;
+            const unsigned int bad = __ballot_sync(full, done && (out == 999.0 || out == -999.0));
+            if (done) {
+                const long long cell = ls_out_cell(p, kidx);
+#if UCB_DIM == 2
+                const long long plane = (long long)p.n_pts * p.n_pts;
+#else
+                const long long plane = p.n_pts;
+#endif
+                p.out_values[k * plane + cell] = out;
+                if (k == 0) {
+                    p.out_flags[cell] = (bad & group) ? -1 : 1;
+                    if (p.out_cell_steps) p.out_cell_steps[cell] = cell_ns;
+                    ns += cell_ns;
+                }
+                busy = false;
+            }
+        }
+    }
+}
+#endif  // UCB_LS_GROUP
 #endif  // UCB_LS_DP5
 
 }  // namespace ucbdev
@@ -717,6 +932,11 @@ __device__ __forceinline__ void ls_cell_dp5(const UcbLsParams& p, long long kidx
 extern "C" __global__ void UCB_LAUNCH_BOUNDS ucb_ls_kernel(const UcbLsParams p) {
     const int lane = threadIdx.x & 31;
     long long ns = 0;
+#if defined(UCB_LS_GROUP)
+    ucbdev::ls_groups_dp5(p, ns);
+    ucbdev::warp_add_steps(p.steps, ns, lane);
+    return;
+#endif
     for (;;) {
         const long long base = ucbdev::warp_fetch(p.counter, lane);
         if (base >= p.total) break;

@@ -52,6 +52,23 @@ ucb_lle2d_request as_lle(const ucb_ls2d_request& q) {
     return l;
 }
 
+// Cells a warp holds at a time when the adaptive method runs with a cell on amount_of_x lanes
+// (ls_groups_dp5); 0: a cell a lane. Groups cut an attempt's latency, lanes its instructions
+// (the state's step is taken once a cell), so groups run while the map has few warps for the
+// B200's 592 schedulers: measured with 4 variables over the wide hyper-chaotic Rossler window
+// (t_end 50, 20,000 attempts; lanes / groups), FP64 16^2 65 / 27 ms, 64^2 66 / 37, 96^2 68 / 46,
+// 120^2 69 / 64, 192^2 98 / 130; FP32 64^2 69 / 36, 128^2 71 / 45, 256^2 98 / 82, 384^2 131 / 151.
+// Fewer groups a warp leave it fewer attempts that wait for a neighbour's Gram-Schmidt, while
+// schedulers are to spare: 16^2 with 1 / 8 groups 27 / 34 ms, 48^2 with 4 / 8 32.5 / 36.7.
+int dp5_groups(const ucb_ls2d_request& q) {
+    constexpr long long kSchedulers = 4 * 148;
+    const int nx = q.amount_of_x;
+    const long long cells = (long long)q.n_pts * q.n_pts;
+    if (q.method != UCB_LS_DP5 || nx < 2 || nx > 8) return 0;
+    if (cells > (q.opt.precision == UCB_PREC_F64 ? 24 : 128) * kSchedulers) return 0;
+    return (int)std::min<long long>((cells + kSchedulers - 1) / kSchedulers, 32 / nx);
+}
+
 CompileRequest ls_compile_request(const ucb_ls2d_request& q, const SweepMap& m, SystemCode& sys) {
     const bool dp5 = q.method == UCB_LS_DP5;
     const int prec = q.opt.precision;
@@ -67,6 +84,7 @@ CompileRequest ls_compile_request(const ucb_ls2d_request& q, const SweepMap& m, 
     std::vector<std::string> defs = dp5 ? clock_defines(sys) : std::vector<std::string>{};
     defs.push_back(dp5 ? "UCB_LS_DP5 1" : "UCB_LS_FIXED 1");
     if (tangent && sys.has_jvp) defs.push_back("UCB_LS_TANGENT 1");
+    if (dp5_groups(q)) defs.push_back("UCB_LS_GROUP 1");
     defs.push_back(prec == UCB_PREC_F64 ? "UCB_GS_BUDGET 20.0" : "UCB_GS_BUDGET 8.0");
     rq.source = make_prelude(prec, q.amount_of_x, q.n_values, m, q.opt.nominal_steps == 0, sys, defs) +
                 "#include \"ucb_device.cuh\"\n#include \"ucb_ls.cuh\"\n";
@@ -192,8 +210,10 @@ int ls_run(ucb_engine* e, const ucb_ls2d_request& q, const SweepMap& m, int n_bl
     pk.put<void*>(ws);
     pk.put<void*>(ws + 8);
     pk.put<void*>(d_cell_steps);
+    const int groups = dp5_groups(q);
+    pk.put<int>(groups);
     const int block = shape.block;
-    const int grid = persistent_grid(e, fn, block, total);
+    const int grid = persistent_grid(e, fn, block, groups ? (total + groups - 1) / groups * 32 : total);
     cudaEventRecord(e->ev0, e->stream);
     int rc = launch_packed(e, fn, grid, block, e->stream, pk, err) ? UCB_OK : UCB_E_CUDA;
     cudaEventRecord(e->ev1, e->stream);
