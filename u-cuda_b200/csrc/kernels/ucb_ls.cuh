@@ -181,13 +181,14 @@ __device__ __forceinline__ int loop_probes(const S& s, numb* x, numb (*y)[UCB_NX
 // trajectories x + eps z, whose differences from x fall below FP32 resolution for small eps,
 // the N tangent vectors v' = J(x) v are advanced with x in one RK4 sweep (the stage sums
 // accumulated stage by stage), and the block's Gram-Schmidt, norms and log sums are FP64.
+template <int M>
 __device__ __forceinline__ void ls_tangent_step(numb* x, numb (*V)[UCB_NX], const numb* a, numb h) {
     const numb hh = h * (numb)0.5, h6 = h * (numb)(1.0 / 6.0), two = (numb)2;
     numb k[UCB_NX], l[UCB_NX], xt[UCB_NX], sx[UCB_NX];
-    numb vt[UCB_NX][UCB_NX], sv[UCB_NX][UCB_NX];
+    numb vt[M][UCB_NX], sv[M][UCB_NX];
     ucb_rhs(x, a, k);
 #pragma unroll
-    for (int j = 0; j < UCB_NX; ++j) {
+    for (int j = 0; j < M; ++j) {
         ucb_jvp(x, a, V[j], l);
 #pragma unroll
         for (int i = 0; i < UCB_NX; ++i) {
@@ -205,7 +206,7 @@ __device__ __forceinline__ void ls_tangent_step(numb* x, numb (*V)[UCB_NX], cons
         const numb c = stage == 2 ? hh : h;
         ucb_rhs(xt, a, k);
 #pragma unroll
-        for (int j = 0; j < UCB_NX; ++j) {
+        for (int j = 0; j < M; ++j) {
             ucb_jvp(xt, a, vt[j], l);
 #pragma unroll
             for (int i = 0; i < UCB_NX; ++i) {
@@ -221,7 +222,7 @@ __device__ __forceinline__ void ls_tangent_step(numb* x, numb (*V)[UCB_NX], cons
     }
     ucb_rhs(xt, a, k);
 #pragma unroll
-    for (int j = 0; j < UCB_NX; ++j) {
+    for (int j = 0; j < M; ++j) {
         ucb_jvp(xt, a, vt[j], l);
 #pragma unroll
         for (int i = 0; i < UCB_NX; ++i) V[j][i] = fma(h6, sv[j][i] + l[i], V[j][i]);
@@ -267,21 +268,22 @@ __device__ __forceinline__ void gs_classical_f64(numb (*V)[UCB_NX], double* dens
 
 // NT-step block of x and the tangent vectors with the divergence test of loop_probes
 // (tangent vectors: non-finite only). 0 if anything diverged.
+template <int M>
 __device__ __forceinline__ int loop_tangents(numb* x, numb (*V)[UCB_NX], const numb* a, numb h, long long iters,
                                              numb maxValue, long long& ns) {
     for (long long i0 = 0; i0 < iters; i0 += kCheckInterval) {
-        ls_tangent_step(x, V, a, h);
+        ls_tangent_step<M>(x, V, a, h);
         ns += UCB_NX + 1;
         bool bad = diverged(x, maxValue);
 #pragma unroll
-        for (int j = 0; j < UCB_NX; ++j) bad = bad || diverged(V[j], (numb)0);
+        for (int j = 0; j < M; ++j) bad = bad || diverged(V[j], (numb)0);
         if (bad) return 0;
         const long long n = (iters - i0 < kCheckInterval) ? iters - i0 : kCheckInterval;
-        for (long long i = 1; i < n; ++i) ls_tangent_step(x, V, a, h);
+        for (long long i = 1; i < n; ++i) ls_tangent_step<M>(x, V, a, h);
         ns += (long long)(UCB_NX + 1) * (n - 1);
     }
 #if UCB_EXTRA_STEP
-    ls_tangent_step(x, V, a, h);
+    ls_tangent_step<M>(x, V, a, h);
     ns += UCB_NX + 1;
 #endif
     return 1;
@@ -347,7 +349,7 @@ __device__ __forceinline__ void ls_cell_fixed(const UcbLsParams& p, long long ki
 #pragma unroll
         for (int k = 0; k < UCB_NX; ++k) sum[k] = 0.0;
         for (int b = 0; b < p.n_blocks; ++b) {
-            if (loop_tangents(x, z, a, h, nt, p.maxv, ns) == 0) {
+            if (loop_tangents<UCB_NX>(x, z, a, h, nt, p.maxv, ns) == 0) {
 #pragma unroll
                 for (int m = 0; m < UCB_NX; ++m) outv[m] = 999.0;
                 ls_store(p, kidx, outv);
@@ -396,6 +398,209 @@ __device__ __forceinline__ void ls_cell_fixed(const UcbLsParams& p, long long ki
     for (int k = 0; k < UCB_NX; ++k) result[k] = (double)(res_n[k] / p.tmax);
     ls_store(p, kidx, result);
 }
+
+#if defined(UCB_LS_GROUP) && UCB_HAXIS == -1
+// ls_cell_fixed with a cell on several lanes, the same values and order of operations: a
+// trajectory a lane (x on the group's first lane and the N shadows after it) or, in the tangent
+// form, x and one tangent vector a lane. Every lane takes the transient; the rows of the
+// Gram-Schmidt pass are exchanged by shuffles, so all lanes of the warp stay in the loop until
+// all its cells are done. @@FIG@@
+#ifdef UCB_LS_FIXED_TANGENT
+constexpr int kLanes = UCB_NX, kFirstRow = 0;
+#else
+constexpr int kLanes = UCB_NX + 1, kFirstRow = 1;
+#endif
+
+// gram_schmidt_classical() over the group's rows: lane kFirstRow + i holds row i (row < 0: none).
+template <class T>
+__device__ __forceinline__ void group_gs(const T* a, T* b, T& dens, int row, int base) {
+#pragma unroll
+    for (int l = 0; l < UCB_NX; ++l) b[l] = a[l];
+#pragma unroll
+    for (int j = 0; j + 1 < UCB_NX; ++j) {
+        T w[UCB_NX];
+#pragma unroll
+        for (int l = 0; l < UCB_NX; ++l) w[l] = __shfl_sync(0xFFFFFFFFu, b[l], base + kFirstRow + j);
+        if (row > j) {
+            T num = 0, den = 0;
+#ifdef UCB_LS_FIXED_TANGENT
+#pragma unroll
+            for (int l = 0; l < UCB_NX; ++l) {
+                num = fma(a[l], w[l], num);
+                den = fma(w[l], w[l], den);
+            }
+            const T frac = den == 0 ? 0 : num / den;
+#pragma unroll
+            for (int l = 0; l < UCB_NX; ++l) b[l] = fma(-frac, w[l], b[l]);
+#else
+#pragma unroll
+            for (int l = 0; l < UCB_NX; ++l) {
+                num += a[l] * w[l];
+                den += w[l] * w[l];
+            }
+            const T frac = den == 0 ? 0 : num / den;
+#pragma unroll
+            for (int l = 0; l < UCB_NX; ++l) b[l] -= frac * w[l];
+#endif
+        }
+        __syncwarp();
+    }
+    T den = 0;
+#ifdef UCB_LS_FIXED_TANGENT
+#pragma unroll
+    for (int l = 0; l < UCB_NX; ++l) den = fma(b[l], b[l], den);
+    den = sqrt(den);
+    const T inv = den == 0 ? 0 : 1.0 / den;
+#pragma unroll
+    for (int l = 0; l < UCB_NX; ++l) b[l] *= inv;
+#else
+#pragma unroll
+    for (int l = 0; l < UCB_NX; ++l) den += b[l] * b[l];
+    den = sqrt(den);
+#pragma unroll
+    for (int l = 0; l < UCB_NX; ++l) b[l] = den == 0 ? 0 : b[l] / den;
+#endif
+    dens = den;
+}
+
+__device__ __forceinline__ void ls_groups_fixed(const UcbLsParams& p, long long& ns) {
+    const unsigned int full = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    const bool member = lane < p.groups * kLanes;
+    const int k = member ? lane % kLanes : 0, base = lane - k, row = member ? k - kFirstRow : -1;
+    const unsigned int group = member ? ((1u << kLanes) - 1u) << base : 0u;
+    const numb h = p.h;
+    for (;;) {
+        const long long first = warp_fetch(p.counter, lane, (unsigned long long)p.groups);
+        if (first >= p.total) return;
+        const long long at = first + lane / kLanes;
+        bool live = member && at < p.total;
+        const bool mine = live;
+        const long long kidx = p.cell_offset + (at < p.total ? at : p.total - 1);
+        numb x[UCB_NX], a[UCB_NV];  // x: this lane's trajectory
+#pragma unroll
+        for (int i = 0; i < UCB_NX; ++i) x[i] = p.ic[i];
+#pragma unroll
+        for (int i = 0; i < UCB_NV; ++i) a[i] = p.vals[i];
+        apply_sweep(cell_axes(kidx, p.n_pts), p.axis0, p.axis1, x, a);
+        numb z[UCB_NX];  // this lane's row
+        {
+            Rng st;
+            rng_init(1234567891ULL, (unsigned long long)kidx, 0ULL, &st);
+#pragma unroll
+            for (int j = 0; j < UCB_NX; ++j) {
+                numb r[UCB_NX];
+                numb zPower = 0;
+#pragma unroll
+                for (int i = 0; i < UCB_NX; ++i) {
+                    r[i] = rng_uniform(&st) - 0.5;
+                    zPower += r[i] * r[i];
+                }
+                zPower = sqrt(zPower);
+#pragma unroll
+                for (int i = 0; i < UCB_NX; ++i)
+                    if (j == row || (j == 0 && row < 0)) z[i] = r[i] / zPower;
+            }
+        }
+        const Stepper st(h);
+        long long steps = 0;  // of the cell, counted by all its lanes
+        if (loop_single(st, x, a, h, p.skip, p.maxv, steps) == 0) live = false;
+#ifdef UCB_LS_FIXED_TANGENT
+        double za[UCB_NX], zb[UCB_NX], dens, sum = 0;
+#pragma unroll
+        for (int i = 0; i < UCB_NX; ++i) za[i] = (double)z[i];
+        group_gs(za, zb, dens, row, base);
+        numb v[1][UCB_NX];
+#pragma unroll
+        for (int i = 0; i < UCB_NX; ++i) v[0][i] = (numb)zb[i];
+        for (int b = 0; b < p.n_blocks; ++b) {
+            if (!__any_sync(full, live)) break;
+            long long own = 0;
+            const int r = loop_tangents<1>(x, v, a, h, p.nt_steps, p.maxv, own);
+            const unsigned int bad = __ballot_sync(full, r == 0);
+            if (bad) {  // the count of the lane that stopped first
+                long long least = own;
+#pragma unroll
+                for (int j = 0; j < kLanes; ++j) {
+                    const long long o = __shfl_sync(full, own, base + j);
+                    least = o < least ? o : least;
+                }
+                own = least;
+            }
+            if (live) steps += own;
+            if (bad & group) live = false;
+#pragma unroll
+            for (int i = 0; i < UCB_NX; ++i) za[i] = (double)v[0][i];
+            group_gs(za, zb, dens, row, base);
+#pragma unroll
+            for (int i = 0; i < UCB_NX; ++i) v[0][i] = (numb)zb[i];
+            if (live) sum += log(dens);
+        }
+        const double out = live ? sum / (double)p.tmax : 999.0;
+#else
+        numb zb[UCB_NX], dens, sum = 0;
+        group_gs(z, zb, dens, row, base);
+        if (row >= 0) {
+#pragma unroll
+            for (int i = 0; i < UCB_NX; ++i) x[i] = zb[i] * p.eps + x[i];
+        }
+        for (int b = 0; b < p.n_blocks; ++b) {
+            if (!__any_sync(full, live)) break;
+#ifdef UCB_NT
+            {
+                const int r = run_nt(st, x, a, h, p.maxv);
+                const unsigned int bad = __ballot_sync(full, r == 0);
+                const bool stop = (bad & group) != 0;
+                if (live) steps += (UCB_NX + 1) * (stop ? 1 : UCB_NT + UCB_EXTRA_STEP);
+                if (stop) live = false;
+            }
+#else
+            for (long long i0 = 0; i0 < p.nt_steps; i0 += kCheckInterval) {
+                const int n = (p.nt_steps - i0 < kCheckInterval) ? (int)(p.nt_steps - i0) : kCheckInterval;
+                const int r = run_single<true>(st, x, a, h, n, p.maxv);
+                const unsigned int bad = __ballot_sync(full, r == 0);
+                const bool stop = (bad & group) != 0;
+                if (live) steps += (UCB_NX + 1) * (stop ? 1 : n);
+                if (stop) live = false;
+            }
+#if UCB_EXTRA_STEP
+            run_single<false>(st, x, a, h, 1, p.maxv);
+            if (live) steps += UCB_NX + 1;
+#endif
+#endif
+            numb xs[UCB_NX], d[UCB_NX];
+#pragma unroll
+            for (int l = 0; l < UCB_NX; ++l) {
+                xs[l] = __shfl_sync(full, x[l], base);
+                d[l] = x[l] - xs[l];
+            }
+            group_gs(d, zb, dens, row, base);
+            if (row >= 0) {
+                sum += log(dens / p.eps);
+#pragma unroll
+                for (int l = 0; l < UCB_NX; ++l) x[l] = (numb)(xs[l] + zb[l] * p.eps);
+            }
+        }
+        const double out = live ? (double)(sum / p.tmax) : 999.0;
+#endif
+        const unsigned int bad = __ballot_sync(full, mine && row >= 0 && (out == 999.0 || out == -999.0));
+        if (mine) {
+            const long long cell = ls_out_cell(p, kidx);
+#if UCB_DIM == 2
+            const long long plane = (long long)p.n_pts * p.n_pts;
+#else
+            const long long plane = p.n_pts;
+#endif
+            if (row >= 0) p.out_values[row * plane + cell] = out;
+            if (k == 0) {
+                p.out_flags[cell] = (bad & group) ? -1 : 1;
+                if (p.out_cell_steps) p.out_cell_steps[cell] = steps;
+                ns += steps;
+            }
+        }
+    }
+}
+#endif  // UCB_LS_GROUP
 #endif  // UCB_LS_FIXED
 
 #if defined(UCB_LS_DP5)
@@ -721,7 +926,7 @@ __device__ __forceinline__ void ls_cell_dp5(const UcbLsParams& p, long long kidx
 // it is done. The exchanges are taken by the whole warp; what a group does between them
 // depends on values that all its lanes hold. (The tangent's stages beside the state's, before
 // its step is accepted, gave the same times.) B200, 96^2 hyper-chaotic Rossler, t_end 50, FP64:
-// 68 -> 46 ms; where each form runs and its times: dp5_groups of ucb_ls.cpp.
+// 68 -> 46 ms; where each form runs and its times: ls_groups of ucb_ls.cpp.
 // mgs() over the group's rows (lane k holds row k), for groups with `act`; the log of the
 // norms added to acc. False if the group's rows are not independent and finite.
 __device__ __forceinline__ bool group_mgs(numb* v, double& acc, bool act, int k, int base, unsigned int group) {
@@ -933,7 +1138,11 @@ extern "C" __global__ void UCB_LAUNCH_BOUNDS ucb_ls_kernel(const UcbLsParams p) 
     const int lane = threadIdx.x & 31;
     long long ns = 0;
 #if defined(UCB_LS_GROUP)
+#if defined(UCB_LS_DP5)
     ucbdev::ls_groups_dp5(p, ns);
+#else
+    ucbdev::ls_groups_fixed(p, ns);
+#endif
     ucbdev::warp_add_steps(p.steps, ns, lane);
     return;
 #endif

@@ -52,24 +52,36 @@ ucb_lle2d_request as_lle(const ucb_ls2d_request& q) {
     return l;
 }
 
-// Cells a warp holds at a time when the adaptive method runs with a cell on amount_of_x lanes
-// (ls_groups_dp5); 0: a cell a lane. Groups cut an attempt's latency, lanes its instructions
-// (the state's step is taken once a cell), so groups run while the map has few warps for the
-// B200's 592 schedulers: measured with 4 variables over the wide hyper-chaotic Rossler window
-// (t_end 50, 20,000 attempts; lanes / groups), FP64 16^2 65 / 27 ms, 64^2 66 / 37, 96^2 68 / 46,
-// 120^2 69 / 64, 192^2 98 / 130; FP32 64^2 69 / 36, 128^2 71 / 45, 256^2 98 / 82, 384^2 131 / 151.
+// Cells a warp holds at a time when a cell runs on several lanes (ls_groups_dp5,
+// ls_groups_fixed); 0: a cell a lane. Lanes shorten a cell's chain and cost instructions (the
+// transient or the state's step, and the shuffled Gram-Schmidt pass, once a lane), so groups run
+// while the map has few warps for the B200's 592 schedulers.
+// Adaptive method, 4 variables over the wide hyper-chaotic Rossler window (t_end 50, 20,000
+// attempts; a cell a lane / groups): FP64 16^2 65 / 27 ms, 64^2 66 / 37, 96^2 68 / 46, 120^2
+// 69 / 64, 192^2 98 / 130; FP32 64^2 69 / 36, 128^2 71 / 45, 256^2 98 / 82, 384^2 131 / 151.
 // Fewer groups a warp leave it fewer attempts that wait for a neighbour's Gram-Schmidt, while
 // schedulers are to spare: 16^2 with 1 / 8 groups 27 / 34 ms, 48^2 with 4 / 8 32.5 / 36.7.
-int dp5_groups(const ucb_ls2d_request& q) {
+// Fixed method, warps of groups a scheduler up to `most` (4 variables, 6,000 steps): FP64 16^2
+// 3.28 / 1.18 ms, 96^2 3.30 / 2.06, 128^2 (4.6) 3.29 / 3.17, 192^2 (10) 5.3 / 6.3; FP32 tangents
+// 96^2 (1.9) 1.95 / 1.36, 128^2 (3.5) 1.95 / 2.37; exact FP32 128^2 9.5 / 6.1, 192^2 (10)
+// 11.8 / 12.4, of 3 variables (7.8) 6.0 / 5.4.
+int ls_groups(const ucb_ls2d_request& q, const SweepMap& m, bool tangent, bool exact) {
     constexpr long long kSchedulers = 4 * 148;
     const int nx = q.amount_of_x;
-    const long long cells = (long long)q.n_pts * q.n_pts;
-    if (q.method != UCB_LS_DP5 || nx < 2 || nx > 8) return 0;
-    if (cells > (q.opt.precision == UCB_PREC_F64 ? 24 : 128) * kSchedulers) return 0;
-    return (int)std::min<long long>((cells + kSchedulers - 1) / kSchedulers, 32 / nx);
+    const bool f64 = q.opt.precision == UCB_PREC_F64, dp5 = q.method == UCB_LS_DP5;
+    const long long cells = m.dim == 2 ? (long long)q.n_pts * q.n_pts : (long long)q.n_pts;
+    if (nx < 2 || nx > 8 || m.h_axis != -1) return 0;
+    const int most_groups = 32 / (dp5 || tangent ? nx : nx + 1);
+    if (dp5) {
+        if (cells > (f64 ? 24 : 128) * kSchedulers) return 0;
+        return (int)std::min<long long>((cells + kSchedulers - 1) / kSchedulers, most_groups);
+    }
+    const long long most = tangent ? 2 : f64 || !exact ? 5 : 8;
+    return cells <= most * kSchedulers * most_groups ? most_groups : 0;
 }
 
-CompileRequest ls_compile_request(const ucb_ls2d_request& q, const SweepMap& m, SystemCode& sys) {
+CompileRequest ls_compile_request(const ucb_ls2d_request& q, const SweepMap& m, SystemCode& sys,
+                                  int* groups_out = nullptr) {
     const bool dp5 = q.method == UCB_LS_DP5;
     const int prec = q.opt.precision;
     // the native FP32 form of the fixed method follows tangent vectors (v' = J(x) v) instead
@@ -84,7 +96,15 @@ CompileRequest ls_compile_request(const ucb_ls2d_request& q, const SweepMap& m, 
     std::vector<std::string> defs = dp5 ? clock_defines(sys) : std::vector<std::string>{};
     defs.push_back(dp5 ? "UCB_LS_DP5 1" : "UCB_LS_FIXED 1");
     if (tangent && sys.has_jvp) defs.push_back("UCB_LS_TANGENT 1");
-    if (dp5_groups(q)) defs.push_back("UCB_LS_GROUP 1");
+    const int groups = ls_groups(q, m, tangent && sys.has_jvp, sys.exact);
+    if (groups) {
+        defs.push_back("UCB_LS_GROUP 1");
+        // the fixed method's block length, known at compile time (plan_lle2d's count)
+        const bool in_double = prec == UCB_PREC_F64 || q.opt.mode == UCB_MODE_NATIVE;
+        const long long nt = in_double ? (long long)(q.NT / q.h) : (long long)((float)q.NT / (float)q.h);
+        if (!dp5 && nt >= 1 && nt <= 100) defs.push_back("UCB_NT " + std::to_string(nt));
+    }
+    if (groups_out) *groups_out = groups;
     defs.push_back(prec == UCB_PREC_F64 ? "UCB_GS_BUDGET 20.0" : "UCB_GS_BUDGET 8.0");
     rq.source = make_prelude(prec, q.amount_of_x, q.n_values, m, q.opt.nominal_steps == 0, sys, defs) +
                 "#include \"ucb_device.cuh\"\n#include \"ucb_ls.cuh\"\n";
@@ -144,7 +164,8 @@ int ls_run(ucb_engine* e, const ucb_ls2d_request& q, const SweepMap& m, int n_bl
     const int prec = q.opt.precision;
     const int nx = q.amount_of_x;
     SystemCode sys;
-    CompileRequest rq = ls_compile_request(q, m, sys);
+    int groups = 0;
+    CompileRequest rq = ls_compile_request(q, m, sys, &groups);
     if (dp5 && !sys.has_jvp)
         return fail(e, res, UCB_E_INVALID, "the DP5 method needs a recognised RK4 body: " + sys.note);
     TuneConfig shape;
@@ -210,7 +231,6 @@ int ls_run(ucb_engine* e, const ucb_ls2d_request& q, const SweepMap& m, int n_bl
     pk.put<void*>(ws);
     pk.put<void*>(ws + 8);
     pk.put<void*>(d_cell_steps);
-    const int groups = dp5_groups(q);
     pk.put<int>(groups);
     const int block = shape.block;
     const int grid = persistent_grid(e, fn, block, groups ? (total + groups - 1) / groups * 32 : total);
