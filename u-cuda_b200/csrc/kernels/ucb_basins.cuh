@@ -21,6 +21,17 @@
 #define UCB_PHASE -1
 #endif
 
+// Steps of the table loop unrolled, so that the next steps' loads run ahead of this one's chain
+// (forced Duffing 512^2, cap 1,000, 1 / 4 / 8 steps: FP64 79.4 / 74.9 / 72.6 ms, FP32 63.5 / 52.1 /
+// 49.9; 96^2 FP32 15.6 / 10.5 / 9.6).
+#if UCB_UNROLL > 1
+#define UCB_TRIG_UNROLL UCB_UNROLL
+#else
+#define UCB_TRIG_UNROLL 8
+#endif
+
+constexpr unsigned int kMaxSms = 256;
+
 struct UcbBasinsParams {
     long long total;
     int n_pts;
@@ -49,6 +60,19 @@ struct UcbBasinsParams {
     // period, so a step's three stage phases are the same in every period and cell); null:
     // the step evaluates them itself.
     const numb* trig;
+    // Slices: a launch takes periods first_period + 1 .. last_period of the cells in `list`
+    // (null: of all), and the cells it leaves unresolved go to next_list with their state.
+    int first_period, last_period;
+    int weight;                // progress of a cell that ends in this slice
+    int sm_count;
+    unsigned int* seats;       // blocks started on each SM (kMaxSms entries, zeroed)
+    const int* list;
+    const unsigned int* n_list;
+    int* next_list;
+    unsigned int* n_next;
+    numb* state;               // per cell, field-major: strobe state and history
+    int* state_runs;           // per cell, field-major: match runs
+    unsigned long long* progress;
 };
 
 namespace ucbdev {
@@ -93,7 +117,8 @@ __device__ __forceinline__ int register_attractor(const UcbBasinsParams& p, int 
     return 0;
 }
 
-__device__ __forceinline__ void basins_cell(const UcbBasinsParams& p, long long cell, long long& ns) {
+// Periods of one cell in this slice; true if it goes on in the next one.
+__device__ __forceinline__ bool basins_cell(const UcbBasinsParams& p, long long cell, long long& ns) {
     const CellAxes c = cell_axes(cell, p.n_pts);
     numb x[UCB_NX], a[UCB_NV];
 #pragma unroll
@@ -107,11 +132,25 @@ __device__ __forceinline__ void basins_cell(const UcbBasinsParams& p, long long 
     int run[UCB_MAXK];
 #pragma unroll
     for (int k = 0; k < UCB_MAXK; ++k) run[k] = 0;
+    if (p.first_period > 0) {
+        const numb* s = p.state + cell;
+        int f = 0;
+#pragma unroll
+        for (int i = 0; i < UCB_NX; ++i)
+            if (i != UCB_PHASE) x[i] = s[p.total * f++];
+#pragma unroll
+        for (int j = 0; j < UCB_MAXK; ++j)
+#pragma unroll
+            for (int i = 0; i < UCB_NS; ++i) hist[j][i] = s[p.total * f++];
+#pragma unroll
+        for (int k = 0; k < UCB_MAXK; ++k) run[k] = p.state_runs[cell + p.total * k];
+    }
     int label = 0, period = 0, n = 0;
-    for (n = 1; n <= p.max_periods; ++n) {
+    bool ended = false;
+    for (n = p.first_period + 1; n <= p.last_period; ++n) {
 #if defined(UCB_TRIG_PHASE) && !defined(UCB_EXACT) && UCB_PHASE == UCB_TRIG_PHASE
         if (p.trig) {
-            UCB_STEP_LOOP
+            UCB_PRAGMA_(unroll UCB_TRIG_UNROLL)
             for (int s = 0; s < p.steps_per_period; ++s) st.step_trig(x, a, p.h, p.trig + 4 * s);
         } else
 #endif
@@ -125,6 +164,7 @@ __device__ __forceinline__ void basins_cell(const UcbBasinsParams& p, long long 
         if (diverged(x, p.maxv)) {
             label = -1;
             period = -1;
+            ended = true;
             break;
         }
         numb P[UCB_NS];
@@ -174,6 +214,7 @@ __device__ __forceinline__ void basins_cell(const UcbBasinsParams& p, long long 
                 }
             }
             label = register_attractor(p, period, cx, cy);
+            ended = true;
             break;
         }
 #pragma unroll
@@ -183,21 +224,73 @@ __device__ __forceinline__ void basins_cell(const UcbBasinsParams& p, long long 
 #pragma unroll
         for (int i = 0; i < UCB_NS; ++i) hist[0][i] = P[i];
     }
+    if (!ended && p.last_period < p.max_periods) {
+        numb* s = p.state + cell;
+        int f = 0;
+#pragma unroll
+        for (int i = 0; i < UCB_NX; ++i)
+            if (i != UCB_PHASE) s[p.total * f++] = x[i];
+#pragma unroll
+        for (int j = 0; j < UCB_MAXK; ++j)
+#pragma unroll
+            for (int i = 0; i < UCB_NS; ++i) s[p.total * f++] = hist[j][i];
+#pragma unroll
+        for (int k = 0; k < UCB_MAXK; ++k) p.state_runs[cell + p.total * k] = run[k];
+        return true;
+    }
     p.out_labels[cell] = label;
     p.out_periods[cell] = period;
     p.out_iters[cell] = n > p.max_periods ? p.max_periods : n;
+    return false;
 }
 
 }  // namespace ucbdev
 
+// A map is taken in slices of periods, one launch each, with the unresolved cells packed into
+// full warps between them. In one launch a warp kept its 32 cells until the slowest was done
+// (28 lanes live on average), and the map ended with a wave of warps up to the cap's 2,000
+// periods long on ever fewer schedulers; cells that reach a slice's end have equal work in the
+// next. B200, forced Duffing, cap 2,000, FP64: 512^2 189 -> 158 ms (with the table loop
+// unrolled 136), 200^2 55.7 -> 37.2; FP32 512^2 148 -> 126 (98) ms.
 extern "C" __global__ void UCB_LAUNCH_BOUNDS ucb_basins_kernel(const UcbBasinsParams p) {
     const int lane = threadIdx.x & 31;
+    const unsigned int full = 0xFFFFFFFFu;
+    const long long cells = p.list ? (long long)*p.n_list : p.total;
+    if (p.list) {
+        // Nearly all listed cells take the whole slice. When its warps are fewer than the grid's,
+        // the blocks that start first would take them all and leave SMs idle: each SM seats as
+        // many blocks as its share needs. (Equal waves for larger lists, 9 warps a scheduler on
+        // 4 slots as 3 + 3 + 3, measured slower than 4 + 4 + 1: 148 against 136 ms at 512^2.)
+        const int per_block = blockDim.x >> 5;
+        const long long per_sm = ((cells + 31) / 32 + p.sm_count - 1) / p.sm_count;
+        __shared__ int seat;
+        if (threadIdx.x == 0) {
+            unsigned int sm;
+            asm("mov.u32 %0, %%smid;" : "=r"(sm));
+            seat = sm < kMaxSms ? (int)atomicAdd(&p.seats[sm], 1u) : 0;
+        }
+        __syncthreads();
+        if (seat >= (per_sm + per_block - 1) / per_block) return;
+    }
     long long ns = 0;
     for (;;) {
         const long long base = ucbdev::warp_fetch(p.counter, lane);
-        if (base >= p.total) break;
+        if (base >= cells) break;
         const long long i = base + lane;
-        if (i < p.total) ucbdev::basins_cell(p, i, ns);
+        bool more = false;
+        long long cell = 0;
+        if (i < cells) {
+            cell = p.list ? p.list[i] : i;
+            more = ucbdev::basins_cell(p, cell, ns);
+        }
+        const unsigned int going = __ballot_sync(full, more), all = __ballot_sync(full, i < cells);
+        unsigned int at = 0;
+        if (lane == 0) {
+            if (going) at = atomicAdd(p.n_next, (unsigned int)__popc(going));
+            atomicAdd(p.progress, (unsigned long long)(__popc(going) + __popc(all ^ going) * p.weight));
+        }
+        at = __shfl_sync(full, at, 0);
+        if (more) p.next_list[at + __popc(going & ((1u << lane) - 1u))] = (int)cell;
     }
     ucbdev::warp_add_steps(p.steps, ns, lane);
 }

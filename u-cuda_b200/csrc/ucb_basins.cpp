@@ -13,6 +13,10 @@ using namespace ucb;
 namespace {
 
 constexpr int kTableSlots = 4096;
+constexpr int kMaxSms = 256;    // of ucb_basins.cuh
+constexpr int kMaxK = 8;        // UCB_MAXK of ucb_basins.cuh
+constexpr int kSlices = 8;      // most slices of a map (at most 8: see the workspace)
+constexpr int kMinSlice = 64;   // periods
 
 bool validate(const ucb_basins_request& q, std::string& err) {
     if (!q.krs_body || !*q.krs_body) { err = "krs_body is empty"; return false; }
@@ -120,7 +124,7 @@ extern "C" int ucb_run_basins(ucb_engine* e, const ucb_basins_request* req, ucb_
     axis_table(prec, n, q.axis_y_lo, q.axis_y_hi, false, t1d, t1f);
     const size_t esz = prec == UCB_PREC_F64 ? 8 : 4;
     const size_t tab_bytes = (size_t)n * esz;
-    // workspace: [0] counter [8] steps [16] overflow | tables at 256.. | attractor table
+    // workspace: counters | tables at 256.. | attractor table
     const size_t off0 = 256, off1 = off0 + ((tab_bytes + 255) / 256) * 256;
     const size_t off_keys = off1 + ((tab_bytes + 255) / 256) * 256;
     const size_t off_pts = off_keys + kTableSlots * 8;
@@ -131,7 +135,8 @@ extern "C" int ucb_run_basins(ucb_engine* e, const ucb_basins_request* req, ucb_
     const bool use_trig = !sys.exact && sys.trig_phase >= 0 && sys.trig_phase == q.phase_var;
     const size_t trig_count = use_trig ? 2 * ((size_t)2 * q.steps_per_period + 1) : 0;
     const size_t off_trig = ((off_map + kTableSlots * 4 + 255) / 256) * 256;
-    const size_t ws_need = off_trig + trig_count * esz + 256;
+    const size_t off_seats = ((off_trig + trig_count * esz + 255) / 256) * 256;
+    const size_t ws_need = off_seats + (size_t)kSlices * kMaxSms * 4 + 256;
     if (!ensure_workspace(e, ws_need, err)) return fail(e, res, UCB_E_CUDA, err);
     char* ws = static_cast<char*>(e->ws);
     cudaStream_t st = e->stream;
@@ -139,8 +144,11 @@ extern "C" int ucb_run_basins(ucb_engine* e, const ucb_basins_request* req, ucb_
                     cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(ws + off1, prec == UCB_PREC_F64 ? (const void*)t1d.data() : (const void*)t1f.data(), tab_bytes,
                     cudaMemcpyHostToDevice, st);
-    cudaMemsetAsync(ws, 0, 32, st);
+    // ws: [0] progress, [8] steps, [16] overflow, [64 ..] work counters of the slices, [128 ..]
+    // lengths of the lists between them
+    cudaMemsetAsync(ws, 0, 256, st);
     cudaMemsetAsync(ws + off_keys, 0, kTableSlots * 8, st);
+    cudaMemsetAsync(ws + off_seats, 0, (size_t)kSlices * kMaxSms * 4, st);
     std::vector<double> trig_d;
     std::vector<float> trig_f;
     if (use_trig) {
@@ -161,6 +169,26 @@ extern "C" int ucb_run_basins(ucb_engine* e, const ucb_basins_request* req, ucb_
         (ce = dev_alloc(e, (void**)&d_periods, (size_t)total * 4, st)) != cudaSuccess ||
         (ce = dev_alloc(e, (void**)&d_iters, (size_t)total * 4, st)) != cudaSuccess)
         return fail(e, res, UCB_E_CUDA, std::string("cudaMallocAsync: ") + cudaGetErrorString(ce));
+    // Slices of the cap (ucb_basins_kernel): the cells' state between them has to fit beside
+    // what is in use; a map of at most a warp a scheduler, or of few periods, is one slice.
+    int slices = 1;
+    char* d_state = nullptr;
+    const int ns = q.amount_of_x - (q.phase_var >= 0 ? 1 : 0);
+    const size_t state_bytes = (((size_t)total * ns * (1 + kMaxK) * esz + 255) / 256) * 256;
+    const size_t runs_bytes = (((size_t)total * kMaxK * 4 + 255) / 256) * 256;
+    const size_t list_bytes = (((size_t)total * 4 + 255) / 256) * 256;
+    const size_t slice_bytes = state_bytes + runs_bytes + 2 * list_bytes;
+    if (total > 32LL * 4 * e->sm_count && q.max_periods > kMinSlice) {
+        size_t free_b = 0, total_b = 0;
+        if (slice_bytes > ((size_t)256 << 20)) cudaMemGetInfo(&free_b, &total_b);
+        if (slice_bytes <= std::max((size_t)256 << 20, (size_t)(0.4 * (double)free_b)) &&
+            dev_alloc(e, (void**)&d_state, slice_bytes, st) == cudaSuccess)
+            slices = std::min(kSlices, (q.max_periods + kMinSlice - 1) / kMinSlice);
+        else
+            cudaGetLastError();
+    }
+    const int slice = (q.max_periods + slices - 1) / slices;
+    slices = (q.max_periods + slice - 1) / slice;
     const double h = q.period / q.steps_per_period;
     ParamPack pk;
     pk.put<long long>(total);
@@ -186,15 +214,34 @@ extern "C" int ucb_run_basins(ucb_engine* e, const ucb_basins_request* req, ucb_
     pk.put<void*>(ws + off_pts);
     pk.put<void*>(ws + off_per);
     pk.put<void*>(ws + 16);
-    pk.put<void*>(ws);
-    pk.put<void*>(ws + 8);
-    pk.put<const void*>(use_trig ? (const void*)(ws + off_trig) : nullptr);
+    const ParamPack head = pk;
     const int block = shape.block;
+    const int grid = persistent_grid(e, fn, block, total);
+    char* lists[2] = {d_state + state_bytes + runs_bytes, d_state + state_bytes + runs_bytes + list_bytes};
+    int rc = UCB_OK;
     cudaEventRecord(e->ev0, st);
-    int rc = launch_packed(e, fn, persistent_grid(e, fn, block, total), block, st, pk, err) ? UCB_OK : UCB_E_CUDA;
+    for (int k = 0; k < slices && rc == UCB_OK; ++k) {
+        pk = head;
+        pk.put<void*>(ws + 64 + 8 * k);
+        pk.put<void*>(ws + 8);
+        pk.put<const void*>(use_trig ? (const void*)(ws + off_trig) : nullptr);
+        pk.put<int>(k * slice);
+        pk.put<int>(std::min((k + 1) * slice, q.max_periods));
+        pk.put<int>(slices - k);
+        pk.put<int>(e->sm_count);
+        pk.put<void*>(ws + off_seats + (size_t)k * kMaxSms * 4);
+        pk.put<const void*>(k ? lists[(k - 1) & 1] : nullptr);
+        pk.put<const void*>(ws + 128 + 4 * (k - 1));
+        pk.put<void*>(lists[k & 1]);
+        pk.put<void*>(ws + 128 + 4 * k);
+        pk.put<void*>(d_state);
+        pk.put<void*>(d_state + state_bytes);
+        pk.put<void*>(ws);
+        if (!launch_packed(e, fn, grid, block, st, pk, err)) rc = UCB_E_CUDA;
+    }
     if (rc == UCB_OK) {
         cudaEventRecord(e->ev1, st);
-        rc = wait_run(e, e->ev1, q.cancel, q.progress, total, err);
+        rc = wait_run(e, e->ev1, q.cancel, q.progress, total * slices, err);
         if (rc == UCB_E_CANCELLED) res->cancelled = 1;
     }
     // attractor table -> host: merge, order, map
@@ -277,6 +324,7 @@ extern "C" int ucb_run_basins(ucb_engine* e, const ucb_basins_request* req, ucb_
     cudaFreeAsync(d_labels, st);
     cudaFreeAsync(d_periods, st);
     cudaFreeAsync(d_iters, st);
+    if (d_state) cudaFreeAsync(d_state, st);
     cudaStreamSynchronize(st);
     if (rc != UCB_OK) return fail(e, res, rc, err);
     if (overflow) return fail(e, res, UCB_E_INVALID, "attractor table overflow (more than 4096 distinct keys)");
