@@ -27,12 +27,15 @@ struct TuneConfig {
 };
 }  // namespace ucb
 
-// Page-locked staging of the run control (kernels/ucb_device.cuh UcbControl lives in device
+// Page-locked side of the run control (kernels/ucb_device.cuh UcbControl lives in device
 // memory): the cancel word on its way to the device, the queue position on its way back.
+// Mapped into the device's address space, `cancel` and `fetched` laid out as UcbControl, for
+// the builds that poll it there (CompileRequest::mapped_control).
 struct ucb_run_control {
-    int32_t cancel;
+    volatile int32_t cancel;
     int32_t pad;
-    unsigned long long fetched;
+    volatile unsigned long long fetched;  // written by those builds
+    unsigned long long position;          // read back from the work counter
 };
 
 struct ucb_engine {

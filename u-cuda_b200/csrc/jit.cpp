@@ -226,11 +226,12 @@ std::shared_ptr<Module> ModuleCache::get(const CompileRequest& rq, std::string& 
         m->functions[k] = f;
         if (d.cuFuncGetAttribute) d.cuFuncGetAttribute(&m->registers, CU_FUNC_ATTRIBUTE_NUM_REGS, f);
     }
-    if (control_ && d.cuModuleGetGlobal && d.cuMemcpyHtoD) {
+    void* const control = rq.mapped_control ? mapped_control_ : control_;
+    if (control && d.cuModuleGetGlobal && d.cuMemcpyHtoD) {
         CUdeviceptr g = 0;
         size_t gsz = 0;
         if (d.cuModuleGetGlobal(&g, &gsz, m->module, "ucb_control") == CUDA_SUCCESS && gsz == sizeof(void*)) {
-            r = d.cuMemcpyHtoD(g, &control_, sizeof(void*));
+            r = d.cuMemcpyHtoD(g, &control, sizeof(void*));
             if (r != CUDA_SUCCESS) {
                 err = "binding the run-control block: " + cu_error_string(r);
                 return nullptr;

@@ -60,6 +60,7 @@ struct CompileRequest {
     std::vector<std::pair<std::string, std::string>> headers;  // name -> text
     std::vector<std::string> options; // extra NVRTC options
     std::vector<std::string> kernels; // extern "C" kernel names to look up
+    bool mapped_control = false;      // run control in mapped host memory (ucb_basins.cpp)
 };
 
 // Compiles (NVRTC, --gpu-architecture=sm_100a) to a CUBIN. Works without a GPU.
@@ -73,8 +74,12 @@ bool precompile_to_disk(const CompileRequest& rq, std::string& err);
 class ModuleCache {
 public:
     // Device address of the owner's run-control block (ucb_device.cuh UcbControl); every
-    // module loaded afterwards that defines the global `ucb_control` gets it.
-    void set_control(void* device_ptr) { control_ = device_ptr; }
+    // module loaded afterwards that defines the global `ucb_control` gets it, or the block in
+    // mapped host memory where its request asks for that.
+    void set_control(void* device_ptr, void* mapped_ptr) {
+        control_ = device_ptr;
+        mapped_control_ = mapped_ptr;
+    }
     std::shared_ptr<Module> get(const CompileRequest& rq, std::string& err);
     // Already-loaded module for this request, or nullptr (never compiles or loads).
     std::shared_ptr<Module> find(const CompileRequest& rq) const;
@@ -85,6 +90,7 @@ private:
     mutable std::mutex mu_;
     std::map<uint64_t, std::shared_ptr<Module>> cache_;
     void* control_ = nullptr;
+    void* mapped_control_ = nullptr;
 };
 
 uint64_t fnv1a64(const std::string& s, uint64_t h = 1469598103934665603ULL);

@@ -22,9 +22,8 @@
 #endif
 
 // Steps of the table loop unrolled, so that the next steps' loads run ahead of this one's chain
-// (forced Duffing 512^2, cap 1,000, 1 / 4 / 8 steps: FP64 79.4 / 74.9 / 72.6 ms, FP32 63.5 / 52.1 /
-// 49.9; 96^2 FP32 15.6 / 10.5 / 9.6).
-#if UCB_UNROLL > 1
+// (forced Duffing 512^2, cap 1,000, 1 / 4 / 8 steps: FP64 79.4 / 74.9 / 72.6 ms).
+#if UCB_UNROLL > 1 || defined(UCB_ONE_SLICE)
 #define UCB_TRIG_UNROLL UCB_UNROLL
 #else
 #define UCB_TRIG_UNROLL 8
@@ -132,6 +131,12 @@ __device__ __forceinline__ bool basins_cell(const UcbBasinsParams& p, long long 
     int run[UCB_MAXK];
 #pragma unroll
     for (int k = 0; k < UCB_MAXK; ++k) run[k] = 0;
+#ifdef UCB_ONE_SLICE
+#define UCB_FIRST_PERIOD 0
+#define UCB_LAST_PERIOD p.max_periods
+#else
+#define UCB_FIRST_PERIOD p.first_period
+#define UCB_LAST_PERIOD p.last_period
     if (p.first_period > 0) {
         const numb* s = p.state + cell;
         int f = 0;
@@ -145,9 +150,10 @@ __device__ __forceinline__ bool basins_cell(const UcbBasinsParams& p, long long 
 #pragma unroll
         for (int k = 0; k < UCB_MAXK; ++k) run[k] = p.state_runs[cell + p.total * k];
     }
+#endif
     int label = 0, period = 0, n = 0;
     bool ended = false;
-    for (n = p.first_period + 1; n <= p.last_period; ++n) {
+    for (n = UCB_FIRST_PERIOD + 1; n <= UCB_LAST_PERIOD; ++n) {
 #if defined(UCB_TRIG_PHASE) && !defined(UCB_EXACT) && UCB_PHASE == UCB_TRIG_PHASE
         if (p.trig) {
             UCB_PRAGMA_(unroll UCB_TRIG_UNROLL)
@@ -224,7 +230,7 @@ __device__ __forceinline__ bool basins_cell(const UcbBasinsParams& p, long long 
 #pragma unroll
         for (int i = 0; i < UCB_NS; ++i) hist[0][i] = P[i];
     }
-    if (!ended && p.last_period < p.max_periods) {
+    if (!ended && UCB_LAST_PERIOD < p.max_periods) {
         numb* s = p.state + cell;
         int f = 0;
 #pragma unroll
@@ -251,9 +257,18 @@ __device__ __forceinline__ bool basins_cell(const UcbBasinsParams& p, long long 
 // (28 lanes live on average), and the map ended with a wave of warps up to the cap's 2,000
 // periods long on ever fewer schedulers; cells that reach a slice's end have equal work in the
 // next. B200, forced Duffing, cap 2,000, FP64: 512^2 189 -> 158 ms (with the table loop
-// unrolled 136), 200^2 55.7 -> 37.2; FP32 512^2 148 -> 126 (98) ms.
+// unrolled 136), 200^2 55.7 -> 37.2. (UCB_ONE_SLICE: first_come_points of ucb_basins.cpp.)
 extern "C" __global__ void UCB_LAUNCH_BOUNDS ucb_basins_kernel(const UcbBasinsParams p) {
     const int lane = threadIdx.x & 31;
+    long long ns = 0;
+#ifdef UCB_ONE_SLICE
+    for (;;) {
+        const long long base = ucbdev::warp_fetch(p.counter, lane);
+        if (base >= p.total) break;
+        const long long i = base + lane;
+        if (i < p.total) ucbdev::basins_cell(p, i, ns);
+    }
+#else
     const unsigned int full = 0xFFFFFFFFu;
     const long long cells = p.list ? (long long)*p.n_list : p.total;
     if (p.list) {
@@ -272,7 +287,6 @@ extern "C" __global__ void UCB_LAUNCH_BOUNDS ucb_basins_kernel(const UcbBasinsPa
         __syncthreads();
         if (seat >= (per_sm + per_block - 1) / per_block) return;
     }
-    long long ns = 0;
     for (;;) {
         const long long base = ucbdev::warp_fetch(p.counter, lane);
         if (base >= cells) break;
@@ -292,6 +306,7 @@ extern "C" __global__ void UCB_LAUNCH_BOUNDS ucb_basins_kernel(const UcbBasinsPa
         at = __shfl_sync(full, at, 0);
         if (more) p.next_list[at + __popc(going & ((1u << lane) - 1u))] = (int)cell;
     }
+#endif
     ucbdev::warp_add_steps(p.steps, ns, lane);
 }
 

@@ -851,6 +851,8 @@ __device__ __forceinline__ void warp_add_steps(unsigned long long* counter, long
 // progress.
 struct UcbControl {
     int cancel;
+    int pad;
+    unsigned long long fetched;  // (in mapped host memory only)
 };
 
 }  // namespace ucbdev
@@ -876,11 +878,23 @@ __device__ __forceinline__ bool run_cancelled() {
 __device__ __forceinline__ long long warp_fetch(unsigned long long* counter, int lane,
                                                 unsigned long long batch = 32ULL) {
     unsigned long long base = 0;
+#ifdef UCB_MAPPED_CONTROL
+    if (lane == 0) {
+        UcbControl* c = ucb_control;
+        if (c && *(volatile int*)&c->cancel) {
+            base = 0x7fffffffffffffffULL;
+        } else {
+            base = atomicAdd(counter, batch);
+            if (c) *(volatile unsigned long long*)&c->fetched = base + batch;
+        }
+    }
+#else
     if (lane == 0) {
         const bool stop = run_cancelled();
         base = atomicAdd(counter, batch);
         if (stop) base = 0x7fffffffffffffffULL;
     }
+#endif
     base = __shfl_sync(0xffffffffu, base, 0);
     return (long long)base;
 }

@@ -84,14 +84,16 @@ bool ensure_init(ucb_engine* e, std::string& err) {
         // run control: the cancel word the kernels poll, in device memory (a poll of mapped
         // host memory crossed PCIe at every fetch of the work queue)
         void* h = nullptr;
+        void* mapped = nullptr;
         void* dptr = nullptr;
-        if (cudaHostAlloc(&h, sizeof(ucb_run_control), cudaHostAllocDefault) == cudaSuccess &&
+        if (cudaHostAlloc(&h, sizeof(ucb_run_control), cudaHostAllocMapped) == cudaSuccess &&
+            cudaHostGetDevicePointer(&mapped, h, 0) == cudaSuccess &&
             cudaMalloc(&dptr, 256) == cudaSuccess && cudaMemset(dptr, 0, 256) == cudaSuccess &&
             cudaStreamCreateWithFlags(&e->control_stream, cudaStreamNonBlocking) == cudaSuccess) {
             std::memset(h, 0, sizeof(ucb_run_control));
             e->control = static_cast<ucb_run_control*>(h);
             e->control_dev = dptr;
-            e->modules.set_control(dptr);
+            e->modules.set_control(dptr, mapped);
         } else {
             if (h) cudaFreeHost(h);
             if (dptr) cudaFree(dptr);
@@ -105,7 +107,8 @@ bool ensure_init(ucb_engine* e, std::string& err) {
 // Writes the cancel word the kernels poll.
 static void set_cancel(ucb_engine* e, int32_t v) {
     e->control->cancel = v;
-    cudaMemcpyAsync(e->control_dev, &e->control->cancel, sizeof(int32_t), cudaMemcpyHostToDevice, e->control_stream);
+    cudaMemcpyAsync(e->control_dev, const_cast<int32_t*>(&e->control->cancel), sizeof(int32_t),
+                    cudaMemcpyHostToDevice, e->control_stream);
     cudaStreamSynchronize(e->control_stream);
 }
 
@@ -135,10 +138,10 @@ int wait_run(ucb_engine* e, cudaEvent_t done, const volatile int32_t* cancel, vo
             cancelled = true;
         }
         if (progress && work_items > 0 &&
-            cudaMemcpyAsync(&c->fetched, e->ws, sizeof(c->fetched), cudaMemcpyDeviceToHost, e->control_stream) ==
+            cudaMemcpyAsync(&c->position, e->ws, sizeof(c->position), cudaMemcpyDeviceToHost, e->control_stream) ==
                 cudaSuccess &&
             cudaStreamSynchronize(e->control_stream) == cudaSuccess) {
-            const double f = (double)c->fetched / (double)work_items;
+            const double f = (double)c->position / (double)work_items;
             *progress = (float)std::min(f, 0.999);
         }
         if (std::chrono::steady_clock::now() - t0 < std::chrono::milliseconds(2))
