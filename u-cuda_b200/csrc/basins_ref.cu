@@ -681,7 +681,7 @@ CompileRequest features_request(const ucb_basins_dbscan_request& q, SystemCode& 
     defs.push_back("UCB_SCALAR_STEP 1");
     rq.source = make_prelude(q.opt.precision, q.amount_of_x, q.n_values, m, true, sys, defs) +
                 "#include \"ucb_device.cuh\"\n#include \"ucb_bif.cuh\"\n#include \"ucb_basins_ref.cuh\"\n";
-    rq.headers = device_headers();
+    rq.headers = &device_headers();
     rq.options.push_back(sys.exact ? "--fmad=false" : "--fmad=true");
     rq.kernels = {"ucb_basins_ref_kernel"};
     return rq;

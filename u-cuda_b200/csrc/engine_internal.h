@@ -156,9 +156,6 @@ SystemCode make_system_code(const std::string& krs_body, int nx, int nv, int pre
 std::string make_prelude(int precision, int nx, int nv, const SweepMap& m, bool extra_step,
                          const SystemCode& sys, const std::vector<std::string>& extra_defines);
 
-// Embedded device headers (generated at build time from csrc/kernels/*.cuh).
-const std::vector<std::pair<std::string, std::string>>& device_headers();
-
 // Axis value table of one sweep axis in numb arithmetic (getValueByIdx,
 // cudaLibrary.cu:1344-1361, and getValueByIdx_log, :1381-1396; valueNumber 0).
 void axis_table(int precision, int n, double lo, double hi, bool log_scale, std::vector<double>& out_d,

@@ -45,6 +45,9 @@ struct Driver {
 Driver& driver();
 std::string cu_error_string(CUresult r);
 
+// Embedded device headers (generated at build time from csrc/kernels/*.cuh).
+const std::vector<std::pair<std::string, std::string>>& device_headers();
+
 // One compiled program: module + looked-up kernels.
 struct Module {
     CUmodule module = nullptr;
@@ -57,7 +60,8 @@ struct Module {
 struct CompileRequest {
     std::string name;                 // program name for diagnostics
     std::string source;               // main translation unit
-    std::vector<std::pair<std::string, std::string>> headers;  // name -> text
+    // name -> text, of static lifetime (hashed once per process)
+    const std::vector<std::pair<std::string, std::string>>* headers = nullptr;
     std::vector<std::string> options; // extra NVRTC options
     std::vector<std::string> kernels; // extern "C" kernel names to look up
     bool mapped_control = false;      // run control in mapped host memory (ucb_basins.cpp)

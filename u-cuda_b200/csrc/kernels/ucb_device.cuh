@@ -642,12 +642,22 @@ template <class S>
 __device__ __forceinline__ int loop_single(const S& s, numb* x, const numb* a, numb h, long long iters,
                                            numb maxValue, long long& ns) {
     for (long long i0 = 0; i0 < iters; i0 += kCheckInterval) {
+#ifdef UCB_SIXTH
         const int n = (iters - i0 < kCheckInterval) ? (int)(iters - i0) : kCheckInterval;
         if (run_single<true>(s, x, a, h, n, maxValue) == 0) {
             ns += 1;
             return 0;
         }
         ns += n;
+#else
+        s.step(x, a, h);
+        ns += 1;
+        if (diverged(x, maxValue)) return 0;
+        const int n = (iters - i0 < kCheckInterval) ? (int)(iters - i0) : kCheckInterval;
+        UCB_STEP_LOOP
+        for (int i = 1; i < n; ++i) s.step(x, a, h);
+        ns += n - 1;
+#endif
     }
 #if UCB_EXTRA_STEP
     numb xPrev[UCB_NX];

@@ -65,7 +65,7 @@ CompileRequest basins_compile_request(const ucb_basins_request& q, SystemCode& s
     }
     rq.source = make_prelude(q.opt.precision, q.amount_of_x, q.n_values, m, true, sys, defs) +
                 "#include \"ucb_device.cuh\"\n#include \"ucb_basins.cuh\"\n";
-    rq.headers = device_headers();
+    rq.headers = &device_headers();
     rq.options.push_back(sys.exact ? "--fmad=false" : "--fmad=true");
     rq.kernels = {"ucb_basins_kernel", "ucb_basins_remap"};
     return rq;

@@ -95,7 +95,7 @@ CompileRequest bif2d_compile_request(const ucb_bif2d_request& q, const SweepMap&
     defs.push_back("UCB_BIF2D 1");
     rq.source = make_prelude(q.opt.precision, q.amount_of_x, q.n_values, m, true, sys, defs) +
                 "#include \"ucb_device.cuh\"\n#include \"ucb_dbscan1d.cuh\"\n#include \"ucb_bif.cuh\"\n";
-    rq.headers = device_headers();
+    rq.headers = &device_headers();
     rq.options.push_back(sys.exact ? "--fmad=false" : "--fmad=true");
     rq.kernels = {"ucb_bif2d_kernel"};
     return rq;

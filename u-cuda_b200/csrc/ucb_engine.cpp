@@ -535,7 +535,7 @@ CompileRequest lle_compile_request(const ucb_lle2d_request& q, const LlePlan& pl
     rq.name = "ucb_lle2d.cu";
     rq.source = make_prelude(prec, q.amount_of_x, q.n_values, plan.map, q.opt.nominal_steps == 0, L.sys, defs) +
                 "#include \"ucb_device.cuh\"\n#include \"ucb_lle.cuh\"\n";
-    rq.headers = device_headers();
+    rq.headers = &device_headers();
     rq.options.push_back(L.sys.exact ? "--fmad=false" : "--fmad=true");
     rq.kernels = {"ucb_lle_kernel", "ucb_state_kernel"};
     if (!tangent && plan.map.h_axis == -1) rq.kernels.insert(rq.kernels.begin(), "ucb_lle_split_kernel");

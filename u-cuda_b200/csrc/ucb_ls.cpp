@@ -108,7 +108,7 @@ CompileRequest ls_compile_request(const ucb_ls2d_request& q, const SweepMap& m, 
     defs.push_back(prec == UCB_PREC_F64 ? "UCB_GS_BUDGET 20.0" : "UCB_GS_BUDGET 8.0");
     rq.source = make_prelude(prec, q.amount_of_x, q.n_values, m, q.opt.nominal_steps == 0, sys, defs) +
                 "#include \"ucb_device.cuh\"\n#include \"ucb_ls.cuh\"\n";
-    rq.headers = device_headers();
+    rq.headers = &device_headers();
     rq.options.push_back(sys.exact ? "--fmad=false" : "--fmad=true");
     rq.kernels = {"ucb_ls_kernel"};
     return rq;
