@@ -12,6 +12,7 @@
 #define __forceinline__ inline
 #define __noinline__
 #define UCB_BIF_NO_KERNELS 1
+#define UCB_WV 0
 #define UCB_NX 1
 #define UCB_NV 1
 #define UCB_STEP_LOOP

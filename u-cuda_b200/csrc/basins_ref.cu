@@ -676,6 +676,7 @@ CompileRequest features_request(const ucb_basins_dbscan_request& q, SystemCode& 
     rq.name = "ucb_basins_ref.cu";
     std::vector<std::string> defs = clock_defines(sys);
     defs.push_back("UCB_BIF_NO_KERNELS 1");
+    defs.push_back("UCB_WV " + std::to_string(q.writable_var));
     // scalar RK4 updates: with the streaming peak finder beside the step, the packed
     // component pairs measured 11 % slower here (FP32 Duffing 1024^2: 987 vs 890 ms)
     defs.push_back("UCB_SCALAR_STEP 1");

@@ -109,7 +109,7 @@ __device__ __forceinline__ void basins_ref_cell(const UcbBasinsRefParams& p, lon
     sums.sp = sums.sp2 = sums.si = sums.si2 = 0;
     PeakScan scan;
     scan.init();
-    if (UCB_RECORDS(flag)) flag = loop_record(st, x, a, p.h, p.points, p.pre_scaller, p.writable_var, p.maxv, scan,
+    if (UCB_RECORDS(flag)) flag = loop_record(st, x, a, p.h, p.points, p.pre_scaller, p.maxv, scan,
                                               sums, ns, flag != 0);
     if (!live) return;
     if (flag == 0) {

@@ -49,23 +49,19 @@ struct PeakScan {
     }
 };
 
-__device__ __forceinline__ numb recorded_value(const numb* x, int wv) {
-    if (wv < 0) {
-#if UCB_NX >= 3
-        return x[0] + pi * x[1] + euler * x[2];
+// The recorded variable is a constant of the build (UCB_WV): a select by a run-time index
+// waited for every component at the end of each step (Lorenz diagram of 1,024 values, FP64,
+// 11,000 steps, kernel: 1.24 -> 1.10 ms).
+__device__ __forceinline__ numb recorded_value(const numb* x) {
+#if UCB_WV >= 0
+    return x[UCB_WV];
+#elif UCB_NX >= 3
+    return x[0] + pi * x[1] + euler * x[2];
 #elif UCB_NX == 2
-        return x[0] + pi * x[1];
+    return x[0] + pi * x[1];
 #else
-        return x[0];
+    return x[0];
 #endif
-    }
-    // a select over the components, not x[wv]: a run-time index would move the state out
-    // of registers into local memory (wv is validated to [0, N) by the host)
-    numb r = x[0];
-#pragma unroll
-    for (int j = 1; j < UCB_NX; ++j)
-        if (wv == j) r = x[j];
-    return r;
 }
 
 // Where the peaks of one point go: the first max_out peaks and intervals of a 1-D
@@ -104,15 +100,16 @@ __device__ __forceinline__ void emit_peak(PeakScan& s, long long j, numb d0, num
 // comparisons are independent of each other and give a bit mask of candidates, and the lanes
 // work through their few peaks of the chunk together. A divisor of kCheckInterval.
 // B200, native FP64: Lorenz diagram of 1,024 values 6.12 -> 3.60 ms, period map 256^2
-// 17.7 -> 14.7 ms; Duffing features 256^2 (FP32) 75.0 -> 73.1 ms.
-constexpr int kScanChunk = 20;
+// 17.7 -> 14.7 ms; Duffing features 256^2 (FP32) 75.0 -> 73.1 ms. (Chunks of 25 took 2-6 % less
+// than chunks of 20.)
+constexpr int kScanChunk = 25;
 // Samples in flight in the comparison loop. A diagram runs about one warp per scheduler, so it
-// takes the whole chunk at once (113 registers; 3.6 against 4.3 ms with 5); the maps keep
+// takes the whole chunk at once (3.6 against 4.3 ms with 5); the maps keep
 // their resident warps (256^2 period map: 64 against 120 registers, 14.7 against 15.1 ms).
 #if defined(UCB_BIF2D) || defined(UCB_BIF_NO_KERNELS)
 #define UCB_SCAN_UNROLL 5
 #else
-#define UCB_SCAN_UNROLL 20
+#define UCB_SCAN_UNROLL 25
 #endif
 
 // Decides the positions q0 - 1 .. q0 + m - 2 of a series of n samples, w[2 .. m + 1] holding
@@ -173,10 +170,10 @@ __device__ __forceinline__ void scan_chunk(PeakScan& s, const numb* w, long long
 // divergence test after the first sample's steps. 0: diverged there.
 template <class S>
 __device__ __forceinline__ int sample_chunk(const S& st, numb* x, const numb* a, numb h, numb* w, int m, bool check,
-                                            int pre, int wv, numb maxv) {
+                                            int pre, numb maxv) {
     int c = 0;
     if (check) {
-        w[2] = recorded_value(x, wv);
+        w[2] = recorded_value(x);
         st.step(x, a, h);
         for (int j = 1; j < pre; ++j) st.step(x, a, h);
         if (diverged(x, maxv)) return 0;
@@ -187,32 +184,32 @@ __device__ __forceinline__ int sample_chunk(const S& st, numb* x, const numb* a,
         // (Lorenz diagram, kernel: FP64 3.11 -> 2.66 ms, FP32 2.59 -> 2.13 ms; period maps 1-5 %)
 #pragma unroll 4
         for (; c < m; ++c) {
-            w[c + 2] = recorded_value(x, wv);
+            w[c + 2] = recorded_value(x);
             st.step(x, a, h);
         }
         return 1;
     }
     for (; c < m; ++c) {
-        w[c + 2] = recorded_value(x, wv);
+        w[c + 2] = recorded_value(x);
         for (int j = 0; j < pre; ++j) st.step(x, a, h);
     }
     return 1;
 }
 
 #ifdef UCB_SIXTH
-__device__ __noinline__ int redo_samples(numb* x, const numb* a, numb h, numb* w, int m, bool check, int pre, int wv,
+__device__ __noinline__ int redo_samples(numb* x, const numb* a, numb h, numb* w, int m, bool check, int pre,
                                          numb maxv) {
-    return sample_chunk(VerbatimStepper(), x, a, h, w, m, check, pre, wv, maxv);
+    return sample_chunk(VerbatimStepper(), x, a, h, w, m, check, pre, maxv);
 }
 __device__ __forceinline__ int run_samples(const Stepper& st, numb* x, const numb* a, numb h, numb* w, int m,
-                                           bool check, int pre, int wv, numb maxv) {
+                                           bool check, int pre, numb maxv) {
     numb keep[UCB_NX];
     copy_state<UCB_NX>(x, keep);
-    int r = st.verbatim ? 0 : sample_chunk(st, x, a, h, w, m, check, pre, wv, maxv);
+    int r = st.verbatim ? 0 : sample_chunk(st, x, a, h, w, m, check, pre, maxv);
     if (st.failed()) {
         numb av[UCB_NV];
         copy_values(a, av);
-        r = redo_samples(keep, av, h, w, m, check, pre, wv, maxv);
+        r = redo_samples(keep, av, h, w, m, check, pre, maxv);
         copy_state<UCB_NX>(keep, x);
     }
     return r;
@@ -220,8 +217,8 @@ __device__ __forceinline__ int run_samples(const Stepper& st, numb* x, const num
 #else
 template <class S>
 __device__ __forceinline__ int run_samples(const S& st, numb* x, const numb* a, numb h, numb* w, int m, bool check,
-                                           int pre, int wv, numb maxv) {
-    return sample_chunk(st, x, a, h, w, m, check, pre, wv, maxv);
+                                           int pre, numb maxv) {
+    return sample_chunk(st, x, a, h, w, m, check, pre, maxv);
 }
 #endif
 
@@ -230,7 +227,7 @@ __device__ __forceinline__ int run_samples(const S& st, numb* x, const numb* a, 
 // without a live cell (past the grid, or diverged) only does not count.
 template <class Sink>
 __device__ __forceinline__ int loop_record(const ForcedStepper& st, numb* x, const numb* a, numb h, long long iters,
-                                           int pre, int wv, numb maxv, PeakScan& scan, const Sink& sink,
+                                           int pre, numb maxv, PeakScan& scan, const Sink& sink,
                                            long long& ns, bool live) {
     if (!__any_sync(0xFFFFFFFFu, live)) return 0;
     numb w[kScanChunk + 2];
@@ -241,7 +238,7 @@ __device__ __forceinline__ int loop_record(const ForcedStepper& st, numb* x, con
         int c = 0;
         if (q0 % kCheckInterval == 0) {
             st.set_phase(x);
-            w[2] = recorded_value(x, wv);
+            w[2] = recorded_value(x);
             st.steps(x, a, h, pre);
             if (live && diverged(x, maxv)) {
                 ns += pre;
@@ -250,13 +247,13 @@ __device__ __forceinline__ int loop_record(const ForcedStepper& st, numb* x, con
             if (!__any_sync(0xFFFFFFFFu, live)) return 0;
             c = 1;
         }
-        if (pre == 1 && wv >= 0 && wv != UCB_TRIG_PHASE) {
+        if (pre == 1 && UCB_WV >= 0 && UCB_WV != UCB_TRIG_PHASE) {
             numb* at = w + c + 2;
-            st.steps(x, a, h, m - c, [&](int i) { at[i] = recorded_value(x, wv); });
+            st.steps(x, a, h, m - c, [&](int i) { at[i] = recorded_value(x); });
         } else {
             for (; c < m; ++c) {
                 st.set_phase(x);
-                w[c + 2] = recorded_value(x, wv);
+                w[c + 2] = recorded_value(x);
                 st.steps(x, a, h, pre);
             }
         }
@@ -308,7 +305,7 @@ __device__ __forceinline__ int loop_transient(const ForcedStepper& st, numb* x, 
 #define UCB_RECORDS(flag) ((flag) == 1 || (flag) == -1)
 template <class S, class Sink>
 __device__ __forceinline__ int loop_record(const S& st, numb* x, const numb* a, numb h, long long iters, int pre,
-                                           int wv, numb maxv, PeakScan& scan, const Sink& sink, long long& ns,
+                                           numb maxv, PeakScan& scan, const Sink& sink, long long& ns,
                                            bool /*live*/) {
     numb w[kScanChunk + 2];
 #pragma unroll
@@ -316,7 +313,7 @@ __device__ __forceinline__ int loop_record(const S& st, numb* x, const numb* a, 
     // The divergence test comes after the steps of samples 0, kCheckInterval, ...
     for (long long q0 = 0; q0 < iters; q0 += kScanChunk) {
         const int m = (iters - q0 < kScanChunk) ? (int)(iters - q0) : kScanChunk;
-        if (run_samples(st, x, a, h, w, m, q0 % kCheckInterval == 0, pre, wv, maxv) == 0) {
+        if (run_samples(st, x, a, h, w, m, q0 % kCheckInterval == 0, pre, maxv) == 0) {
             ns += pre;
             return 0;
         }
@@ -357,7 +354,189 @@ __device__ __forceinline__ int loop_transient(const S& st, numb* x, const numb* 
 
 }  // namespace ucbdev
 
-#if !defined(UCB_BIF2D) && !defined(UCB_BIF_NO_KERNELS)
+#if defined(UCB_BIF_PAIRED) && !defined(UCB_BIF2D) && !defined(UCB_BIF_NO_KERNELS)
+// A diagram with two warps for 32 points: the first integrates and leaves a chunk's samples in
+// shared memory, the second searches them for peaks while the first takes the next chunk. One
+// warp doing both spent 100 of a sample's 230 cycles on the search, with no other warp on its
+// scheduler to use them (B200, Lorenz, 1,024 values, native FP64,
+// 25,000 steps, kernel: 2.3 -> 1.79 ms). The two meet at a
+// barrier of their own once a chunk; both run the same number of chunks.
+namespace ucbdev {
+
+struct BifPair {
+    numb samples[2][kScanChunk][32];
+    int m[2][32];     // samples of a lane's chunk (0: none, diverged or past its end)
+    int live[2];      // any lane goes on
+    int found[32];
+};
+
+__device__ __forceinline__ void pair_barrier(int pair) {
+    __syncwarp();
+    asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory");
+}
+
+// Samples of one chunk to `out` (stride 32), with the steps of sample_chunk().
+template <class S>
+__device__ __forceinline__ int sample_strided(const S& st, numb* x, const numb* a, numb h, numb* out, int m, bool check,
+                                              int pre, numb maxv) {
+    int c = 0;
+    if (check) {
+        out[0] = recorded_value(x);
+        st.step(x, a, h);
+        for (int j = 1; j < pre; ++j) st.step(x, a, h);
+        if (diverged(x, maxv)) return 0;
+        c = 1;
+    }
+    if (pre == 1) {
+#pragma unroll 4
+        for (; c < m; ++c) {
+            out[c * 32] = recorded_value(x);
+            st.step(x, a, h);
+        }
+        return 1;
+    }
+    for (; c < m; ++c) {
+        out[c * 32] = recorded_value(x);
+        for (int j = 0; j < pre; ++j) st.step(x, a, h);
+    }
+    return 1;
+}
+#ifdef UCB_SIXTH
+__device__ __noinline__ int redo_strided(numb* x, const numb* a, numb h, numb* out, int m, bool check, int pre,
+                                         numb maxv) {
+    return sample_strided(VerbatimStepper(), x, a, h, out, m, check, pre, maxv);
+}
+__device__ __forceinline__ int run_strided(const Stepper& st, numb* x, const numb* a, numb h, numb* out, int m,
+                                           bool check, int pre, numb maxv) {
+    numb keep[UCB_NX];
+    copy_state<UCB_NX>(x, keep);
+    int r = st.verbatim ? 0 : sample_strided(st, x, a, h, out, m, check, pre, maxv);
+    if (st.failed()) {
+        numb av[UCB_NV];
+        copy_values(a, av);
+        r = redo_strided(keep, av, h, out, m, check, pre, maxv);
+        copy_state<UCB_NX>(keep, x);
+    }
+    return r;
+}
+#else
+template <class S>
+__device__ __forceinline__ int run_strided(const S& st, numb* x, const numb* a, numb h, numb* out, int m, bool check,
+                                           int pre, numb maxv) {
+    return sample_strided(st, x, a, h, out, m, check, pre, maxv);
+}
+#endif
+
+}  // namespace ucbdev
+
+extern "C" __global__ void __launch_bounds__(2 * UCB_BLOCK) ucb_bif_kernel(const UcbBifParams p) {
+    using namespace ucbdev;
+    __shared__ BifPair pairs[UCB_BLOCK / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pair = warp % (UCB_BLOCK / 32);
+    const bool integrates = warp < UCB_BLOCK / 32;
+    BifPair& s = pairs[pair];
+    const long long cell = ((long long)blockIdx.x * (UCB_BLOCK / 32) + pair) * 32 + lane;
+    const bool here = cell < p.n_pts;
+    const long long at = here ? cell : p.n_pts - 1;
+    numb h = p.h;
+    long long skip = p.skip, iters = p.iters, most = p.iters;
+#if UCB_HAXIS == 0
+    h = p.axis0[at];
+    if (h > 0) {
+        skip = (long long)ceil(p.transient / h);
+        const long long il = (long long)ceil(p.tmax / h / (numb)p.pre_scaller);
+        iters = il > p.iters ? p.iters : il;
+    }
+#endif
+    if (integrates) {
+        numb x[UCB_NX], a[UCB_NV];
+#pragma unroll
+        for (int i = 0; i < UCB_NX; ++i) x[i] = p.ic[i];
+#pragma unroll
+        for (int i = 0; i < UCB_NV; ++i) a[i] = p.vals[i];
+#if UCB_HAXIS != 0
+#if UCB_POV == 1
+        a[UCB_IDX0] = p.axis0[at];
+#else
+        x[UCB_IDX0] = p.axis0[at];
+#endif
+#endif
+        long long ns = 0;
+        const Stepper st(h);
+        int flag = -1;
+        bool live = here && h > 0;
+        if (live) {
+            flag = loop_transient(st, x, a, h, skip, p.pre_scaller, p.maxv, ns, true);
+            live = flag != 0;
+        }
+        int b = 0, since = 0;  // samples since the divergence test
+        for (long long q0 = 0; q0 < most; q0 += kScanChunk, b ^= 1) {
+            int m = 0;
+            if (live && q0 < iters) {
+                m = (iters - q0 < kScanChunk) ? (int)(iters - q0) : kScanChunk;
+                if (run_strided(st, x, a, h, &s.samples[b][0][lane], m, since == 0, p.pre_scaller, p.maxv) == 0) {
+                    ns += p.pre_scaller;
+                    m = 0;
+                    flag = 0;
+                    live = false;
+                } else {
+                    ns += (long long)p.pre_scaller * m;
+                }
+            }
+            since = since + kScanChunk == kCheckInterval ? 0 : since + kScanChunk;
+            __syncwarp();
+            s.m[b][lane] = m;
+            const int go = __any_sync(0xFFFFFFFFu, live);
+            if (lane == 0) s.live[b] = go;
+            pair_barrier(pair);
+            if (!go) break;
+        }
+        if (live) {
+            numb xPrev[UCB_NX];
+#pragma unroll
+            for (int j = 0; j < UCB_NX; ++j) xPrev[j] = x[j];
+            run_single<false>(st, x, a, h, p.pre_scaller, p.maxv);
+            ns += p.pre_scaller;
+            flag = fixed_point_flag(x, xPrev);
+        }
+        pair_barrier(pair);  // the second warp's counts
+        if (here) {
+            int count = flag;
+            if (live && flag == 1) {
+                int n = (s.found[lane] > 1) ? s.found[lane] - 1 : 0;
+                if (n >= kMaxAmountOfPeaks) n = kMaxAmountOfPeaks;
+                count = (iters < 5) ? 0 : n;
+            }
+            p.out_counts[cell] = count;
+        }
+        warp_add_steps(p.steps, ns, lane);
+    } else {
+        PeakScan scan;
+        scan.init();
+        const Bif1dSink sink{p.out_peaks + at * p.max_out, p.out_intervals + at * p.max_out, p.max_out, p.time_step};
+        numb w[kScanChunk + 2];
+#pragma unroll
+        for (int k = 0; k < kScanChunk + 2; ++k) w[k] = 0;
+        int b = 0;
+        for (long long q0 = 0; q0 < most; q0 += kScanChunk, b ^= 1) {
+            pair_barrier(pair);
+            const int m = s.m[b][lane];
+            if (m > 0) {
+#pragma unroll
+                for (int c = 0; c < kScanChunk; ++c) w[c + 2] = s.samples[b][c][lane];
+                scan_chunk(scan, w, q0, m, iters, sink);
+                w[0] = w[m];
+                w[1] = w[m + 1];
+            }
+            if (!s.live[b]) break;
+        }
+        s.found[lane] = scan.found;
+        pair_barrier(pair);
+    }
+}
+#endif  // UCB_BIF_PAIRED
+
+#if !defined(UCB_BIF_PAIRED) && !defined(UCB_BIF2D) && !defined(UCB_BIF_NO_KERNELS)
 extern "C" __global__ void UCB_LAUNCH_BOUNDS ucb_bif_kernel(const UcbBifParams p) {
     long long cell = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
@@ -398,7 +577,7 @@ extern "C" __global__ void UCB_LAUNCH_BOUNDS ucb_bif_kernel(const UcbBifParams p
                 scan.init();
                 const ucbdev::Bif1dSink sink{p.out_peaks + cell * p.max_out, p.out_intervals + cell * p.max_out,
                                              p.max_out, p.time_step};
-                flag = ucbdev::loop_record(st, x, a, h, iters, p.pre_scaller, p.writable_var, p.maxv, scan, sink,
+                flag = ucbdev::loop_record(st, x, a, h, iters, p.pre_scaller, p.maxv, scan, sink,
                                            ns, flag != 0);
                 if (flag == 1) {
                     int n = (scan.found > 1) ? scan.found - 1 : 0;
@@ -538,7 +717,7 @@ __device__ __forceinline__ int bif2d_peaks(const UcbBif2dParams& p, long long ki
             ucbdev::PeakScan scan;
             scan.init();
             const ucbdev::Bif2dSink sink{row, p.cap};
-            flag = ucbdev::loop_record(st, x, a, h, iters, p.pre_scaller, p.writable_var, p.maxv, scan, sink,
+            flag = ucbdev::loop_record(st, x, a, h, iters, p.pre_scaller, p.maxv, scan, sink,
                                        ns, flag != 0);
             if (flag == 1) {
                 int n = (scan.found > 1) ? scan.found - 1 : 0;

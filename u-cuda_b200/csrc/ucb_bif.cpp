@@ -44,7 +44,16 @@ bool validate_bif(const ucb_bif1d_request& q, std::string& err) {
     return true;
 }
 
-CompileRequest bif_compile_request(const ucb_bif1d_request& q, SystemCode& sys) {
+// Whether a diagram runs with two warps for 32 points (ucb_bif.cuh, UCB_BIF_PAIRED): while both
+// have a scheduler of their own on the B200's 148 SMs. Native Lorenz, FP64, 11,000 steps, one /
+// two warps (kernel): 1,024 values 1.04 / 0.81 ms, 40,000 values 2.19 / 3.04. Its shared memory
+// is laid out for blocks of up to 64 points, and builds whose warp shares a forcing phase have
+// their own loops.
+bool pairs_pay(const ucb_bif1d_request& q, const SystemCode& sys) {
+    return q.n_pts <= 16 * 4 * 148 && q.opt.block_threads <= 64 && sys.trig_phase < 0;
+}
+
+CompileRequest bif_compile_request(const ucb_bif1d_request& q, SystemCode& sys, bool* paired = nullptr) {
     SweepMap m;
     m.dim = 1;
     m.par_or_var = q.sweep_over_var ? 0 : 1;
@@ -53,7 +62,12 @@ CompileRequest bif_compile_request(const ucb_bif1d_request& q, SystemCode& sys) 
     sys = make_system_code(q.krs_body, q.amount_of_x, q.n_values, q.opt.precision, q.opt.mode, false);
     CompileRequest rq;
     rq.name = "ucb_bif1d.cu";
-    rq.source = make_prelude(q.opt.precision, q.amount_of_x, q.n_values, m, true, sys, clock_defines(sys)) +
+    std::vector<std::string> defs = clock_defines(sys);
+    defs.push_back("UCB_WV " + std::to_string(q.writable_var));
+    const bool two = pairs_pay(q, sys);
+    if (two) defs.push_back("UCB_BIF_PAIRED 1");
+    if (paired) *paired = two;
+    rq.source = make_prelude(q.opt.precision, q.amount_of_x, q.n_values, m, true, sys, defs) +
                 "#include \"ucb_device.cuh\"\n#include \"ucb_bif.cuh\"\n";
     rq.headers = &device_headers();
     rq.options.push_back(sys.exact ? "--fmad=false" : "--fmad=true");
@@ -118,7 +132,8 @@ extern "C" int ucb_run_bif1d(ucb_engine* e, const ucb_bif1d_request* req, ucb_bi
     if (!ensure_init(e, err)) return fail(e, res, UCB_E_NOGPU, err);
 
     SystemCode sys;
-    CompileRequest rq = bif_compile_request(q, sys);
+    bool paired = false;
+    CompileRequest rq = bif_compile_request(q, sys, &paired);
     TuneConfig shape;
     if (!tune_request(e, q.opt, 32, rq, shape, err)) return fail(e, res, UCB_E_INVALID, err);
     auto mod = e->modules.get(rq, err);
@@ -165,7 +180,7 @@ extern "C" int ucb_run_bif1d(ucb_engine* e, const ucb_bif1d_request* req, ucb_bi
     pk.put<void*>(ws + 8);
     const int block = shape.block;  // default 32: latency-bound, spread the few points over many SMs
     cudaEventRecord(e->ev0, e->stream);
-    const bool launched = launch_packed(e, fn, (n + block - 1) / block, block, e->stream, pk, err);
+    const bool launched = launch_packed(e, fn, (n + block - 1) / block, paired ? 2 * block : block, e->stream, pk, err);
     cudaEventRecord(e->ev1, e->stream);
     int rc = launched ? UCB_OK : UCB_E_CUDA;
     std::vector<double> hp(pk_elems), hi(pk_elems);

@@ -93,6 +93,7 @@ CompileRequest bif2d_compile_request(const ucb_bif2d_request& q, const SweepMap&
     rq.name = "ucb_bif2d.cu";
     std::vector<std::string> defs = clock_defines(sys);
     defs.push_back("UCB_BIF2D 1");
+    defs.push_back("UCB_WV " + std::to_string(q.writable_var));
     rq.source = make_prelude(q.opt.precision, q.amount_of_x, q.n_values, m, true, sys, defs) +
                 "#include \"ucb_device.cuh\"\n#include \"ucb_dbscan1d.cuh\"\n#include \"ucb_bif.cuh\"\n";
     rq.headers = &device_headers();
