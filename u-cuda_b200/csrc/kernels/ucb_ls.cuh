@@ -404,7 +404,7 @@ __device__ __forceinline__ void ls_cell_fixed(const UcbLsParams& p, long long ki
 // trajectory a lane (x on the group's first lane and the N shadows after it) or, in the tangent
 // form, x and one tangent vector a lane. Every lane takes the transient; the rows of the
 // Gram-Schmidt pass are exchanged by shuffles, so all lanes of the warp stay in the loop until
-// all its cells are done. @@FIG@@
+// all its cells are done. Where each form runs and its times: ls_groups of ucb_ls.cpp.
 #ifdef UCB_LS_FIXED_TANGENT
 constexpr int kLanes = UCB_NX, kFirstRow = 0;
 #else
