@@ -1581,6 +1581,8 @@ bool ensure_rows(Mlp& m, int rows, std::string& err) {
     if (!(m.blk = dalloc<float>((R + 31) / 32 * 3, o, err, "NLL block sums")) ||
         !(m.done = dalloc<unsigned int>(1, o, err, "block tickets")))
         return false;
+    // the buffers are cleared on the default stream, which the caller's stream need not wait for
+    if (!cu_ok(cudaStreamSynchronize(nullptr), err, "clear buffers")) return false;
     m.rows = rows;
     return true;
 }
@@ -1925,9 +1927,13 @@ bool mlp_reinit(Mlp* m, std::string& err) {
     for (auto& v : hb) v = c.fourier_scale * nd(rng);
     m->y_mean = 0.f;
     m->y_std = 1.f;
-    if (!cu_ok(cudaMemcpy(m->p, hp.data(), m->n_params * sizeof(float), cudaMemcpyHostToDevice), err,
+    // on the stream of the kernel that reads them: a copy from pageable memory may return while
+    // its last part is still on the way, and the engine's stream does not wait for the default one
+    cudaStream_t st = m->e->stream;
+    if (!cu_ok(cudaMemcpyAsync(m->p, hp.data(), m->n_params * sizeof(float), cudaMemcpyHostToDevice, st), err,
                "upload params") ||
-        !cu_ok(cudaMemcpy(m->Bf, hb.data(), hb.size() * sizeof(float), cudaMemcpyHostToDevice), err, "upload B"))
+        !cu_ok(cudaMemcpyAsync(m->Bf, hb.data(), hb.size() * sizeof(float), cudaMemcpyHostToDevice, st), err,
+               "upload B"))
         return false;
     return refresh(*m, m->e->stream, err) && cu_ok(cudaStreamSynchronize(m->e->stream), err, "init");
 }
@@ -2134,7 +2140,9 @@ int ucb_mlp_set_params(ucb_mlp* m, const float* in, long long n) {
     if (!m || !in || n != m->m->n_params) return UCB_E_INVALID;
     cudaSetDevice(m->e->device);
     std::string err;
-    if (cudaMemcpy(m->m->p, in, n * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) return UCB_E_CUDA;
+    // the copy and the BF16 refresh share a stream (see mlp_reinit)
+    if (cudaMemcpyAsync(m->m->p, in, n * sizeof(float), cudaMemcpyHostToDevice, m->e->stream) != cudaSuccess)
+        return UCB_E_CUDA;
     if (!refresh(*m->m, m->e->stream, err) || cudaStreamSynchronize(m->e->stream) != cudaSuccess) {
         m->e->last_error = err;
         return UCB_E_CUDA;
@@ -2166,8 +2174,8 @@ int ucb_mlp_loss_grad(ucb_mlp* h, const float* u, const float* y, long long n, f
     cudaStream_t st = h->e->stream;
     if (!ensure_rows(m, rows, err) || !cu_ok(cudaMalloc(&du, n * 2 * sizeof(float)), err, "alloc u") ||
         !cu_ok(cudaMalloc(&dy, n * sizeof(float)), err, "alloc y") ||
-        !cu_ok(cudaMemcpy(du, u, n * 2 * sizeof(float), cudaMemcpyHostToDevice), err, "upload u") ||
-        !cu_ok(cudaMemcpy(dy, y, n * sizeof(float), cudaMemcpyHostToDevice), err, "upload y") ||
+        !cu_ok(cudaMemcpyAsync(du, u, n * 2 * sizeof(float), cudaMemcpyHostToDevice, st), err, "upload u") ||
+        !cu_ok(cudaMemcpyAsync(dy, y, n * sizeof(float), cudaMemcpyHostToDevice, st), err, "upload y") ||
         !cu_ok(cudaMemsetAsync(m.err, 0, sizeof(int), st), err, "reset err")) {
         rc = UCB_E_CUDA;
     } else {

@@ -89,6 +89,7 @@ bool ensure_init(ucb_engine* e, std::string& err) {
         if (cudaHostAlloc(&h, sizeof(ucb_run_control), cudaHostAllocMapped) == cudaSuccess &&
             cudaHostGetDevicePointer(&mapped, h, 0) == cudaSuccess &&
             cudaMalloc(&dptr, 256) == cudaSuccess && cudaMemset(dptr, 0, 256) == cudaSuccess &&
+            cudaStreamSynchronize(nullptr) == cudaSuccess &&
             cudaStreamCreateWithFlags(&e->control_stream, cudaStreamNonBlocking) == cudaSuccess) {
             std::memset(h, 0, sizeof(ucb_run_control));
             e->control = static_cast<ucb_run_control*>(h);
