@@ -20,7 +20,8 @@
 //
 // Prediction: one fused kernel per call (mlp_infer_kernel) runs features, every hidden
 // layer and the output transform of a 128-row tile inside one CTA, with the activations in
-// shared memory; HBM sees the inputs and the two outputs per row only.
+// shared memory; HBM sees the inputs and the two outputs per row only. The forward half of a
+// training step is the same kernel (TRAIN), which also leaves what the backward pass reads.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -296,6 +297,16 @@ __device__ __forceinline__ void rows_staged(uint32_t* stage, const uint32_t (&va
 // Transposed BF16: column j of the chunk (its 32 rows) to outt + j * ld (elements; outt points
 // at column 0, row 0 of the warp). The buffer holds the chunk column-major, so each column's
 // 64 bytes are contiguous; a store instruction writes 16-byte pieces of eight columns.
+__device__ __forceinline__ void cols_from_stage(const uint32_t* stage, bf16* outt, size_t ld) {
+    const int lane = threadIdx.x & 31;
+    const uint4* s4 = reinterpret_cast<const uint4*>(stage);
+#pragma unroll
+    for (int pass = 0; pass < 4; ++pass) {
+        const int j = pass * 8 + lane / 4, q = lane % 4;
+        *reinterpret_cast<uint4*>(outt + (size_t)j * ld + q * 8) = s4[j * 4 + q];
+    }
+    __syncwarp();
+}
 __device__ __forceinline__ void cols_staged(uint32_t* stage, const float (&g)[32], bf16* outt, size_t ld) {
     const int lane = threadIdx.x & 31;
     unsigned short* s2 = reinterpret_cast<unsigned short*>(stage);
@@ -305,13 +316,20 @@ __device__ __forceinline__ void cols_staged(uint32_t* stage, const float (&g)[32
         s2[j * 32 + lane] = *reinterpret_cast<const unsigned short*>(&b);
     }
     __syncwarp();
-    const uint4* s4 = reinterpret_cast<const uint4*>(stage);
+    cols_from_stage(stage, outt, ld);
+}
+
+// The same from a row's 32 values already rounded to BF16, two a word.
+__device__ __forceinline__ void cols_staged(uint32_t* stage, const uint32_t (&pk)[16], bf16* outt, size_t ld) {
+    const int lane = threadIdx.x & 31;
+    unsigned short* s2 = reinterpret_cast<unsigned short*>(stage);
 #pragma unroll
-    for (int pass = 0; pass < 4; ++pass) {
-        const int j = pass * 8 + lane / 4, q = lane % 4;
-        *reinterpret_cast<uint4*>(outt + (size_t)j * ld + q * 8) = s4[j * 4 + q];
+    for (int j = 0; j < 16; ++j) {
+        s2[(2 * j) * 32 + lane] = (unsigned short)(pk[j] & 0xffffu);
+        s2[(2 * j + 1) * 32 + lane] = (unsigned short)(pk[j] >> 16);
     }
     __syncwarp();
+    cols_from_stage(stage, outt, ld);
 }
 
 template <int MODE>
@@ -693,6 +711,17 @@ __device__ __forceinline__ void feature_sincos(float u0, float u1, const float* 
     __sincosf(__fmul_rn(6.283185307179586f, __fsub_rn(x, rintf(x))), &s, &c);
 }
 
+// The input that row r of a batch (or of this chunk) takes; false past the last one.
+__device__ __forceinline__ bool batch_row(const FeatureArgs& a, int r, long long& i) {
+    if (a.step) {
+        const unsigned long long h = mix64(a.seed ^ mix64(*a.step * 0x100000001B3ULL + (unsigned long long)r));
+        i = (long long)(h % (unsigned long long)a.n);
+        return a.n > 0;
+    }
+    i = a.row0 + r;
+    return i < a.n;
+}
+
 // X[r, j] = sin(2 pi u.B_j), X[r, fourier + j] = cos(...). One thread per (row, group of
 // 8 frequencies); consecutive threads take consecutive rows of one group, so the transposed
 // copy's stores are contiguous across a warp and each row's 8 values go out as 16 bytes.
@@ -705,15 +734,7 @@ __global__ void features_kernel(FeatureArgs a) {
     const int r = (int)(t % a.rows);
     const int j0 = 8 * (int)(t / a.rows);
     long long i;
-    bool valid;
-    if (a.step) {
-        const unsigned long long h = mix64(a.seed ^ mix64(*a.step * 0x100000001B3ULL + (unsigned long long)r));
-        i = (long long)(h % (unsigned long long)a.n);
-        valid = a.n > 0;
-    } else {
-        i = a.row0 + r;
-        valid = i < a.n;
-    }
+    const bool valid = batch_row(a, r, i);
     float u0 = 0.f, u1 = 0.f;
     if (valid) input_point(a, i, u0, u1);
     float sv[8], cv[8];
@@ -916,6 +937,18 @@ __global__ void unscale_kernel(const float* out, int rows, long long n_left, flo
 // stages, once per tile and layer; they stay in L2.
 // The epilogue writes a layer's output over the activations its MMAs have finished
 // reading, so one activation buffer per slot suffices. Waits are bounded as in the GEMM.
+//
+// TRAIN: the forward half of a training step (features of the batch's rows, hidden layers,
+// output layer and loss) with the same roles. Rows do not mix before the weight gradients, so
+// a CTA carries its 128 rows through every layer, and what the backward pass reads leaves on
+// the way: the features and the activations transposed, Z, and the loss's gradients. A batch
+// has few tiles, so each CTA keeps one in flight and its two TMEM accumulators alternate by
+// layer: the epilogue first writes the next layer's operand and releases the MMAs, then reads
+// the accumulator once more and stores Z and H^T while they run. The space of the second
+// tile's activations stages those stores. A layer a launch was bound by latency (launch,
+// prologue, one tile's loads, MMAs and epilogue, drain: 9-10 us for a microsecond of MMAs).
+// Here a layer of 128 is 4 us of a CTA, one of 256 is 8.5 us (the stores' passes through shared
+// memory); forward_train has the times of a step.
 struct InferMaps {
     CUtensorMap w[kMaxLayers];  // layer l's BF16 weights [rows, K]: boxes of 64 (K) x H rows (16 for the output layer)
 };
@@ -936,19 +969,32 @@ struct InferArgs {
     long long tiles;         // ceil(n / 128)
 };
 
+// What the forward pass of a training step takes and leaves besides (TRAIN).
+struct TrainArgs {
+    FeatureArgs f;           // the batch's rows; Xt and yb are written, X is not
+    float* Z[kMaxLayers];    // rows x H pre-activations of each hidden layer
+    bf16* Ht[kMaxLayers];    // H x rows activations
+    Epilogue loss;           // the fields of nll_rows
+};
+struct NoTrainArgs {};
+
 constexpr int kInferEpiWarps = 16;  // four per 32-lane TMEM quadrant, a quarter of the columns each
 constexpr int kInferThreads = 64 + 32 * kInferEpiWarps;
 
-template <int H>
+template <int H, bool TRAIN = false>
 struct InferCfg {
+    static constexpr int kSlots = TRAIN ? 1 : 2;             // tiles in flight
     static constexpr int kOutN = 16;                         // MMA width of the output layer (2 used)
     static constexpr int kChunkBytes = kBM * kBK * 2;        // one 128 x 64 operand chunk (16 KB)
     static constexpr int kActBytes = (H / kBK) * kChunkBytes; // one slot's activations
     static constexpr int kWBytes = H * kBK * 2;              // one weight stage: H rows x 64 K
     static constexpr int kWStages = H == 256 ? 3 : 6;
-    // barriers: weight full / empty per stage, accumulator full and epilogue done per slot, drain
-    static constexpr int kBarriers = 2 * kWStages + 4 + 1;
-    static constexpr int kSmem = 1024 + 2 * kActBytes + kWStages * kWBytes + 8 * kBarriers + 16;
+    // barriers: weight full / empty per stage, accumulator full and epilogue done per slot, drain,
+    // and (TRAIN) a tile's activations read back
+    static constexpr int kBarriers = 2 * kWStages + 4 + 1 + (TRAIN ? 1 : 0);
+    static constexpr int kStoreStage = TRAIN ? 4096 : 0;     // per epilogue warp: one 32 x 32 chunk on its way out
+    static constexpr int kWOffset = kSlots * kActBytes + kInferEpiWarps * kStoreStage;
+    static constexpr int kSmem = 1024 + kWOffset + kWStages * kWBytes + 8 * kBarriers + 16;
     using MmaH = SM100_MMA_F16BF16_SS<bf16, bf16, float, kBM, H, UMMA::Major::K, UMMA::Major::K>;
     using MmaO = SM100_MMA_F16BF16_SS<bf16, bf16, float, kBM, kOutN, UMMA::Major::K, UMMA::Major::K>;
     using TiledH = decltype(make_tiled_mma(MmaH{}));
@@ -980,6 +1026,9 @@ __device__ __forceinline__ uint32_t act_offset(int r, int col) {
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
+__device__ __forceinline__ void ld_shared_v4(uint32_t addr, uint32_t& x, uint32_t& y, uint32_t& z, uint32_t& w) {
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x), "=r"(y), "=r"(z), "=r"(w) : "r"(addr) : "memory");
+}
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
@@ -987,16 +1036,18 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
-template <int H>
+template <int H, bool TRAIN>
 __global__ void __launch_bounds__(kInferThreads, 1)
-    mlp_infer_kernel(const __grid_constant__ InferMaps maps, const InferArgs a, int* err) {
-    using Cfg = InferCfg<H>;
+    mlp_infer_kernel(const __grid_constant__ InferMaps maps, const InferArgs a,
+                       const std::conditional_t<TRAIN, TrainArgs, NoTrainArgs> tr, int* err) {
+    using Cfg = InferCfg<H, TRAIN>;
+    constexpr int kSlots = Cfg::kSlots;
     constexpr int S = Cfg::kWStages;
     typename Cfg::TiledH mma_h;
     typename Cfg::TiledO mma_o;
     extern __shared__ char smem_raw[];
     char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    char* wst = base + 2 * Cfg::kActBytes;
+    char* wst = base + Cfg::kWOffset;
     uint64_t* bars = reinterpret_cast<uint64_t*>(wst + S * Cfg::kWBytes);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::kBarriers);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -1005,6 +1056,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
     auto accf = [&](int t) { return smem_u32(bars + 2 * S + t); };
     auto epid = [&](int t) { return smem_u32(bars + 2 * S + 2 + t); };
     const uint32_t drain_bar = smem_u32(bars + 2 * S + 4);
+    const uint32_t read_bar = smem_u32(bars + 2 * S + 5);  // TRAIN
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
     cute::TMEM::Allocator1Sm tmem;
@@ -1019,6 +1071,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
             mbar_init(epid(t), kInferEpiWarps);
         }
         mbar_init(drain_bar, 1);
+        if (TRAIN) mbar_init(read_bar, kInferEpiWarps);
         *abort_flag = 0;
         cutlass::arch::fence_barrier_init();
     }
@@ -1030,12 +1083,20 @@ __global__ void __launch_bounds__(kInferThreads, 1)
         atomicExch(err, 1);
     };
 
+    if constexpr (TRAIN) {
+        // prologue done; nothing of the previous step is read or overwritten before it has ended
+        griddep_launch_dependents();
+        griddep_wait();
+    }
+
     const int L = a.layers, F = 2 * a.fourier;
-    // slot s of this CTA takes tiles 2 blockIdx.x + s + 2 gridDim.x i, i = 0, 1, ...; every
+    // slot s of this CTA takes tiles kSlots (blockIdx.x + gridDim.x i) + s, i = 0, 1, ...; every
     // role walks the same (i, layer, slot) sequence and skips a slot whose tile is past the end
-    const long long stride = 2LL * gridDim.x;
-    auto tile_of = [&](int s, long long i) { return 2LL * blockIdx.x + s + i * stride; };
-    const long long iters = (a.tiles - 2LL * blockIdx.x + stride - 1) / stride;
+    const long long stride = (long long)kSlots * gridDim.x;
+    auto tile_of = [&](int s, long long i) { return (long long)kSlots * blockIdx.x + s + i * stride; };
+    const long long iters = (a.tiles - (long long)kSlots * blockIdx.x + stride - 1) / stride;
+    // the accumulator of a slot, or, with one slot, of its n-th layer product
+    auto acc_of = [&](int s, long long n) { return tmem_base + (uint32_t)((TRAIN ? (int)(n & 1) : s) * H); };
 
     if (warp == 0) {
         // ---- weight producer (lane 0)
@@ -1050,7 +1111,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
             bool stop = false;
             for (long long i = 0; i < iters && !stop; ++i)
                 for (int l = 0; l <= L && !stop; ++l)
-                    for (int s = 0; s < 2 && !stop; ++s) {
+                    for (int s = 0; s < kSlots && !stop; ++s) {
                         if (tile_of(s, i) >= a.tiles) continue;
                         const int nk = (l == 0 ? F : H) / kBK;
                         const uint32_t bytes = (uint32_t)((l == L ? Cfg::kOutN : H) * kBK * 2);
@@ -1082,7 +1143,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
         bool stop = false;
         for (long long i = 0; i < iters && !stop; ++i)
             for (int l = 0; l <= L && !stop; ++l)
-                for (int s = 0; s < 2 && !stop; ++s) {
+                for (int s = 0; s < kSlots && !stop; ++s) {
                     if (tile_of(s, i) >= a.tiles) continue;
                     // the slot's activations for this layer are written and its accumulator is free
                     if (*abort_flag || !mbar_wait_bounded(epid(s), ep_phase[s])) {
@@ -1094,7 +1155,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
                     tc_fence_after();
                     const int nk = (l == 0 ? F : H) / kBK;
                     char* act = base + s * Cfg::kActBytes;
-                    const uint32_t acc = tmem_base + (uint32_t)(s * H);
+                    const uint32_t acc = acc_of(s, i * (L + 1) + l);
                     for (int kc = 0; kc < nk; ++kc) {
                         if (*abort_flag || !mbar_wait_bounded(wfull(stage), phase)) {
                             fail();
@@ -1156,10 +1217,16 @@ __global__ void __launch_bounds__(kInferThreads, 1)
         // X[r, j] = sin(phase_j), X[r, fourier + j] = cos(phase_j), zero past the last input
         auto features = [&](int s, long long t) {
             const uint32_t act = smem_u32(base + s * Cfg::kActBytes);
-            const long long i = t * kBM + r;
-            const bool valid = i < a.n;
+            long long i = t * kBM + r;
+            bool valid;
+            if constexpr (TRAIN)
+                valid = batch_row(tr.f, (int)(t * kBM + r), i);
+            else
+                valid = i < a.n;
             float u0 = 0.f, u1 = 0.f;
             if (valid) input_point(a.u, a.cells, a.grid_n, i, u0, u1);
+            if constexpr (TRAIN)
+                if (part == 0) tr.f.yb[t * kBM + r] = valid ? (tr.f.y[i] - tr.f.y_mean) * tr.f.y_inv_std : 0.f;
             const int fq = a.fourier / 4;
             for (int g = 0; g < fq; g += 8) {
                 const int j0 = part * fq + g;
@@ -1176,9 +1243,19 @@ __global__ void __launch_bounds__(kInferThreads, 1)
                 }
                 st_shared_v4(act + act_offset(r, j0), ps[0], ps[1], ps[2], ps[3]);
                 st_shared_v4(act + act_offset(r, a.fourier + j0), pc[0], pc[1], pc[2], pc[3]);
+                if constexpr (TRAIN) {  // a warp's rows are consecutive: 64-byte pieces of X^T's rows
+                    unsigned short* xs = reinterpret_cast<unsigned short*>(tr.f.Xt) + (size_t)j0 * tr.f.rows +
+                                         (size_t)(t * kBM + r);
+                    unsigned short* xc = xs + (size_t)a.fourier * tr.f.rows;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        xs[(size_t)q * tr.f.rows] = (unsigned short)(ps[q / 2] >> (16 * (q & 1)));
+                        xc[(size_t)q * tr.f.rows] = (unsigned short)(pc[q / 2] >> (16 * (q & 1)));
+                    }
+                }
             }
         };
-        for (int s = 0; s < 2; ++s)
+        for (int s = 0; s < kSlots; ++s)
             if (tile_of(s, 0) < a.tiles) {
                 features(s, tile_of(s, 0));
                 signal(s);
@@ -1186,7 +1263,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
         bool stop = false;
         for (long long i = 0; i < iters && !stop; ++i)
             for (int l = 0; l <= L && !stop; ++l)
-                for (int s = 0; s < 2; ++s) {
+                for (int s = 0; s < kSlots; ++s) {
                     const long long t = tile_of(s, i);
                     if (t >= a.tiles) continue;
                     if (*abort_flag || !mbar_wait_bounded(accf(s), acc_phase[s])) {
@@ -1196,8 +1273,62 @@ __global__ void __launch_bounds__(kInferThreads, 1)
                     }
                     acc_phase[s] ^= 1;
                     tc_fence_after();
-                    const uint32_t tq = tmem_base + (uint32_t)(s * H) + ((uint32_t)(quad * 32) << 16);
-                    if (l < L) {
+                    const uint32_t tq = acc_of(s, i * (L + 1) + l) + ((uint32_t)(quad * 32) << 16);
+                    if (TRAIN && l < L) {
+                        if constexpr (TRAIN) {
+                            const uint32_t act = smem_u32(base);
+                            const float4* b4 = reinterpret_cast<const float4*>(a.params + a.b_off[l]);
+                            auto z_chunk = [&](int c0, uint32_t(&z)[32]) {
+                                tmem_ld32(tq + (uint32_t)c0, z);
+#pragma unroll
+                                for (int q = 0; q < 8; ++q) {
+                                    const float4 b = __ldg(b4 + c0 / 4 + q);
+                                    z[4 * q] = __float_as_uint(__fadd_rn(__uint_as_float(z[4 * q]), b.x));
+                                    z[4 * q + 1] = __float_as_uint(__fadd_rn(__uint_as_float(z[4 * q + 1]), b.y));
+                                    z[4 * q + 2] = __float_as_uint(__fadd_rn(__uint_as_float(z[4 * q + 2]), b.z));
+                                    z[4 * q + 3] = __float_as_uint(__fadd_rn(__uint_as_float(z[4 * q + 3]), b.w));
+                                }
+                            };
+#pragma unroll 1
+                            for (int c0 = part * (H / 4); c0 < (part + 1) * (H / 4); c0 += 32) {
+                                uint32_t z[32], pk[16];
+                                z_chunk(c0, z);
+#pragma unroll
+                                for (int q = 0; q < 16; ++q) {
+                                    const float2 g = gelu2(
+                                        make_float2(__uint_as_float(z[2 * q]), __uint_as_float(z[2 * q + 1])));
+                                    pk[q] = pack_bf16x2(g.x, g.y);
+                                }
+#pragma unroll
+                                for (int q = 0; q < 4; ++q)
+                                    st_shared_v4(act + act_offset(r, c0 + 8 * q), pk[4 * q], pk[4 * q + 1],
+                                                 pk[4 * q + 2], pk[4 * q + 3]);
+                            }
+                            signal(s);
+                            // beside the next layer's MMAs, which read the activations and write the
+                            // other accumulator: this accumulator is written again only after this
+                            // warp's next signal, and this row's activations by this thread alone
+                            uint32_t* stage = reinterpret_cast<uint32_t*>(base + Cfg::kActBytes +
+                                                                          (warp - 2) * Cfg::kStoreStage);
+                            const size_t m0 = (size_t)(t * kBM + quad * 32);
+#pragma unroll 1
+                            for (int c0 = part * (H / 4); c0 < (part + 1) * (H / 4); c0 += 32) {
+                                uint32_t z[32], pk[16];
+                                z_chunk(c0, z);
+                                rows_staged<32>(stage, z, reinterpret_cast<char*>(tr.Z[l] + m0 * H + c0),
+                                                (size_t)H * 4);
+#pragma unroll
+                                for (int q = 0; q < 4; ++q)
+                                    ld_shared_v4(act + act_offset(r, c0 + 8 * q), pk[4 * q], pk[4 * q + 1],
+                                                 pk[4 * q + 2], pk[4 * q + 3]);
+                                cols_staged(stage, pk, tr.Ht[l] + (size_t)c0 * tr.f.rows + m0, (size_t)tr.f.rows);
+                            }
+                            if (l == L - 1) {
+                                __syncwarp();
+                                if (lane == 0) mbar_arrive(read_bar);
+                            }
+                        }
+                    } else if (l < L) {
                         // bias + GELU -> BF16 activations of layer l + 1, over this slot's buffer
                         const uint32_t act = smem_u32(base + s * Cfg::kActBytes);
                         const float4* b4 = reinterpret_cast<const float4*>(a.params + a.b_off[l]);
@@ -1237,16 +1368,29 @@ __global__ void __launch_bounds__(kInferThreads, 1)
                                          : "r"(tq));
                             asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
                             const float* bo = a.params + a.b_off[L];
-                            const float mu = __fmaf_rn(__uint_as_float(o0), 0.5f, __ldg(bo));
-                            const float lv = __fmaf_rn(__uint_as_float(o1), 0.5f, __ldg(bo + 1));
-                            const long long row = t * kBM + r;
-                            if (row < a.n) {
-                                a.mean[row] = __fmaf_rn(mu, a.y_std, a.y_mean);
-                                a.sd[row] = __fmul_rn(expf(0.5f * fminf(fmaxf(lv, -16.f), 16.f)), a.y_std);
+                            if constexpr (TRAIN) {
+                                nll_rows(tr.loss, (int)(t * kBM + r), __fadd_rn(__uint_as_float(o0), __ldg(bo)),
+                                         __fadd_rn(__uint_as_float(o1), __ldg(bo + 1)));
+                            } else {
+                                const float mu = __fmaf_rn(__uint_as_float(o0), 0.5f, __ldg(bo));
+                                const float lv = __fmaf_rn(__uint_as_float(o1), 0.5f, __ldg(bo + 1));
+                                const long long row = t * kBM + r;
+                                if (row < a.n) {
+                                    a.mean[row] = __fmaf_rn(mu, a.y_std, a.y_mean);
+                                    a.sd[row] = __fmul_rn(expf(0.5f * fminf(fmaxf(lv, -16.f), 16.f)), a.y_std);
+                                }
                             }
                         }
                         const long long tn = tile_of(s, i + 1);
                         if (tn < a.tiles) {
+                            if constexpr (TRAIN) {
+                                // a warp's features lie over columns that other warps still read back
+                                if (*abort_flag || !mbar_wait_bounded(read_bar, (uint32_t)(i & 1))) {
+                                    fail();
+                                    stop = true;
+                                    break;
+                                }
+                            }
                             features(s, tn);
                             signal(s);
                         }
@@ -1418,12 +1562,14 @@ bool set_gemm_attributes(int device, std::string& err) {
         if (ce == cudaSuccess) ce = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     });
     if (!cu_ok(ce, err, "cudaFuncSetAttribute(gemm)")) return false;
-    ce = cudaFuncSetAttribute(ucbmlp::mlp_infer_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              ucbmlp::InferCfg<128>::kSmem);
-    if (!cu_ok(ce, err, "cudaFuncSetAttribute(infer 128)")) return false;
-    ce = cudaFuncSetAttribute(ucbmlp::mlp_infer_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              ucbmlp::InferCfg<256>::kSmem);
-    if (!cu_ok(ce, err, "cudaFuncSetAttribute(infer 256)")) return false;
+    auto attribute = [&](auto kernel, int smem) {
+        if (ce == cudaSuccess) ce = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    };
+    attribute(ucbmlp::mlp_infer_kernel<128, false>, ucbmlp::InferCfg<128>::kSmem);
+    attribute(ucbmlp::mlp_infer_kernel<256, false>, ucbmlp::InferCfg<256>::kSmem);
+    attribute(ucbmlp::mlp_infer_kernel<128, true>, ucbmlp::InferCfg<128, true>::kSmem);
+    attribute(ucbmlp::mlp_infer_kernel<256, true>, ucbmlp::InferCfg<256, true>::kSmem);
+    if (!cu_ok(ce, err, "cudaFuncSetAttribute(forward)")) return false;
     g_attr_devices.push_back(device);
     return true;
 }
@@ -1534,6 +1680,37 @@ ucbmlp::Epilogue epi() {
     return ep;
 }
 
+// Whether the fused forward kernel covers this network (hidden width 128 or 256, features no
+// wider than a hidden layer).
+bool fused_supported(const Mlp& m) {
+    return (m.H == 128 || m.H == 256) && m.F <= m.H && m.F % ucbmlp::kBK == 0 && (m.F / 2) % 32 == 0 &&
+           m.L + 1 <= ucbmlp::kMaxLayers;
+}
+
+// What the fused forward kernel takes for prediction and training alike.
+bool fused_args(Mlp& m, const MlpInputs& in, ucbmlp::InferMaps& maps, ucbmlp::InferArgs& a, std::string& err) {
+    std::memset(&maps, 0, sizeof maps);
+    for (int l = 0; l < m.L; ++l)
+        if (!tensor_map(&maps.w[l], m.W[l], m.H, m.in[l], m.H, err)) return false;
+    if (!tensor_map(&maps.w[m.L], m.W[m.L], m.out_pad[m.L], m.H, ucbmlp::InferCfg<256>::kOutN, err)) return false;
+    a.u = in.u;
+    a.cells = in.cells;
+    a.n = in.n;
+    a.grid_n = in.grid_n;
+    a.Bf = m.Bf;
+    a.fourier = m.cfg.fourier;
+    a.layers = m.L;
+    a.params = m.p;
+    for (int l = 0; l <= m.L; ++l) {
+        if (m.b_off[l] % 4) {
+            err = "fused forward pass: bias not 16-byte aligned";
+            return false;
+        }
+        a.b_off[l] = m.b_off[l];
+    }
+    return true;
+}
+
 bool ensure_rows(Mlp& m, int rows, std::string& err) {
     if (rows <= m.rows) return true;
     if (m.graph) {
@@ -1548,11 +1725,13 @@ bool ensure_rows(Mlp& m, int rows, std::string& err) {
     m.rows = 0;
     auto& o = m.act_owned;
     const size_t R = rows;
-    if (!(m.X = dalloc<bf16>(R * m.F, o, err, "features")) || !(m.Xt = dalloc<bf16>(R * m.F, o, err, "features^T")))
+    // the fused forward pass keeps the row-major features and activations on chip
+    const size_t Rm = fused_supported(m) ? 0 : R;
+    if (!(m.X = dalloc<bf16>(Rm * m.F, o, err, "features")) || !(m.Xt = dalloc<bf16>(R * m.F, o, err, "features^T")))
         return false;
     for (int l = 0; l < m.L; ++l) {
         float* z = dalloc<float>(R * m.H, o, err, "Z");
-        bf16* h = dalloc<bf16>(R * m.H, o, err, "H");
+        bf16* h = dalloc<bf16>(Rm * m.H, o, err, "H");
         bf16* ht = dalloc<bf16>(R * m.H, o, err, "H^T");
         if (!z || !h || !ht) return false;
         m.Z.push_back(z);
@@ -1648,6 +1827,18 @@ bool features(Mlp& m, const ucbmlp::FeatureArgs& a, cudaStream_t st, std::string
                   "features launch", a);
 }
 
+// The loss of the first n_valid of `rows` rows against m.yb, and its gradients.
+void loss_epilogue(const Mlp& m, int rows, int n_valid, ucbmlp::Epilogue& ep) {
+    ep.nll = 1;
+    ep.yb = m.yb;
+    ep.n_valid = n_valid;
+    ep.rows = rows;
+    ep.beta = m.cfg.beta_nll;
+    ep.dout = m.dout;
+    ep.doutT = m.doutT;
+    ep.blk = m.blk;
+}
+
 // Forward pass over `rows` rows of m.X. keep: store Z and H^T for the backward pass and
 // evaluate the loss of the first n_valid rows against m.yb (dOut, dOut^T, block sums).
 bool forward(Mlp& m, int rows, bool keep, cudaStream_t st, std::string& err, int n_valid = 0) {
@@ -1674,17 +1865,40 @@ bool forward(Mlp& m, int rows, bool keep, cudaStream_t st, std::string& err, int
     ep.outf = m.outp;
     ep.ldf = 2;
     ep.n_store = 2;
-    if (keep) {
-        ep.nll = 1;
-        ep.yb = m.yb;
-        ep.n_valid = n_valid;
-        ep.rows = rows;
-        ep.beta = m.cfg.beta_nll;
-        ep.dout = m.dout;
-        ep.doutT = m.doutT;
-        ep.blk = m.blk;
-    }
+    if (keep) loss_epilogue(m, rows, n_valid, ep);
     return gemm(m, x, m.W[m.L], rows, m.out_pad[m.L], m.H, ep, st, err);
+}
+
+// The forward half of a training step: the features of fa's rows, the hidden layers and the
+// loss of the first n_valid rows. Networks that the fused kernel covers take it at every batch
+// size; us a training step, a layer a launch -> fused:
+//   4 layers of 128: batch 1,024 89.4 -> 72.2, 8,192 95.1 -> 76.6, 16,384 114 -> 93, 65,536 359 -> 330
+//   256 wide (layers): 1,024 (4) 97.8 -> 97.7, 2,048 (4) 98.0 -> 99.7, 4,096 (3) 82.7 -> 81.0,
+//   8,192 (4) 130.6 -> 130.8, 16,384 (5) 218 -> 199, 32,768 (4) 330 -> 307, 65,536 (4) 593 -> 563
+// (at 256 the layer kernels split a CTA's rows in two tiles, so they keep twice the SMs busy while
+// the batch has fewer tiles than SMs: the two forms meet there).
+bool forward_train(Mlp& m, const MlpInputs& in, const ucbmlp::FeatureArgs& fa, int rows, int n_valid, cudaStream_t st,
+                   std::string& err) {
+    if (!fused_supported(m)) return features(m, fa, st, err) && forward(m, rows, true, st, err, n_valid);
+    ucbmlp::InferMaps maps;
+    ucbmlp::InferArgs a{};
+    if (!fused_args(m, in, maps, a, err)) return false;
+    a.tiles = rows / ucbmlp::kBM;
+    ucbmlp::TrainArgs t{};
+    t.f = fa;
+    for (int l = 0; l < m.L; ++l) {
+        t.Z[l] = m.Z[l];
+        t.Ht[l] = m.Ht[l];
+    }
+    loss_epilogue(m, rows, n_valid, t.loss);
+    const int grid = (int)std::min<long long>(a.tiles, std::max(m.e->sm_count, 1));
+    m.e->launches += 1;
+    auto go = [&](auto kernel, int smem) {
+        return launch(m.pdl, kernel, dim3(grid), dim3(ucbmlp::kInferThreads), smem, st, err, "forward launch", maps, a,
+                      t, m.err);
+    };
+    return m.H == 256 ? go(ucbmlp::mlp_infer_kernel<256, true>, ucbmlp::InferCfg<256, true>::kSmem)
+                      : go(ucbmlp::mlp_infer_kernel<128, true>, ucbmlp::InferCfg<128, true>::kSmem);
 }
 
 // Inference forward pass over `rows` rows of m.pX (activations ping-pong in m.pH).
@@ -1847,13 +2061,13 @@ bool check_kernel_error(Mlp& m, cudaStream_t st, std::string& err) {
 // One training step (features of a random batch, forward with the loss in the output
 // layer's epilogue, backward, and the optimiser kernel: gradient sums, Adam, BF16 weights,
 // step count): the sequence that is captured into a CUDA graph, 16 kernels for 4 hidden
-// layers.
+// layers, 11 where the forward pass is one.
 bool train_step(Mlp& m, const MlpInputs& in, const float* d_y, cudaStream_t st, std::string& err) {
     const int rows = m.cfg.batch;
     ucbmlp::FeatureArgs fa = feature_args(m, in, 0, rows, true);
     fa.y = d_y;
     fa.yb = m.yb;
-    return features(m, fa, st, err) && forward(m, rows, true, st, err, rows) && backward(m, rows, st, err) &&
+    return forward_train(m, in, fa, rows, rows, st, err) && backward(m, rows, st, err) &&
            adam(m, rows, true, st, err);
 }
 
@@ -1949,35 +2163,10 @@ void mlp_destroy(Mlp* m) {
 long long mlp_param_count(const Mlp* m) { return m ? m->n_params : 0; }
 int mlp_features(const Mlp* m) { return m ? m->F : 0; }
 
-// Whether the fused prediction kernel covers this network (hidden width 128 or 256, features
-// no wider than a hidden layer).
-static bool fused_predict_supported(const Mlp& m) {
-    return (m.H == 128 || m.H == 256) && m.F <= m.H && m.F % ucbmlp::kBK == 0 && (m.F / 2) % 32 == 0 &&
-           m.L + 1 <= ucbmlp::kMaxLayers;
-}
-
 static bool predict_fused(Mlp& m, const MlpInputs& in, float* d_mean, float* d_std, cudaStream_t st, std::string& err) {
     ucbmlp::InferMaps maps;
-    std::memset(&maps, 0, sizeof maps);
-    for (int l = 0; l < m.L; ++l)
-        if (!tensor_map(&maps.w[l], m.W[l], m.H, m.in[l], m.H, err)) return false;
-    if (!tensor_map(&maps.w[m.L], m.W[m.L], m.out_pad[m.L], m.H, ucbmlp::InferCfg<256>::kOutN, err)) return false;
     ucbmlp::InferArgs a{};
-    a.u = in.u;
-    a.cells = in.cells;
-    a.n = in.n;
-    a.grid_n = in.grid_n;
-    a.Bf = m.Bf;
-    a.fourier = m.cfg.fourier;
-    a.layers = m.L;
-    a.params = m.p;
-    for (int l = 0; l <= m.L; ++l) {
-        if (m.b_off[l] % 4) {
-            err = "fused prediction: bias not 16-byte aligned";
-            return false;
-        }
-        a.b_off[l] = m.b_off[l];
-    }
+    if (!fused_args(m, in, maps, a, err)) return false;
     a.y_mean = m.y_mean;
     a.y_std = m.y_std;
     a.mean = d_mean;
@@ -1986,16 +2175,18 @@ static bool predict_fused(Mlp& m, const MlpInputs& in, float* d_mean, float* d_s
     const long long pairs = (a.tiles + 1) / 2;
     const int grid = (int)std::min<long long>(pairs, std::max(m.e->sm_count, 1));
     if (m.H == 256)
-        ucbmlp::mlp_infer_kernel<256><<<grid, ucbmlp::kInferThreads, ucbmlp::InferCfg<256>::kSmem, st>>>(maps, a, m.err);
+        ucbmlp::mlp_infer_kernel<256, false>
+            <<<grid, ucbmlp::kInferThreads, ucbmlp::InferCfg<256>::kSmem, st>>>(maps, a, {}, m.err);
     else
-        ucbmlp::mlp_infer_kernel<128><<<grid, ucbmlp::kInferThreads, ucbmlp::InferCfg<128>::kSmem, st>>>(maps, a, m.err);
+        ucbmlp::mlp_infer_kernel<128, false>
+            <<<grid, ucbmlp::kInferThreads, ucbmlp::InferCfg<128>::kSmem, st>>>(maps, a, {}, m.err);
     m.e->launches += 1;
     return cu_ok(cudaPeekAtLastError(), err, "fused prediction launch");
 }
 
 bool mlp_predict(Mlp* m, const MlpInputs& in, float* d_mean, float* d_std, cudaStream_t st, std::string& err) {
     if (in.n <= 0) return true;
-    if (fused_predict_supported(*m)) return predict_fused(*m, in, d_mean, d_std, st, err);
+    if (fused_supported(*m)) return predict_fused(*m, in, d_mean, d_std, st, err);
     const long long chunk = 1 << 18;
     const long long rows_needed = std::min<long long>(chunk, ((in.n + 127) / 128) * 128);
     if (!ensure_pred_rows(*m, (int)rows_needed, err)) return false;
@@ -2186,7 +2377,7 @@ int ucb_mlp_loss_grad(ucb_mlp* h, const float* u, const float* y, long long n, f
         fa.Xt = m.Xt;
         fa.y = dy;
         fa.yb = m.yb;
-        if (!features(m, fa, st, err) || !forward(m, rows, true, st, err, (int)n) || !backward(m, rows, st, err) ||
+        if (!forward_train(m, in, fa, rows, (int)n, st, err) || !backward(m, rows, st, err) ||
             !adam(m, rows, false, st, err) || !check_kernel_error(m, st, err) ||
             !cu_ok(cudaMemcpy(grad, m.g, m.n_params * sizeof(float), cudaMemcpyDeviceToHost), err, "read grad") ||
             !cu_ok(cudaMemcpy(loss, m.loss, sizeof(float), cudaMemcpyDeviceToHost), err, "read loss"))
