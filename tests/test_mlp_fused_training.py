@@ -1,6 +1,7 @@
 """The one-launch forward pass of a training batch (hidden widths 128 and 256): loss and gradient
 against the CPU oracle where it can go wrong: one tile, rows that are padded, a second tile on
-some CTAs."""
+some CTAs. A width of 384 goes a layer a launch; its weight gradients, like all, read the
+activations and dL/dZ row-major, here over three column tiles."""
 import numpy as np
 import pytest
 
@@ -19,7 +20,7 @@ def ucb_engine():
 # 148 SMs: 149 tiles give one CTA a second tile
 @pytest.mark.gpu
 @pytest.mark.parametrize("hidden,layers,rows", [(128, 1, 5), (128, 3, 128), (128, 2, 300), (128, 3, 149 * 128 - 7),
-                                                (256, 1, 128), (256, 2, 73 * 128 + 1), (256, 2, 150 * 128)])
+                                                (256, 1, 128), (256, 2, 73 * 128 + 1), (256, 2, 150 * 128), (384, 2, 300)])
 def test_gradient_matches_the_oracle(ucb_engine, hidden, layers, rows):
     import ucb
 

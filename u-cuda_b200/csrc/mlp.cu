@@ -10,13 +10,13 @@
 // -> FP32) from one elected lane into one of two TMEM accumulators, and warps 2-17 read a
 // finished accumulator with tcgen05.ld (four warps per 32-lane TMEM quadrant, a quarter of
 // the columns each; thread t of a quadrant owns row t) while the next tile's MMAs run,
-// apply bias / GELU and store FP32, BF16 and / or transposed BF16 copies through a per-warp
+// apply bias / GELU and store FP32 and / or BF16 copies through a per-warp
 // shared-memory staging buffer (whole 16-byte pieces per store instruction). Waits are
 // bounded; on a timeout the kernel records an error, waits for its own copies and MMAs,
 // frees TMEM and returns. A split-K launch stores each split's partial tile in its own
 // slice of a buffer, and the optimiser kernel adds the slices in split order (so a
-// training step gives the same bits every time it runs). Backward products are the same TN
-// GEMM on transposed copies, which the forward and dL/dZ epilogues write as they go.
+// training step gives the same bits every time it runs). The weight gradients, whose K is the
+// batch, read dL/dZ and the activations row-major, contiguous along M and N (GemmCfg's MN form).
 //
 // Prediction: one fused kernel per call (mlp_infer_kernel) runs features, every hidden
 // layer and the output transform of a 128-row tile inside one CTA, with the activations in
@@ -59,14 +59,20 @@ constexpr int kGemmThreads = 64 + 32 * kEpiWarps;  // warp 0 TMA, warp 1 MMA, wa
 constexpr int kMaxLayers = 9;     // hidden layers + the output layer
 
 // Shapes and shared-memory layout of the persistent GEMM for a tile width BN (128 or 256).
-template <int BN>
+// MN: the operands are A [K, M] and B [K, N], contiguous along M and N (the weight gradients read
+// dL/dZ and the activations as the other products left them). A stage then holds an operand as
+// chunks of 64 columns, each 64 rows of K by 128 swizzled bytes: what one TMA box writes.
+template <int BN, bool MN = false>
 struct GemmCfg {
-    using MmaOp = SM100_MMA_F16BF16_SS<bf16, bf16, float, kBM, BN, UMMA::Major::K, UMMA::Major::K>;
+    static constexpr UMMA::Major kMajor = MN ? UMMA::Major::MN : UMMA::Major::K;
+    using Atom = std::conditional_t<MN, UMMA::Layout_MN_SW128_Atom<bf16>, UMMA::Layout_K_SW128_Atom<bf16>>;
+    using Order = std::conditional_t<MN, Step<_2, _1>, Step<_1, _2>>;  // which of (M or N, K) tiles first
+    using MmaOp = SM100_MMA_F16BF16_SS<bf16, bf16, float, kBM, BN, kMajor, kMajor>;
     using TiledMma = decltype(make_tiled_mma(MmaOp{}));
     using LayoutA = decltype(UMMA::tile_to_mma_shape(
-        UMMA::Layout_K_SW128_Atom<bf16>{}, partition_shape_A(TiledMma{}, make_shape(Int<kBM>{}, Int<kBK>{}))));
+        Atom{}, partition_shape_A(TiledMma{}, make_shape(Int<kBM>{}, Int<kBK>{})), Order{}));
     using LayoutB = decltype(UMMA::tile_to_mma_shape(
-        UMMA::Layout_K_SW128_Atom<bf16>{}, partition_shape_B(TiledMma{}, make_shape(Int<BN>{}, Int<kBK>{}))));
+        Atom{}, partition_shape_B(TiledMma{}, make_shape(Int<BN>{}, Int<kBK>{})), Order{}));
     static constexpr int kStages = BN == 256 ? 3 : 4;
     static constexpr int kABytes = kBM * kBK * 2;
     static constexpr int kBBytes = BN * kBK * 2;
@@ -83,34 +89,30 @@ struct GemmCfg {
 struct Epilogue {
     const float* bias;  // bias[n] for n < nb (0 beyond)
     int nb;
-    int gelu;           // outh / outt receive GELU(v) instead of v
+    int gelu;           // outh receives GELU(v) instead of v
     float* outf;        // FP32 result (pre-activation), row stride ldf
     int ldf;
     int atomic;         // split-K: outf is a buffer of partial tiles, one slice per K split
     long long split_stride;  // floats between the slices of consecutive splits
     bf16* outh;         // BF16 copy, row stride ldh
     int ldh;
-    bf16* outt;         // BF16 transposed copy outt[n * ldt + m]
-    int ldt;
     int m_store, n_store;  // only rows m < m_store and columns n < n_store are stored
-    // backward through GELU: the product is dL/dH of a hidden layer; outh / outt receive
+    // backward through GELU: the product is dL/dH of a hidden layer; outh receives
     // dZ = dL/dH GELU'(Z) with Z = zin (FP32, row stride ldz)
     const float* zin;
     int ldz;
-    // sums over each 32-row block of the BF16 values stored to outh / outt (the bias gradient
+    // sums over each 32-row block of the BF16 values stored to outh (the bias gradient
     // of dZ): colsum[(m / 32) ldc + n]
     float* colsum;
     int ldc;
     // output layer of a training batch (columns 0 = mean, 1 = log-variance): the beta-NLL
     // against the standardised targets yb of the first n_valid of `rows` rows -> dout (row
-    // stride 64, columns 0 and 1), doutT (rows 0 and 1 of a [128, rows] matrix), and per
-    // 32-row block the sums of the two BF16 gradients and of the loss in blk[3 (m / 32) + 0..2]
+    // stride 64, columns 0 and 1), and per 32-row block the sums of the two BF16 gradients and of the loss in blk[3 (m / 32) + 0..2]
     int nll;
     const float* yb;
     int n_valid, rows;
     float beta;
     bf16* dout;
-    bf16* doutT;
     float* blk;
 };
 
@@ -219,7 +221,7 @@ __device__ __forceinline__ int column_sums32(float (&v)[32]) {
 }
 
 // Beta-NLL of one output row (mean mu, log-variance lv_raw) of a training batch, the
-// gradients dout / doutT, and the fixed-order sums over the warp's 32 rows into blk.
+// gradients dout, and the fixed-order sums over the warp's 32 rows into blk.
 __device__ __forceinline__ void nll_rows(const Epilogue& ep, int r, float mu, float lv_raw) {
     float g0 = 0.f, g1 = 0.f, l = 0.f;
     if (r < ep.rows && r < ep.n_valid) {
@@ -236,8 +238,6 @@ __device__ __forceinline__ void nll_rows(const Epilogue& ep, int r, float mu, fl
     if (r < ep.rows) {
         ep.dout[(size_t)r * 64] = b0;
         ep.dout[(size_t)r * 64 + 1] = b1;
-        ep.doutT[r] = b0;
-        ep.doutT[(size_t)ep.rows + r] = b1;
     }
     float s0 = float(b0), s1 = float(b1), sl = l;
 #pragma unroll
@@ -254,16 +254,16 @@ __device__ __forceinline__ void nll_rows(const Epilogue& ep, int r, float mu, fl
 }
 
 // One 32-column chunk of one accumulator row (this thread's) through the epilogue: bias,
-// the FP32 / BF16 / transposed BF16 stores. v: the raw accumulator values.
+// the FP32 / BF16 stores. v: the raw accumulator values.
 // Epilogue features compiled into a GEMM instantiation (a launch only runs the code of its
 // own mode: with one tile per CTA, as in a training step, every CTA executes the epilogue
 // once, so code it does not need costs instruction fetches from L2).
 enum : int {
-    kEpBias = 1, kEpGelu = 2, kEpOutF = 4, kEpOutH = 8, kEpOutT = 16, kEpZin = 32, kEpColsum = 64, kEpNll = 128,
-    kEpAll = 255,
-    kModeForward = kEpBias | kEpGelu | kEpOutF | kEpOutH | kEpOutT,  // hidden layer of a training batch
+    kEpBias = 1, kEpGelu = 2, kEpOutF = 4, kEpOutH = 8, kEpZin = 16, kEpColsum = 32, kEpNll = 64,
+    kEpAll = 127,
+    kModeForward = kEpBias | kEpGelu | kEpOutF | kEpOutH,  // hidden layer of a training batch
     kModeLoss = kEpBias | kEpOutF | kEpNll,                           // output layer of a training batch
-    kModeDz = kEpZin | kEpOutH | kEpOutT | kEpColsum,                 // dL/dZ of a hidden layer
+    kModeDz = kEpZin | kEpOutH | kEpColsum,                 // dL/dZ of a hidden layer
     kModeSplit = kEpOutF,                                             // split-K slices
     kModeHidden = kEpBias | kEpGelu | kEpOutH,                        // prediction, hidden layer
     kModeOut = kEpBias | kEpOutF,                                     // prediction, output layer
@@ -294,44 +294,6 @@ __device__ __forceinline__ void rows_staged(uint32_t* stage, const uint32_t (&va
     }
     __syncwarp();
 }
-// Transposed BF16: column j of the chunk (its 32 rows) to outt + j * ld (elements; outt points
-// at column 0, row 0 of the warp). The buffer holds the chunk column-major, so each column's
-// 64 bytes are contiguous; a store instruction writes 16-byte pieces of eight columns.
-__device__ __forceinline__ void cols_from_stage(const uint32_t* stage, bf16* outt, size_t ld) {
-    const int lane = threadIdx.x & 31;
-    const uint4* s4 = reinterpret_cast<const uint4*>(stage);
-#pragma unroll
-    for (int pass = 0; pass < 4; ++pass) {
-        const int j = pass * 8 + lane / 4, q = lane % 4;
-        *reinterpret_cast<uint4*>(outt + (size_t)j * ld + q * 8) = s4[j * 4 + q];
-    }
-    __syncwarp();
-}
-__device__ __forceinline__ void cols_staged(uint32_t* stage, const float (&g)[32], bf16* outt, size_t ld) {
-    const int lane = threadIdx.x & 31;
-    unsigned short* s2 = reinterpret_cast<unsigned short*>(stage);
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-        const bf16 b = bf16(g[j]);
-        s2[j * 32 + lane] = *reinterpret_cast<const unsigned short*>(&b);
-    }
-    __syncwarp();
-    cols_from_stage(stage, outt, ld);
-}
-
-// The same from a row's 32 values already rounded to BF16, two a word.
-__device__ __forceinline__ void cols_staged(uint32_t* stage, const uint32_t (&pk)[16], bf16* outt, size_t ld) {
-    const int lane = threadIdx.x & 31;
-    unsigned short* s2 = reinterpret_cast<unsigned short*>(stage);
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        s2[(2 * j) * 32 + lane] = (unsigned short)(pk[j] & 0xffffu);
-        s2[(2 * j + 1) * 32 + lane] = (unsigned short)(pk[j] >> 16);
-    }
-    __syncwarp();
-    cols_from_stage(stage, outt, ld);
-}
-
 template <int MODE>
 __device__ __forceinline__ void epilogue_chunk(const Epilogue& ep, float* outf, int m, int n0, float (&v)[32],
                                                uint32_t* stage) {
@@ -377,7 +339,7 @@ __device__ __forceinline__ void epilogue_chunk(const Epilogue& ep, float* outf, 
         }
     }
     if ((MODE & kEpNll) && ep.nll && n0 == 0) nll_rows(ep, m, v[0], v[1]);
-    if (!(MODE & (kEpOutH | kEpOutT)) || (!ep.outh && !ep.outt)) return;
+    if (!(MODE & kEpOutH) || !ep.outh) return;
     float g[32];
     if ((MODE & kEpZin) && ep.zin) {
         if (row_ok && full && (ep.ldz & 3) == 0) {
@@ -435,15 +397,6 @@ __device__ __forceinline__ void epilogue_chunk(const Epilogue& ep, float* outf, 
                 if (n0 + j < ep.n_store) p[j] = bf16(g[j]);
         }
     }
-    if ((MODE & kEpOutT) && ep.outt && warp_rows && full && (ep.ldt & 7) == 0 &&
-        (reinterpret_cast<uintptr_t>(ep.outt) & 15) == 0) {
-        cols_staged(stage, g, ep.outt + (size_t)n0 * ep.ldt + m0, (size_t)ep.ldt);
-    } else if ((MODE & kEpOutT) && ep.outt && row_ok) {
-        // consecutive threads own consecutive rows: each column's stores are contiguous
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-            if (n0 + j < ep.n_store) ep.outt[(size_t)(n0 + j) * ep.ldt + m] = bf16(g[j]);
-    }
     if ((MODE & kEpColsum) && ep.colsum) {
         // column sums over the warp's 32 rows of the BF16-rounded values (rows past m_store
         // add 0): a fixed butterfly that leaves column n0 + lane in lane `lane`
@@ -468,7 +421,8 @@ template <int BN, int MODE>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     gemm_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmWork w,
                     Epilogue ep, int* err) {
-    using Cfg = GemmCfg<BN>;
+    constexpr bool kMN = MODE == kModeSplit;
+    using Cfg = GemmCfg<BN, kMN>;
     constexpr int S = Cfg::kStages;
     typename Cfg::TiledMma tiled_mma;
     extern __shared__ char smem_raw[];
@@ -533,8 +487,20 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                     }
                     const uint32_t a_dst = smem_u32(base + stage * Cfg::kStageBytes);
                     mbar_expect_tx(full_bar(stage), Cfg::kStageBytes);
-                    tma_load_2d(a_dst, &tmA, full_bar(stage), (kt0 + i) * kBK, tm * kBM);
-                    tma_load_2d(a_dst + Cfg::kABytes, &tmB, full_bar(stage), (kt0 + i) * kBK, tn * BN);
+                    if constexpr (kMN) {
+                        constexpr int kChunk = kBK * kBK * 2;
+#pragma unroll
+                        for (int c = 0; c < kBM / kBK; ++c)
+                            tma_load_2d(a_dst + c * kChunk, &tmA, full_bar(stage), tm * kBM + c * kBK,
+                                        (kt0 + i) * kBK);
+#pragma unroll
+                        for (int c = 0; c < BN / kBK; ++c)
+                            tma_load_2d(a_dst + Cfg::kABytes + c * kChunk, &tmB, full_bar(stage), tn * BN + c * kBK,
+                                        (kt0 + i) * kBK);
+                    } else {
+                        tma_load_2d(a_dst, &tmA, full_bar(stage), (kt0 + i) * kBK, tm * kBM);
+                        tma_load_2d(a_dst + Cfg::kABytes, &tmB, full_bar(stage), (kt0 + i) * kBK, tn * BN);
+                    }
                     ++issued[stage];
                     if (++stage == S) {
                         stage = 0;
@@ -675,7 +641,6 @@ struct FeatureArgs {
     int fourier;
     int rows;                  // rows of this chunk (multiple of 128)
     bf16* X;                   // rows x 2 fourier
-    bf16* Xt;                  // 2 fourier x rows (optional)
 };
 
 __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
@@ -723,8 +688,7 @@ __device__ __forceinline__ bool batch_row(const FeatureArgs& a, int r, long long
 }
 
 // X[r, j] = sin(2 pi u.B_j), X[r, fourier + j] = cos(...). One thread per (row, group of
-// 8 frequencies); consecutive threads take consecutive rows of one group, so the transposed
-// copy's stores are contiguous across a warp and each row's 8 values go out as 16 bytes.
+// 8 frequencies); each row's 8 values go out as 16 bytes.
 __global__ void features_kernel(FeatureArgs a) {
     griddep_launch_dependents();
     griddep_wait();
@@ -754,13 +718,6 @@ __global__ void features_kernel(FeatureArgs a) {
 #undef UCB_PACK
     *reinterpret_cast<uint4*>(a.X + (size_t)r * F + j0) = ps;
     *reinterpret_cast<uint4*>(a.X + (size_t)r * F + a.fourier + j0) = pc;
-    if (a.Xt) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            a.Xt[(size_t)(j0 + q) * a.rows + r] = bf16(sv[q]);
-            a.Xt[(size_t)(a.fourier + j0 + q) * a.rows + r] = bf16(cv[q]);
-        }
-    }
     if (j0 == 0 && a.yb) a.yb[r] = valid ? (a.y[i] - a.y_mean) * a.y_inv_std : 0.f;
 }
 
@@ -941,14 +898,14 @@ __global__ void unscale_kernel(const float* out, int rows, long long n_left, flo
 // TRAIN: the forward half of a training step (features of the batch's rows, hidden layers,
 // output layer and loss) with the same roles. Rows do not mix before the weight gradients, so
 // a CTA carries its 128 rows through every layer, and what the backward pass reads leaves on
-// the way: the features and the activations transposed, Z, and the loss's gradients. A batch
+// the way: the features, Z, the activations, and the loss's gradients. A batch
 // has few tiles, so each CTA keeps one in flight and its two TMEM accumulators alternate by
 // layer: the epilogue first writes the next layer's operand and releases the MMAs, then reads
-// the accumulator once more and stores Z and H^T while they run. The space of the second
+// the accumulator once more and stores Z and H while they run. The space of the second
 // tile's activations stages those stores. A layer a launch was bound by latency (launch,
 // prologue, one tile's loads, MMAs and epilogue, drain: 9-10 us for a microsecond of MMAs).
-// Here a layer of 128 is 4 us of a CTA, one of 256 is 8.5 us (the stores' passes through shared
-// memory); forward_train has the times of a step.
+// A CTA is bound by its epilogue (the stores' passes through shared memory, GELU); forward_train
+// has the times of a step.
 struct InferMaps {
     CUtensorMap w[kMaxLayers];  // layer l's BF16 weights [rows, K]: boxes of 64 (K) x H rows (16 for the output layer)
 };
@@ -971,9 +928,9 @@ struct InferArgs {
 
 // What the forward pass of a training step takes and leaves besides (TRAIN).
 struct TrainArgs {
-    FeatureArgs f;           // the batch's rows; Xt and yb are written, X is not
+    FeatureArgs f;           // the batch's rows
     float* Z[kMaxLayers];    // rows x H pre-activations of each hidden layer
-    bf16* Ht[kMaxLayers];    // H x rows activations
+    bf16* H[kMaxLayers];     // rows x H activations
     Epilogue loss;           // the fields of nll_rows
 };
 struct NoTrainArgs {};
@@ -1243,15 +1200,10 @@ __global__ void __launch_bounds__(kInferThreads, 1)
                 }
                 st_shared_v4(act + act_offset(r, j0), ps[0], ps[1], ps[2], ps[3]);
                 st_shared_v4(act + act_offset(r, a.fourier + j0), pc[0], pc[1], pc[2], pc[3]);
-                if constexpr (TRAIN) {  // a warp's rows are consecutive: 64-byte pieces of X^T's rows
-                    unsigned short* xs = reinterpret_cast<unsigned short*>(tr.f.Xt) + (size_t)j0 * tr.f.rows +
-                                         (size_t)(t * kBM + r);
-                    unsigned short* xc = xs + (size_t)a.fourier * tr.f.rows;
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        xs[(size_t)q * tr.f.rows] = (unsigned short)(ps[q / 2] >> (16 * (q & 1)));
-                        xc[(size_t)q * tr.f.rows] = (unsigned short)(pc[q / 2] >> (16 * (q & 1)));
-                    }
+                if constexpr (TRAIN) {
+                    bf16* x = tr.f.X + (size_t)(t * kBM + r) * F + j0;
+                    *reinterpret_cast<uint4*>(x) = make_uint4(ps[0], ps[1], ps[2], ps[3]);
+                    *reinterpret_cast<uint4*>(x + a.fourier) = make_uint4(pc[0], pc[1], pc[2], pc[3]);
                 }
             }
         };
@@ -1307,21 +1259,24 @@ __global__ void __launch_bounds__(kInferThreads, 1)
                             signal(s);
                             // beside the next layer's MMAs, which read the activations and write the
                             // other accumulator: this accumulator is written again only after this
-                            // warp's next signal, and this row's activations by this thread alone
+                            // warp's next signal, and this part of the activations by this warp alone
                             uint32_t* stage = reinterpret_cast<uint32_t*>(base + Cfg::kActBytes +
                                                                           (warp - 2) * Cfg::kStoreStage);
                             const size_t m0 = (size_t)(t * kBM + quad * 32);
 #pragma unroll 1
                             for (int c0 = part * (H / 4); c0 < (part + 1) * (H / 4); c0 += 32) {
-                                uint32_t z[32], pk[16];
+                                uint32_t z[32];
                                 z_chunk(c0, z);
                                 rows_staged<32>(stage, z, reinterpret_cast<char*>(tr.Z[l] + m0 * H + c0),
                                                 (size_t)H * 4);
+                                // the warp's 32 x 32 activations: eight rows of 64 bytes a store
 #pragma unroll
-                                for (int q = 0; q < 4; ++q)
-                                    ld_shared_v4(act + act_offset(r, c0 + 8 * q), pk[4 * q], pk[4 * q + 1],
-                                                 pk[4 * q + 2], pk[4 * q + 3]);
-                                cols_staged(stage, pk, tr.Ht[l] + (size_t)c0 * tr.f.rows + m0, (size_t)tr.f.rows);
+                                for (int q = 0; q < 4; ++q) {
+                                    const int row = 8 * q + lane / 4, col = c0 + 8 * (lane % 4);
+                                    uint4 h;
+                                    ld_shared_v4(act + act_offset(quad * 32 + row, col), h.x, h.y, h.z, h.w);
+                                    *reinterpret_cast<uint4*>(tr.H[l] + (m0 + row) * H + col) = h;
+                                }
                             }
                             if (l == L - 1) {
                                 __syncwarp();
@@ -1471,13 +1426,13 @@ struct Mlp {
     float* loss = nullptr;
     float y_mean = 0.f, y_std = 1.f;
     int rows = 0;                  // activation capacity (rows)
-    bf16 *X = nullptr, *Xt = nullptr;
+    bf16* X = nullptr;
     std::vector<float*> Z;
-    std::vector<bf16*> Hb, Ht;
+    std::vector<bf16*> Hb;
     float* outp = nullptr;         // rows x 2
     float* yb = nullptr;
-    bf16 *dout = nullptr, *doutT = nullptr;
-    std::vector<bf16*> dZ, dZt;    // dL/dZ of each hidden layer and its transposed copy
+    bf16* dout = nullptr;
+    std::vector<bf16*> dZ;         // dL/dZ of each hidden layer
     // training-step launches: programmatic dependent launch on, and a second stream for the
     // weight-gradient products (forked from / joined to the caller's stream with events)
     bool pdl = false;
@@ -1542,7 +1497,6 @@ int gemm_mode(const ucbmlp::Epilogue& ep) {
     if (ep.gelu) need |= ucbmlp::kEpGelu;
     if (ep.outf) need |= ucbmlp::kEpOutF;
     if (ep.outh) need |= ucbmlp::kEpOutH;
-    if (ep.outt) need |= ucbmlp::kEpOutT;
     if (ep.zin) need |= ucbmlp::kEpZin;
     if (ep.colsum) need |= ucbmlp::kEpColsum;
     if (ep.nll) need |= ucbmlp::kEpNll;
@@ -1567,8 +1521,6 @@ bool set_gemm_attributes(int device, std::string& err) {
     };
     attribute(ucbmlp::mlp_infer_kernel<128, false>, ucbmlp::InferCfg<128>::kSmem);
     attribute(ucbmlp::mlp_infer_kernel<256, false>, ucbmlp::InferCfg<256>::kSmem);
-    attribute(ucbmlp::mlp_infer_kernel<128, true>, ucbmlp::InferCfg<128, true>::kSmem);
-    attribute(ucbmlp::mlp_infer_kernel<256, true>, ucbmlp::InferCfg<256, true>::kSmem);
     if (!cu_ok(ce, err, "cudaFuncSetAttribute(forward)")) return false;
     g_attr_devices.push_back(device);
     return true;
@@ -1616,13 +1568,14 @@ bool tensor_map(CUtensorMap* map, const bf16* ptr, int rows, int K, int box_rows
     return true;
 }
 
-// C = A B^T (+ epilogue). ep.atomic: K is split into up to kMaxSplits slices per tile and
+// C = A B^T (+ epilogue), A [M, K] and B [N, K]. ep.atomic: C = A^T B with A [K, lda] and
+// B [K, N] (columns of A from lda on count as zero), K is split into up to kMaxSplits slices per tile and
 // each slice's partial tile (rows < m_store, columns < n_store) is stored at
 // ep.outf + slice * m_eff * ep.ldf (m_eff = min(M, m_store)); *splits_out receives the
 // number of slices and part_cap bounds the buffer (floats). The slices are added later, in
 // slice order, by the optimiser kernel.
 bool gemm(Mlp& m, const bf16* A, const bf16* B, int M, int N, int K, const ucbmlp::Epilogue& ep_in, cudaStream_t st,
-          std::string& err, int* splits_out = nullptr, long long part_cap = 0) {
+          std::string& err, int* splits_out = nullptr, long long part_cap = 0, int lda = 0) {
     ucbmlp::Epilogue ep = ep_in;
     if (M <= 0 || N <= 0 || K <= 0 || M % ucbmlp::kBM || N % 128 || K % ucbmlp::kBK) {
         err = "gemm: unsupported shape " + std::to_string(M) + "x" + std::to_string(N) + "x" + std::to_string(K);
@@ -1653,11 +1606,17 @@ bool gemm(Mlp& m, const bf16* A, const bf16* B, int M, int N, int K, const ucbml
         ep.split_stride = 0;
     }
     CUtensorMap ta, tb;
-    if (!tensor_map(&ta, A, M, K, ucbmlp::kBM, err) || !tensor_map(&tb, B, N, K, bn, err)) return false;
+    if (ep.atomic ? (!tensor_map(&ta, A, K, lda, ucbmlp::kBK, err) || !tensor_map(&tb, B, K, N, ucbmlp::kBK, err))
+                  : (!tensor_map(&ta, A, M, K, ucbmlp::kBM, err) || !tensor_map(&tb, B, N, K, bn, err)))
+        return false;
     ucbmlp::GemmWork w{N / bn, splits, kt, per, tiles * splits};
     const int grid = std::min(w.items, sms);
     m.e->launches += 1;
     const int mode = gemm_mode(ep);
+    if ((mode == ucbmlp::kModeSplit) != (ep.atomic != 0)) {
+        err = "gemm: split-K launches alone take [K, M] operands";
+        return false;
+    }
     bool ok = false, found = false;
     auto go = [&](auto kernel, int smem, int md) {
         if (found || md != mode) return;
@@ -1713,6 +1672,16 @@ bool fused_args(Mlp& m, const MlpInputs& in, ucbmlp::InferMaps& maps, ucbmlp::In
 
 bool ensure_rows(Mlp& m, int rows, std::string& err) {
     if (rows <= m.rows) return true;
+    if (fused_supported(m)) {  // the training form is loaded by the first batch, not by a prediction
+        const cudaError_t ce =
+            m.H == 256 ? cudaFuncSetAttribute(ucbmlp::mlp_infer_kernel<256, true>,
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              ucbmlp::InferCfg<256, true>::kSmem)
+                       : cudaFuncSetAttribute(ucbmlp::mlp_infer_kernel<128, true>,
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              ucbmlp::InferCfg<128, true>::kSmem);
+        if (!cu_ok(ce, err, "cudaFuncSetAttribute(forward)")) return false;
+    }
     if (m.graph) {
         cudaGraphExecDestroy(m.graph);
         m.graph = nullptr;
@@ -1721,31 +1690,23 @@ bool ensure_rows(Mlp& m, int rows, std::string& err) {
     m.act_owned.clear();
     m.Z.clear();
     m.Hb.clear();
-    m.Ht.clear();
     m.rows = 0;
     auto& o = m.act_owned;
     const size_t R = rows;
-    // the fused forward pass keeps the row-major features and activations on chip
-    const size_t Rm = fused_supported(m) ? 0 : R;
-    if (!(m.X = dalloc<bf16>(Rm * m.F, o, err, "features")) || !(m.Xt = dalloc<bf16>(R * m.F, o, err, "features^T")))
-        return false;
+    if (!(m.X = dalloc<bf16>(R * m.F, o, err, "features"))) return false;
     for (int l = 0; l < m.L; ++l) {
         float* z = dalloc<float>(R * m.H, o, err, "Z");
-        bf16* h = dalloc<bf16>(Rm * m.H, o, err, "H");
-        bf16* ht = dalloc<bf16>(R * m.H, o, err, "H^T");
-        if (!z || !h || !ht) return false;
+        bf16* h = dalloc<bf16>(R * m.H, o, err, "H");
+        if (!z || !h) return false;
         m.Z.push_back(z);
         m.Hb.push_back(h);
-        m.Ht.push_back(ht);
     }
     if (!(m.outp = dalloc<float>(R * 2, o, err, "out")) || !(m.yb = dalloc<float>(R, o, err, "y batch")) ||
-        !(m.dout = dalloc<bf16>(R * 64, o, err, "dOut")) || !(m.doutT = dalloc<bf16>(R * 128, o, err, "dOut^T")))
+        !(m.dout = dalloc<bf16>(R * 64, o, err, "dOut")))
         return false;
     m.dZ.assign(m.L, nullptr);
-    m.dZt.assign(m.L, nullptr);
     for (int l = 0; l < m.L; ++l)
-        if (!(m.dZ[l] = dalloc<bf16>(R * m.H, o, err, "dZ")) || !(m.dZt[l] = dalloc<bf16>(R * m.H, o, err, "dZ^T")))
-            return false;
+        if (!(m.dZ[l] = dalloc<bf16>(R * m.H, o, err, "dZ"))) return false;
     m.part.assign(m.L + 1, nullptr);
     m.part_cap.assign(m.L + 1, 0);
     m.splits.assign(m.L + 1, 0);
@@ -1816,7 +1777,6 @@ ucbmlp::FeatureArgs feature_args(Mlp& m, const MlpInputs& in, long long row0, in
     a.fourier = m.cfg.fourier;
     a.rows = rows;
     a.X = m.X;
-    a.Xt = train ? m.Xt : nullptr;
     return a;
 }
 
@@ -1835,12 +1795,11 @@ void loss_epilogue(const Mlp& m, int rows, int n_valid, ucbmlp::Epilogue& ep) {
     ep.rows = rows;
     ep.beta = m.cfg.beta_nll;
     ep.dout = m.dout;
-    ep.doutT = m.doutT;
     ep.blk = m.blk;
 }
 
-// Forward pass over `rows` rows of m.X. keep: store Z and H^T for the backward pass and
-// evaluate the loss of the first n_valid rows against m.yb (dOut, dOut^T, block sums).
+// Forward pass over `rows` rows of m.X. keep: store Z for the backward pass and
+// evaluate the loss of the first n_valid rows against m.yb (dOut, block sums).
 bool forward(Mlp& m, int rows, bool keep, cudaStream_t st, std::string& err, int n_valid = 0) {
     const bf16* x = m.X;
     int k = m.F;
@@ -1853,8 +1812,6 @@ bool forward(Mlp& m, int rows, bool keep, cudaStream_t st, std::string& err, int
         ep.ldf = m.H;
         ep.outh = m.Hb[l];
         ep.ldh = m.H;
-        ep.outt = keep ? m.Ht[l] : nullptr;
-        ep.ldt = rows;
         if (!gemm(m, x, m.W[l], rows, m.H, k, ep, st, err)) return false;
         x = m.Hb[l];
         k = m.H;
@@ -1871,10 +1828,11 @@ bool forward(Mlp& m, int rows, bool keep, cudaStream_t st, std::string& err, int
 
 // The forward half of a training step: the features of fa's rows, the hidden layers and the
 // loss of the first n_valid rows. Networks that the fused kernel covers take it at every batch
-// size; us a training step, a layer a launch -> fused:
-//   4 layers of 128: batch 1,024 89.4 -> 72.2, 8,192 95.1 -> 76.6, 16,384 114 -> 93, 65,536 359 -> 330
-//   256 wide (layers): 1,024 (4) 97.8 -> 97.7, 2,048 (4) 98.0 -> 99.7, 4,096 (3) 82.7 -> 81.0,
-//   8,192 (4) 130.6 -> 130.8, 16,384 (5) 218 -> 199, 32,768 (4) 330 -> 307, 65,536 (4) 593 -> 563
+// size; us a training step, a layer a launch -> fused (both with the transposed copies that the
+// weight gradients read then, see backward):
+//   4 layers of 128: batch 1,024 88.8 -> 70.7, 8,192 94.4 -> 75.8, 16,384 114 -> 93, 65,536 359 -> 329
+//   256 wide (layers): 1,024 (4) 97.8 -> 97.6, 2,048 (4) 98.0 -> 99.4, 4,096 (3) 82.4 -> 81.0,
+//   8,192 (4) 130.5 -> 130.6, 16,384 (5) 218 -> 199, 32,768 (4) 330 -> 306, 65,536 (4) 593 -> 561
 // (at 256 the layer kernels split a CTA's rows in two tiles, so they keep twice the SMs busy while
 // the batch has fewer tiles than SMs: the two forms meet there).
 bool forward_train(Mlp& m, const MlpInputs& in, const ucbmlp::FeatureArgs& fa, int rows, int n_valid, cudaStream_t st,
@@ -1888,7 +1846,7 @@ bool forward_train(Mlp& m, const MlpInputs& in, const ucbmlp::FeatureArgs& fa, i
     t.f = fa;
     for (int l = 0; l < m.L; ++l) {
         t.Z[l] = m.Z[l];
-        t.Ht[l] = m.Ht[l];
+        t.H[l] = m.Hb[l];
     }
     loss_epilogue(m, rows, n_valid, t.loss);
     const int grid = (int)std::min<long long>(a.tiles, std::max(m.e->sm_count, 1));
@@ -1926,12 +1884,17 @@ bool forward_infer(Mlp& m, int rows, cudaStream_t st, std::string& err) {
 }
 
 // Backward pass for the batch of the last forward(keep) (which already left dL/dOut in
-// dOut / dOut^T and the NLL block sums in blk): every product stores partial results only
+// dOut and the NLL block sums in blk): every product stores partial results only
 // (split-K slices of the weight gradients, 32-row block sums of the bias gradients); the
 // optimiser kernel adds them. dL/dZ of a hidden layer comes straight out of the epilogue of
 // the product that gives dL/dH (GELU backward fused). The weight-gradient products run on a
 // second stream beside that chain (each one forked when its dL/dZ is written, all joined
 // before the caller's stream goes on), so only the dL/dZ chain is on the critical path.
+// They read dL/dZ and the activations as the epilogues leave them, contiguous along the layer
+// (GemmCfg's MN form): transposed copies cost every epilogue 80 of its 176 passes through shared
+// memory a 32 x 32 chunk and 2 bytes a value of traffic. us a step with -> without them: 4 layers
+// of 256, batch 1,024 97.6 -> 89.7, 8,192 130.6 -> 122.1, 32,768 306 -> 282, 65,536 561 -> 522; of
+// 128, 1,024 70.7 -> 64.2, 8,192 75.8 -> 69.6, 65,536 329 -> 303; 2 layers of 384, 2,048 65.6 -> 63.5.
 bool backward(Mlp& m, int rows, cudaStream_t st, std::string& err) {
     const int Lo = m.L;
     int evi = 0;
@@ -1940,17 +1903,18 @@ bool backward(Mlp& m, int rows, cudaStream_t st, std::string& err) {
         return cu_ok(cudaEventRecord(e, st), err, "fork record") &&
                cu_ok(cudaStreamWaitEvent(m.side, e, 0), err, "fork wait");
     };
-    auto weight_grad = [&](int l, const bf16* At, const bf16* prevT) {
+    auto weight_grad = [&](int l, const bf16* A, const bf16* prev) {
         ucbmlp::Epilogue eg = epi();
         eg.outf = m.part[l];
         eg.ldf = m.in[l];
         eg.atomic = 1;
-        int M = m.H;
-        if (l == Lo) {  // dOut^T H: M padded to 128, rows 0 and 1 stored
+        int M = m.H, lda = m.H;
+        if (l == Lo) {  // dOut^T H: 64 columns (two in use), M padded to 128, rows 0 and 1 stored
             eg.m_store = 2;
             M = 128;
+            lda = 64;
         }
-        return gemm(m, At, prevT, M, m.in[l], rows, eg, m.side, err, &m.splits[l], m.part_cap[l]);
+        return gemm(m, A, prev, M, m.in[l], rows, eg, m.side, err, &m.splits[l], m.part_cap[l], lda);
     };
     auto dz = [&](int l, const bf16* A, const bf16* Bt, int K) {  // dL/dZ of hidden layer l
         ucbmlp::Epilogue ep = epi();
@@ -1958,17 +1922,15 @@ bool backward(Mlp& m, int rows, cudaStream_t st, std::string& err) {
         ep.ldz = m.H;
         ep.outh = m.dZ[l];
         ep.ldh = m.H;
-        ep.outt = m.dZt[l];
-        ep.ldt = rows;
         ep.colsum = m.dbp[l];
         ep.ldc = m.H;
         return gemm(m, A, Bt, rows, m.H, K, ep, st, err);
     };
-    // output layer: its weight gradient needs only dOut^T; dL/dZ of the last hidden layer is
+    // output layer: its weight gradient needs only dOut; dL/dZ of the last hidden layer is
     // (dOut W_out) GELU'(Z), K padded to 64
-    if (!fork() || !weight_grad(Lo, m.doutT, m.Ht[Lo - 1]) || !dz(Lo - 1, m.dout, m.Wt[Lo], 64)) return false;
+    if (!fork() || !weight_grad(Lo, m.dout, m.Hb[Lo - 1]) || !dz(Lo - 1, m.dout, m.Wt[Lo], 64)) return false;
     for (int l = Lo - 1; l >= 0; --l) {
-        if (!fork() || !weight_grad(l, m.dZt[l], l > 0 ? m.Ht[l - 1] : m.Xt)) return false;
+        if (!fork() || !weight_grad(l, m.dZ[l], l > 0 ? m.Hb[l - 1] : m.X)) return false;
         if (l > 0 && !dz(l - 1, m.dZ[l], m.Wt[l], m.H)) return false;
     }
     cudaEvent_t j = m.ev[evi++];
@@ -2374,7 +2336,6 @@ int ucb_mlp_loss_grad(ucb_mlp* h, const float* u, const float* y, long long n, f
         in.u = du;
         in.n = n;
         ucbmlp::FeatureArgs fa = feature_args(m, in, 0, rows, false);
-        fa.Xt = m.Xt;
         fa.y = dy;
         fa.yb = m.yb;
         if (!forward_train(m, in, fa, rows, (int)n, st, err) || !backward(m, rows, st, err) ||
