@@ -1737,6 +1737,7 @@ bool ensure_pred_rows(Mlp& m, int rows, std::string& err) {
     if (!(m.pX = dalloc<bf16>(R * m.F, o, err, "features")) || !(m.pH[0] = dalloc<bf16>(R * m.H, o, err, "H")) ||
         !(m.pH[1] = dalloc<bf16>(R * m.H, o, err, "H")) || !(m.pOut = dalloc<float>(R * 2, o, err, "out")))
         return false;
+    if (!cu_ok(cudaStreamSynchronize(nullptr), err, "clear buffers")) return false;  // as in ensure_rows
     m.pred_rows = rows;
     return true;
 }
@@ -2079,6 +2080,9 @@ Mlp* mlp_create(ucb_engine* e, const ucb_mlp_config& c, std::string& err) {
         m->W.push_back(w);
         m->Wt.push_back(wt);
     }
+    // the buffers are cleared on the default stream, behind whatever the caller has there: the
+    // parameters go up on the engine's stream, which does not wait for it
+    if (!cu_ok(cudaStreamSynchronize(nullptr), err, "clear buffers")) return nullptr;
     if (!cu_ok(cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking), err, "weight-gradient stream"))
         return nullptr;
     m->ev.assign(m->L + 2, nullptr);
