@@ -2034,6 +2034,13 @@ bool train_step(Mlp& m, const MlpInputs& in, const float* d_y, cudaStream_t st, 
            adam(m, rows, true, st, err);
 }
 
+// Orders the engine's stream after the work queued on the default stream, where a caller's tensors
+// come from: a fit that is given no stream runs on the engine's, right after its parameters are set.
+bool after_default_stream(Mlp& m, std::string& err) {
+    return cu_ok(cudaEventRecord(m.ev[0], nullptr), err, "default stream") &&
+           cu_ok(cudaStreamWaitEvent(m.e->stream, m.ev[0], 0), err, "default stream");
+}
+
 }  // namespace
 
 Mlp* mlp_create(ucb_engine* e, const ucb_mlp_config& c, std::string& err) {
@@ -2110,7 +2117,8 @@ bool mlp_reinit(Mlp* m, std::string& err) {
     // on the stream of the kernel that reads them: a copy from pageable memory may return while
     // its last part is still on the way, and the engine's stream does not wait for the default one
     cudaStream_t st = m->e->stream;
-    if (!cu_ok(cudaMemcpyAsync(m->p, hp.data(), m->n_params * sizeof(float), cudaMemcpyHostToDevice, st), err,
+    if (!after_default_stream(*m, err) ||
+        !cu_ok(cudaMemcpyAsync(m->p, hp.data(), m->n_params * sizeof(float), cudaMemcpyHostToDevice, st), err,
                "upload params") ||
         !cu_ok(cudaMemcpyAsync(m->Bf, hb.data(), hb.size() * sizeof(float), cudaMemcpyHostToDevice, st), err,
                "upload B"))
@@ -2298,8 +2306,12 @@ int ucb_mlp_set_params(ucb_mlp* m, const float* in, long long n) {
     cudaSetDevice(m->e->device);
     std::string err;
     // the copy and the BF16 refresh share a stream (see mlp_reinit)
-    if (cudaMemcpyAsync(m->m->p, in, n * sizeof(float), cudaMemcpyHostToDevice, m->e->stream) != cudaSuccess)
+    if (!after_default_stream(*m->m, err) ||
+        !cu_ok(cudaMemcpyAsync(m->m->p, in, n * sizeof(float), cudaMemcpyHostToDevice, m->e->stream), err,
+               "upload params")) {
+        m->e->last_error = err;
         return UCB_E_CUDA;
+    }
     if (!refresh(*m->m, m->e->stream, err) || cudaStreamSynchronize(m->e->stream) != cudaSuccess) {
         m->e->last_error = err;
         return UCB_E_CUDA;
