@@ -32,6 +32,7 @@
 
 #include "csv_export.h"
 #include "engine_internal.h"
+#include "heavy_parts.h"
 
 namespace ucbbr {
 
@@ -294,7 +295,7 @@ __global__ void join_kernel(const double* sf1, const double* sf2, const unsigned
 
 // Bounding boxes of a square's cells by kSub x kSub parts of its box, as floats relative to
 // the box's lower corner and rounded outwards (non-negative, so ordered as integers).
-constexpr int kSub = 16, kParts = kSub * kSub;
+constexpr int kParts = kSub * kSub;
 struct PartBoxes {
     float x0[kParts], x1[kParts], y0[kParts], y1[kParts];
 };
@@ -302,13 +303,11 @@ struct PartBoxes {
 struct Frame {  // a square's box
     double x0, y0, ix, iy;
     __device__ __forceinline__ explicit Frame(const Box& b) : x0(dval(b.x0)), y0(dval(b.y0)) {
-        const double wx = dval(b.x1) - x0, wy = dval(b.y1) - y0;
-        ix = wx > 0 ? kSub / wx : 0;
-        iy = wy > 0 ? kSub / wy : 0;
+        ix = part_scale(dval(b.x1) - x0);
+        iy = part_scale(dval(b.y1) - y0);
     }
     __device__ __forceinline__ int part(double x, double y) const {
-        const int i = min(kSub - 1, (int)((x - x0) * ix)), j = min(kSub - 1, (int)((y - y0) * iy));
-        return j * kSub + i;
+        return part_index(y - y0, iy) * kSub + part_index(x - x0, ix);
     }
 };
 
