@@ -148,6 +148,10 @@ inline double trial_scale(double cells, double steps_per_cell, double target_ste
     return full <= target_steps ? 1.0 : target_steps / full;
 }
 
+// Multiprocessors that the rules between kernel forms count with: the device's, or the B200's where
+// there is none (a precompilation).
+inline int multiprocessors(const ucb_engine* e) { return e && e->sm_count > 0 ? e->sm_count : 148; }
+
 // Builds the step-function source for a run.
 SystemCode make_system_code(const std::string& krs_body, int nx, int nv, int precision, int mode,
                             bool want_jvp);

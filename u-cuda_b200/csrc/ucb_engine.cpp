@@ -510,7 +510,24 @@ struct LleLaunch {
     TuneConfig shape;  // launch shape (block size used by the launch)
 };
 
-CompileRequest lle_compile_request(const ucb_lle2d_request& q, const LlePlan& plan, LleLaunch& L) {
+// Whether a shadow map of `cells` cells runs with a trajectory a lane (ucb_lle_split_kernel):
+// while its warps (16 cells each) have a scheduler of their own. A step then waits for one
+// trajectory's chain; with a second warp on a scheduler the two forms issue the same
+// instructions, and the pair form takes the transient and the renormalisation once a cell.
+// The verbatim step waits longer for its chain, which two warps still share.
+// B200, pair / split, Chen maps: native FP64 96^2 0.87 / 0.63 ms, 100^2 (two warps on some
+// schedulers) 0.87 / 0.90, 300^2 3.6 / 4.2; exact FP64 90^2 1.69 / 0.97, 137^2 1.70 / 1.53,
+// 170^2 2.71 / 2.95; exact FP32 137^2 1.75 / 1.36, 170^2 2.37 / 2.60.
+bool split_pays(const ucb_engine* e, const LleLaunch& L, long long cells) {
+    return cells <= 16LL * (L.sys.exact ? 2 : 1) * 4 * multiprocessors(e);
+}
+
+long long map_cells(const ucb_lle2d_request& q, const SweepMap& m) {
+    return m.dim == 2 ? (long long)q.n_pts * q.n_pts : (long long)q.n_pts;
+}
+
+CompileRequest lle_compile_request(const ucb_engine* e, const ucb_lle2d_request& q, const LlePlan& plan,
+                                   LleLaunch& L) {
     const int prec = q.opt.precision;
     bool tangent = false;
     if (q.opt.lle_method == UCB_LLE_TANGENT) tangent = true;
@@ -539,15 +556,26 @@ CompileRequest lle_compile_request(const ucb_lle2d_request& q, const LlePlan& pl
     rq.headers = &device_headers();
     rq.options.push_back(L.sys.exact ? "--fmad=false" : "--fmad=true");
     rq.kernels = {"ucb_lle_kernel", "ucb_state_kernel"};
-    if (!tangent && plan.map.h_axis == -1) rq.kernels.insert(rq.kernels.begin(), "ucb_lle_split_kernel");
+    // The kernel that a map of this size runs comes first: a shape search looks at its registers and
+    // keeps the shapes of the two forms apart (the order is part of the key).
+    if (!tangent && plan.map.h_axis == -1)
+        rq.kernels.insert(split_pays(e, L, map_cells(q, plan.map)) ? rq.kernels.begin() : rq.kernels.end(),
+                          "ucb_lle_split_kernel");
     return rq;
+}
+
+// Key of a prepared build: one for all map sizes (the program is the same, and a prepared launch picks
+// its kernel by the size it is called with).
+std::string pin_key(CompileRequest rq) {
+    std::sort(rq.kernels.begin(), rq.kernels.end());
+    return tune_key(rq);
 }
 
 // The compile request with the launch shape of this run applied (e may be null: explicit
 // options only).
 bool lle_tuned_request(ucb_engine* e, const ucb_lle2d_request& q, const LlePlan& plan, LleLaunch& L,
                        CompileRequest& rq, std::string& err) {
-    rq = lle_compile_request(q, plan, L);
+    rq = lle_compile_request(e, q, plan, L);
     return tune_request(e, q.opt, 128, rq, L.shape, err);
 }
 
@@ -565,18 +593,6 @@ bool prepare_lle(ucb_engine* e, const ucb_lle2d_request& q, const LlePlan& plan,
     if (!L.mod) return false;
     bind_lle(L);
     return true;
-}
-
-// Whether a shadow map of `cells` cells runs with a trajectory a lane (ucb_lle_split_kernel):
-// while its warps (16 cells each) have a scheduler of their own. A step then waits for one
-// trajectory's chain; with a second warp on a scheduler the two forms issue the same
-// instructions, and the pair form takes the transient and the renormalisation once a cell.
-// The verbatim step waits longer for its chain, which two warps still share.
-// B200, pair / split, Chen maps: native FP64 96^2 0.87 / 0.63 ms, 100^2 (two warps on some
-// schedulers) 0.87 / 0.90, 300^2 3.6 / 4.2; exact FP64 90^2 1.69 / 0.97, 137^2 1.70 / 1.53,
-// 170^2 2.71 / 2.95; exact FP32 137^2 1.75 / 1.36, 170^2 2.37 / 2.60.
-bool split_pays(const ucb_engine* e, const LleLaunch& L, long long cells) {
-    return cells <= 16LL * (L.sys.exact ? 2 : 1) * 4 * e->sm_count;
 }
 
 // Enqueues the LLE kernel. Workspace layout: [0] work counter, [8] step counter,
@@ -616,7 +632,7 @@ int enqueue_lle_fn(ucb_engine* e, const ucb_lle2d_request& q, const LlePlan& pla
         err = std::string("CUDA upload: ") + cudaGetErrorString(ce);
         return UCB_E_CUDA;
     }
-    const long long total = d_cell_list ? n_list : (plan.map.dim == 2 ? (long long)n * n : (long long)n);
+    const long long total = d_cell_list ? n_list : map_cells(q, plan.map);
     std::vector<char> params;
     if (prec == UCB_PREC_F64) {
         LleParamsT<double> hd{total, 0, n, plan.map.swap_xy ? 1 : 0, plan.amountOfPointsInBlock, 0,
@@ -785,8 +801,8 @@ int lle2d_pin(ucb_engine* e, const ucb_lle2d_request& q, std::string& err) {
     if (!plan_lle2d(q, plan, err)) return UCB_E_INVALID;
     if (!ensure_init(e, err)) return UCB_E_NOGPU;
     auto L = std::make_shared<LleLaunch>();
-    CompileRequest rq = lle_compile_request(q, plan, *L);
-    const std::string key = tune_key(rq);
+    CompileRequest rq = lle_compile_request(e, q, plan, *L);
+    const std::string key = pin_key(rq);
     if (!tune_request(e, q.opt, 128, rq, L->shape, err)) return UCB_E_INVALID;
     L->mod = e->modules.get(rq, err);
     if (!L->mod) return UCB_E_COMPILE;
@@ -805,7 +821,7 @@ int lle2d_find_pinned(ucb_engine* e, const ucb_lle2d_request& q, std::string& er
     }
     cudaSetDevice(e->device);
     LleLaunch probe;
-    const std::string key = tune_key(lle_compile_request(q, *plan, probe));
+    const std::string key = pin_key(lle_compile_request(e, q, *plan, probe));
     auto it = e->pinned_lle.find(key);
     if (it == e->pinned_lle.end()) {
         err = "kernel not prepared for this request: call ucb_prepare_lle2d first (loading a module allocates "
@@ -1176,7 +1192,7 @@ int ucb_autotune_lle2d(ucb_engine* e, const ucb_lle2d_request* req, int32_t forc
     base.cancel = nullptr;
     base.progress = nullptr;
     LleLaunch L0;
-    const std::string key = tune_key(lle_compile_request(base, plan, L0));
+    const std::string key = tune_key(lle_compile_request(e, base, plan, L0));
     // trial workload: the same window on a grid of at most 768^2 cells (a few resident
     // waves), horizon scaled to about 1.2e10 steps in all
     ucb_lle2d_request t = base;
@@ -1227,6 +1243,10 @@ int ucb_autotune_lle2d(ucb_engine* e, const ucb_lle2d_request* req, int32_t forc
             const double ms_per_cell = rep->default_ms / trial_steps * steps_cell;
             const double cells = std::min((double)base.n_pts * base.n_pts, 1500.0 / std::max(ms_per_cell, 1e-12));
             cq.n_pts = std::max(64, std::min(base.n_pts, (int)std::floor(std::sqrt(cells))));
+            // (a grid that runs the kernel the map runs)
+            while (cq.n_pts < base.n_pts && !split_pays(e, L0, map_cells(base, plan.map)) &&
+                   split_pays(e, L0, map_cells(cq, plan.map)))
+                ++cq.n_pts;
             rep->confirm_n_pts = cq.n_pts;
             cvals.resize((size_t)cq.n_pts * cq.n_pts);
             cflags.resize(cvals.size());
