@@ -778,6 +778,7 @@ extern "C" int ucb_run_basins_dbscan(ucb_engine* e, const ucb_basins_dbscan_requ
     cudaMemcpyAsync(ws + off1, prec == UCB_PREC_F64 ? (const void*)t1d.data() : (const void*)t1f.data(), tab_bytes,
                     cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(ws, 0, 16, st);
+    counters_cleared(e);
     if (q.progress_phase) *q.progress_phase = 1;
     if (q.progress) *q.progress = 0.0f;
     // 1. classes and features (UcbBasinsRefParams field by field)

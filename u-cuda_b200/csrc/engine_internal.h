@@ -46,6 +46,7 @@ struct ucb_engine {
     ucb::ModuleCache modules;
     cudaStream_t stream = nullptr;   // engine stream for the host-buffer entry points
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t cleared = nullptr;  // a run's counters are zero (counters_cleared)
     // Device workspace: work counters, step counters, axis tables. Grown on demand.
     void* ws = nullptr;
     size_t ws_bytes = 0;
@@ -204,13 +205,16 @@ ucb_lle2d_request as_lle2d(const ucb_lle1d_request& q);
 // Launch helper: persistent grid size for a kernel.
 int persistent_grid(ucb_engine* e, CUfunction f, int block, long long work_items);
 
-// Run control of the host-buffer entry points (ucb_run_*). wait_run waits for `done` (an
+// Run control of the host-buffer entry points (ucb_run_*). counters_cleared marks the point of
+// the engine's stream where the run's counters have been zeroed: wait_run reads no progress
+// before it (until then the words are those of the call before). wait_run waits for `done` (an
 // event recorded after the run's main kernel, whose work counter is the workspace's first
 // word); while it waits it mirrors the caller's *cancel into the control block (the kernels'
 // warps then take no more cells and an adaptive cell abandons its steps) and writes the
 // queue position / work_items to *progress. Without cancel and progress words it simply
 // synchronises. Returns UCB_OK, UCB_E_CANCELLED (the control block is clear again once the
 // kernel has ended) or UCB_E_CUDA.
+void counters_cleared(ucb_engine* e);
 int wait_run(ucb_engine* e, cudaEvent_t done, const volatile int32_t* cancel, volatile float* progress,
              long long work_items, std::string& err);
 

@@ -159,6 +159,7 @@ extern "C" int ucb_run_basins(ucb_engine* e, const ucb_basins_request* req, ucb_
     // ws: [0] progress, [8] steps, [16] overflow, [64 ..] work counters of the slices, [128 ..]
     // lengths of the lists between them
     cudaMemsetAsync(ws, 0, 256, st);
+    counters_cleared(e);
     cudaMemsetAsync(ws + off_keys, 0, kTableSlots * 8, st);
     cudaMemsetAsync(ws + off_seats, 0, (size_t)kSlices * kMaxSms * 4, st);
     std::vector<double> trig_d;

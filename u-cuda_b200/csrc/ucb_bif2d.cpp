@@ -206,6 +206,7 @@ extern "C" int ucb_run_bif2d(ucb_engine* e, const ucb_bif2d_request* req, ucb_bi
     cudaMemcpyAsync(ws + off1, prec == UCB_PREC_F64 ? (const void*)t1d.data() : (const void*)t1f.data(), tab_bytes,
                     cudaMemcpyHostToDevice, e->stream);
     cudaMemsetAsync(ws, 0, 16, e->stream);
+    counters_cleared(e);
     if (q.progress) *q.progress = 0.0f;
     int rc = UCB_OK;
     // UcbBif2dParams field by field

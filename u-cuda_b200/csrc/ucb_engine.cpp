@@ -76,7 +76,8 @@ bool ensure_init(ucb_engine* e, std::string& err) {
         }
     }
     if ((ce = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking)) != cudaSuccess ||
-        (ce = cudaEventCreate(&e->ev0)) != cudaSuccess || (ce = cudaEventCreate(&e->ev1)) != cudaSuccess) {
+        (ce = cudaEventCreate(&e->ev0)) != cudaSuccess || (ce = cudaEventCreate(&e->ev1)) != cudaSuccess ||
+        (ce = cudaEventCreateWithFlags(&e->cleared, cudaEventDisableTiming)) != cudaSuccess) {
         err = std::string("stream/event creation: ") + cudaGetErrorString(ce);
         return false;
     }
@@ -113,6 +114,8 @@ static void set_cancel(ucb_engine* e, int32_t v) {
     cudaStreamSynchronize(e->control_stream);
 }
 
+void counters_cleared(ucb_engine* e) { cudaEventRecord(e->cleared, e->stream); }
+
 int wait_run(ucb_engine* e, cudaEvent_t done, const volatile int32_t* cancel, volatile float* progress,
              long long work_items, std::string& err) {
     ucb_run_control* c = e->control;
@@ -138,7 +141,7 @@ int wait_run(ucb_engine* e, cudaEvent_t done, const volatile int32_t* cancel, vo
             set_cancel(e, 1);
             cancelled = true;
         }
-        if (progress && work_items > 0 &&
+        if (progress && work_items > 0 && cudaEventQuery(e->cleared) == cudaSuccess &&
             cudaMemcpyAsync(&c->position, e->ws, sizeof(c->position), cudaMemcpyDeviceToHost, e->control_stream) ==
                 cudaSuccess &&
             cudaStreamSynchronize(e->control_stream) == cudaSuccess) {
@@ -632,6 +635,7 @@ int enqueue_lle_fn(ucb_engine* e, const ucb_lle2d_request& q, const LlePlan& pla
         err = std::string("CUDA upload: ") + cudaGetErrorString(ce);
         return UCB_E_CUDA;
     }
+    if (stream == e->stream) counters_cleared(e);
     const long long total = d_cell_list ? n_list : map_cells(q, plan.map);
     std::vector<char> params;
     if (prec == UCB_PREC_F64) {
@@ -885,6 +889,7 @@ void ucb_destroy(ucb_engine* e) {
         e->modules.clear();
         if (e->ws) cudaFree(e->ws);
         if (e->ev0) cudaEventDestroy(e->ev0);
+        if (e->cleared) cudaEventDestroy(e->cleared);
         if (e->ev1) cudaEventDestroy(e->ev1);
         if (e->stream) cudaStreamDestroy(e->stream);
         if (e->pool) cudaMemPoolDestroy(e->pool);

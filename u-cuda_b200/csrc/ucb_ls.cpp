@@ -190,6 +190,7 @@ int ls_run(ucb_engine* e, const ucb_ls2d_request& q, const SweepMap& m, int n_bl
     cudaMemcpyAsync(ws + off1, prec == UCB_PREC_F64 ? (const void*)t1d.data() : (const void*)t1f.data(), tab_bytes,
                     cudaMemcpyHostToDevice, e->stream);
     cudaMemsetAsync(ws, 0, 16, e->stream);
+    counters_cleared(e);
     double* d_values = nullptr;
     int32_t* d_flags = nullptr;
     long long* d_cell_steps = nullptr;
