@@ -161,6 +161,7 @@ __device__ __forceinline__ bool basins_cell(const UcbBasinsParams& p, long long 
         } else
 #endif
         {
+            meet(st);
             run_single<false>(st, x, a, p.h, p.steps_per_period, p.maxv);
         }
         ns += p.steps_per_period;

@@ -199,7 +199,12 @@ __device__ __forceinline__ int sample_chunk(const S& st, numb* x, const numb* a,
 #ifdef UCB_SIXTH
 __device__ __noinline__ int redo_samples(numb* x, const numb* a, numb h, numb* w, int m, bool check, int pre,
                                          numb maxv) {
-    return sample_chunk(VerbatimStepper(), x, a, h, w, m, check, pre, maxv);
+    numb xr[UCB_NX], ar[UCB_NV];
+    copy_state<UCB_NX>(x, xr);
+    copy_values(a, ar);
+    const int r = sample_chunk(VerbatimStepper(), xr, ar, h, w, m, check, pre, maxv);
+    copy_state<UCB_NX>(xr, x);
+    return r;
 }
 __device__ __forceinline__ int run_samples(const Stepper& st, numb* x, const numb* a, numb h, numb* w, int m,
                                            bool check, int pre, numb maxv) {
@@ -313,6 +318,7 @@ __device__ __forceinline__ int loop_record(const S& st, numb* x, const numb* a, 
     // The divergence test comes after the steps of samples 0, kCheckInterval, ...
     for (long long q0 = 0; q0 < iters; q0 += kScanChunk) {
         const int m = (iters - q0 < kScanChunk) ? (int)(iters - q0) : kScanChunk;
+        if (q0 % kCheckInterval == 0) meet(st);
         if (run_samples(st, x, a, h, w, m, q0 % kCheckInterval == 0, pre, maxv) == 0) {
             ns += pre;
             return 0;
@@ -337,6 +343,7 @@ __device__ __forceinline__ int loop_transient(const S& st, numb* x, const numb* 
                                               numb maxv, long long& ns, bool /*live*/) {
     for (long long i0 = 0; i0 < iters; i0 += kCheckInterval) {
         const int n = (iters - i0 < kCheckInterval) ? (int)(iters - i0) : kCheckInterval;
+        meet(st);
         if (run_single<true>(st, x, a, h, n, maxv) == 0) {
             ns += 1;
             return 0;
@@ -404,7 +411,12 @@ __device__ __forceinline__ int sample_strided(const S& st, numb* x, const numb* 
 #ifdef UCB_SIXTH
 __device__ __noinline__ int redo_strided(numb* x, const numb* a, numb h, numb* out, int m, bool check, int pre,
                                          numb maxv) {
-    return sample_strided(VerbatimStepper(), x, a, h, out, m, check, pre, maxv);
+    numb xr[UCB_NX], ar[UCB_NV];
+    copy_state<UCB_NX>(x, xr);
+    copy_values(a, ar);
+    const int r = sample_strided(VerbatimStepper(), xr, ar, h, out, m, check, pre, maxv);
+    copy_state<UCB_NX>(xr, x);
+    return r;
 }
 __device__ __forceinline__ int run_strided(const Stepper& st, numb* x, const numb* a, numb h, numb* out, int m,
                                            bool check, int pre, numb maxv) {
@@ -474,6 +486,7 @@ extern "C" __global__ void __launch_bounds__(2 * UCB_BLOCK) ucb_bif_kernel(const
             int m = 0;
             if (live && q0 < iters) {
                 m = (iters - q0 < kScanChunk) ? (int)(iters - q0) : kScanChunk;
+                if (since == 0) meet(st);
                 if (run_strided(st, x, a, h, &s.samples[b][0][lane], m, since == 0, p.pre_scaller, p.maxv) == 0) {
                     ns += p.pre_scaller;
                     m = 0;

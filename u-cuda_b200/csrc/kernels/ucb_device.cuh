@@ -129,7 +129,7 @@ struct VerbatimStepper {
 // The body with its division by six replaced (ucb_exact.cuh). The bits are the division's
 // while `range` stays within kSixthRange; run_single / run_pair / run_probes and the
 // sampling of ucb_bif.cuh take a block of steps again with VerbatimStepper otherwise, and the
-// trajectory's later blocks with it from the start.
+// trajectory's later blocks with it from the start, as those of its warp (meet).
 struct Stepper {
     mutable unsigned int range;
     mutable bool verbatim;
@@ -144,6 +144,16 @@ struct Stepper {
         return verbatim;
     }
 };
+// A lane whose blocks are taken with the division has the lanes that step with it take theirs
+// so too (the same bits), or they would wait for its pass after their own: loops ask at intervals of
+// about a hundred steps. Forms with a trajectory a lane do not ask: both passes of one trajectory
+// are still less than the division for several, and the vote costs them up to 4 %.
+// B200, exact FP32 Lorenz maps some of whose cells settle on the origin, the division everywhere /
+// the settled lanes alone / the warp together: exponent 256^2 (60,000 steps a cell) 51 / 60 / 49 ms,
+// diagram of 1,024 values (30,000) 32.0 / 36.1 / 30.4, spectrum 256^2 (52,000) 45 / 55 / 46.5; no cell
+// settling: exponent 28.4 / 21.0 / 20.3, spectrum 27.2 / 22.3 / 22.3; FP64, none settling: 31.4 / 20.6 /
+// 20.9, 31.8 / 22.7 / 22.7. A trajectory a lane, 64^2: 34.2 / 31.1 / (asking 28.6).
+__device__ __forceinline__ void meet(const Stepper& s) { s.verbatim = __any_sync(__activemask(), s.verbatim); }
 #else
 struct Stepper : VerbatimStepper {
     __device__ __forceinline__ explicit Stepper(numb) {}
@@ -471,6 +481,9 @@ __device__ __forceinline__ bool diverged2(const float2* x, float maxValue, int c
 // `iters` steps, the divergence test after iterations 0, 100, 200, ... of this call,
 // then one extra step and the fixed-point test. 1 ok / -1 fixed point / 0 diverged.
 // ---------------------------------------------------------------------------
+template <class S>
+__device__ __forceinline__ void meet(const S&) {}  // (steps that are never taken again)
+
 // `n` steps of x; with Check the divergence test after the first of them. 0: diverged there.
 template <bool Check, class S>
 __device__ __forceinline__ int block_single(const S& s, numb* x, const numb* a, numb h, int n, numb maxValue) {
@@ -540,18 +553,6 @@ __device__ __forceinline__ int block_nt(const S& s, numb* x, const numb* a, numb
 #endif
 
 #ifdef UCB_SIXTH
-// Blocks taken again with the division. The state at the start of the block waits in local
-// memory (the arrays these calls take), not in registers.
-template <bool Check>
-__device__ __noinline__ int redo_single(numb* x, const numb* a, numb h, int n, numb maxValue) {
-    return block_single<Check>(VerbatimStepper(), x, a, h, n, maxValue);
-}
-__device__ __noinline__ int redo_pair(numb* xy, const numb* a, numb h, int n, numb maxValue, bool whole_nt) {
-#ifdef UCB_NT
-    if (whole_nt) return block_pair_nt(VerbatimStepper(), xy, xy + UCB_NX, a, h, maxValue);
-#endif
-    return block_pair(VerbatimStepper(), xy, xy + UCB_NX, a, h, n, maxValue);
-}
 __device__ __forceinline__ void copy_values(const numb* a, numb* out) {
 #pragma unroll
     for (int i = 0; i < UCB_NV; ++i) out[i] = a[i];
@@ -560,6 +561,34 @@ template <int N>
 __device__ __forceinline__ void copy_state(const numb* x, numb* out) {
 #pragma unroll
     for (int i = 0; i < N; ++i) out[i] = x[i];
+}
+
+// Blocks taken with the division. The state at the start of the block waits in local memory (the
+// arrays these calls take), not in registers; the steps run on copies of it in registers.
+template <bool Check>
+__device__ __noinline__ int redo_single(numb* x, const numb* a, numb h, int n, numb maxValue) {
+    numb xr[UCB_NX], ar[UCB_NV];
+    copy_state<UCB_NX>(x, xr);
+    copy_values(a, ar);
+    const int r = block_single<Check>(VerbatimStepper(), xr, ar, h, n, maxValue);
+    copy_state<UCB_NX>(xr, x);
+    return r;
+}
+__device__ __noinline__ int redo_pair(numb* xy, const numb* a, numb h, int n, numb maxValue, bool whole_nt) {
+    numb xr[UCB_NX], yr[UCB_NX], ar[UCB_NV];
+    copy_state<UCB_NX>(xy, xr);
+    copy_state<UCB_NX>(xy + UCB_NX, yr);
+    copy_values(a, ar);
+    int r;
+#ifdef UCB_NT
+    if (whole_nt)
+        r = block_pair_nt(VerbatimStepper(), xr, yr, ar, h, maxValue);
+    else
+#endif
+        r = block_pair(VerbatimStepper(), xr, yr, ar, h, n, maxValue);
+    copy_state<UCB_NX>(xr, xy);
+    copy_state<UCB_NX>(yr, xy + UCB_NX);
+    return r;
 }
 
 template <bool Check>
@@ -638,12 +667,13 @@ __device__ __forceinline__ int run_pair_nt(const S& s, numb* x, numb* y, const n
 #endif
 #endif
 
-template <class S>
+template <bool Meet = true, class S>
 __device__ __forceinline__ int loop_single(const S& s, numb* x, const numb* a, numb h, long long iters,
                                            numb maxValue, long long& ns) {
     for (long long i0 = 0; i0 < iters; i0 += kCheckInterval) {
 #ifdef UCB_SIXTH
         const int n = (iters - i0 < kCheckInterval) ? (int)(iters - i0) : kCheckInterval;
+        if (Meet) meet(s);
         if (run_single<true>(s, x, a, h, n, maxValue) == 0) {
             ns += 1;
             return 0;
@@ -680,6 +710,7 @@ __device__ __forceinline__ int loop_pair(const S& s, numb* x, numb* y, const num
                                          long long iters, numb maxValue, long long& ns) {
     for (long long i0 = 0; i0 < iters; i0 += kCheckInterval) {
         const int n = (iters - i0 < kCheckInterval) ? (int)(iters - i0) : kCheckInterval;
+        if (i0 > 0) meet(s);
         if (run_pair(s, x, y, a, h, n, maxValue) == 0) {
             ns += 2;
             return 0;

@@ -13,8 +13,9 @@
 // The remainder has to be a normal number: `range` gathers the largest distance of an
 // argument from the smallest exponent allowed (zero counts as in range), and steps with a
 // nonzero argument below 2^-959 (2^-63 in FP32), an infinity or a NaN among them are taken
-// again with the division (Stepper of ucb_device.cuh) — one branch for a block of steps, where
-// a branch a component cost as much as the division.
+// again with the division, and the trajectory's later steps too (Stepper and meet of
+// ucb_device.cuh: what that costs) — one branch for a block of steps, where a branch a component
+// cost as much as the division.
 // B200, cycles of a Lorenz step at one warp a scheduler: 492 -> 214 (FP64), 437 -> 292 (FP32);
 // FP64 maps, whole calls: Rossler 300^2 19.9 -> 14.8 ms, curve of 200 values 12.7 -> 5.4 ms,
 // hyper-chaotic Rossler spectrum 200^2 18.3 -> 13.5 ms.

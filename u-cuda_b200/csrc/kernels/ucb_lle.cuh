@@ -94,6 +94,7 @@ __device__ __forceinline__ double lle_cell_shadow(const UcbLleParams& p, long lo
     LogProduct prod;  // same sum, one log at the end
 #endif
     for (int b = 0; b < p.n_blocks; ++b) {
+        if ((b & 7) == 0) meet(st);
 #if defined(UCB_NT) && UCB_HAXIS == -1
         if (loop_pair_nt(st, x, y, a, cs.h, p.maxv, ns) == 0) return 999.0;
 #else
@@ -144,7 +145,7 @@ __device__ __forceinline__ double lle_cell_split(const UcbLleParams& p, long lon
     apply_sweep(c, p.axis0, p.axis1, x, a);
     const Stepper st(h);
     long long steps = 0;  // of the cell, counted by both lanes
-    if (loop_single(st, x, a, h, p.skip, p.maxv, steps) == 0) live = false;
+    if (loop_single<false>(st, x, a, h, p.skip, p.maxv, steps) == 0) live = false;
     {
         numb z[UCB_NX];
         probe_direction((unsigned long long)kidx, z);
@@ -494,6 +495,7 @@ extern "C" __global__ void UCB_LAUNCH_BOUNDS ucb_state_kernel(const UcbLleParams
     const ucbdev::Stepper st(cs.h);
     for (long long s = 0; s < p.skip; s += ucbdev::kCheckInterval) {
         const int n = p.skip - s < ucbdev::kCheckInterval ? (int)(p.skip - s) : ucbdev::kCheckInterval;
+        ucbdev::meet(st);
         ucbdev::run_single<false>(st, x, a, cs.h, n, p.maxv);
     }
 #pragma unroll

@@ -128,8 +128,16 @@ __device__ __forceinline__ int block_probes(const S& s, numb* x, numb (*y)[UCB_N
 #ifdef UCB_SIXTH
 template <bool Check>
 __device__ __noinline__ int redo_probes(numb* xy, const numb* a, numb h, int n, numb maxValue) {
-    return block_probes<Check>(VerbatimStepper(), xy, reinterpret_cast<numb(*)[UCB_NX]>(xy + UCB_NX), a, h, n,
-                               maxValue);
+    numb xr[UCB_NX], yr[UCB_NX][UCB_NX], ar[UCB_NV];
+    copy_state<UCB_NX>(xy, xr);
+#pragma unroll
+    for (int j = 0; j < UCB_NX; ++j) copy_state<UCB_NX>(xy + UCB_NX + j * UCB_NX, yr[j]);
+    copy_values(a, ar);
+    const int r = block_probes<Check>(VerbatimStepper(), xr, yr, ar, h, n, maxValue);
+    copy_state<UCB_NX>(xr, xy);
+#pragma unroll
+    for (int j = 0; j < UCB_NX; ++j) copy_state<UCB_NX>(yr[j], xy + UCB_NX + j * UCB_NX);
+    return r;
 }
 template <bool Check>
 __device__ __forceinline__ int run_probes(const Stepper& s, numb* x, numb (*y)[UCB_NX], const numb* a, numb h, int n,
@@ -163,6 +171,7 @@ __device__ __forceinline__ int loop_probes(const S& s, numb* x, numb (*y)[UCB_NX
                                            long long iters, numb maxValue, long long& ns) {
     for (long long i0 = 0; i0 < iters; i0 += kCheckInterval) {
         const int n = (iters - i0 < kCheckInterval) ? (int)(iters - i0) : kCheckInterval;
+        if (i0 > 0) meet(s);
         if (run_probes<true>(s, x, y, a, h, n, maxValue) == 0) {
             ns += UCB_NX + 1;
             return 0;
@@ -376,6 +385,7 @@ __device__ __forceinline__ void ls_cell_fixed(const UcbLsParams& p, long long ki
 #pragma unroll
     for (int k = 0; k < UCB_NX; ++k) res_n[k] = 0;
     for (int b = 0; b < p.n_blocks; ++b) {
+        if ((b & 7) == 0) meet(st);
         if (loop_probes(st, x, y, a, h, nt, p.maxv, ns) == 0) {
 #pragma unroll
             for (int m = 0; m < UCB_NX; ++m) outv[m] = 999.0;
@@ -504,7 +514,7 @@ __device__ __forceinline__ void ls_groups_fixed(const UcbLsParams& p, long long&
         }
         const Stepper st(h);
         long long steps = 0;  // of the cell, counted by all its lanes
-        if (loop_single(st, x, a, h, p.skip, p.maxv, steps) == 0) live = false;
+        if (loop_single<false>(st, x, a, h, p.skip, p.maxv, steps) == 0) live = false;
 #ifdef UCB_LS_FIXED_TANGENT
         double za[UCB_NX], zb[UCB_NX], dens, sum = 0;
 #pragma unroll
