@@ -441,7 +441,14 @@ __device__ __forceinline__ int run_strided(const S& st, numb* x, const numb* a, 
 
 }  // namespace ucbdev
 
-extern "C" __global__ void __launch_bounds__(2 * UCB_BLOCK) ucb_bif_kernel(const UcbBifParams p) {
+// A register cap is a number of resident blocks of UCB_BLOCK threads (UCB_LAUNCH_BOUNDS): half as many
+// of twice the threads.
+#ifdef UCB_MIN_BLOCKS
+#define UCB_PAIRED_BOUNDS __launch_bounds__(2 * UCB_BLOCK, (UCB_MIN_BLOCKS + 1) / 2)
+#else
+#define UCB_PAIRED_BOUNDS __launch_bounds__(2 * UCB_BLOCK)
+#endif
+extern "C" __global__ void UCB_PAIRED_BOUNDS ucb_bif_kernel(const UcbBifParams p) {
     using namespace ucbdev;
     __shared__ BifPair pairs[UCB_BLOCK / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pair = warp % (UCB_BLOCK / 32);
