@@ -45,15 +45,16 @@ bool validate_bif(const ucb_bif1d_request& q, std::string& err) {
 }
 
 // Whether a diagram runs with two warps for 32 points (ucb_bif.cuh, UCB_BIF_PAIRED): while both
-// have a scheduler of their own on the B200's 148 SMs. Native Lorenz, FP64, 11,000 steps, one /
+// have a scheduler of their own. B200, native Lorenz, FP64, 11,000 steps, one /
 // two warps (kernel): 1,024 values 1.04 / 0.81 ms, 40,000 values 2.19 / 3.04. Its shared memory
 // is laid out for blocks of up to 64 points, and builds whose warp shares a forcing phase have
 // their own loops.
-bool pairs_pay(const ucb_bif1d_request& q, const SystemCode& sys) {
-    return q.n_pts <= 16 * 4 * 148 && q.opt.block_threads <= 64 && sys.trig_phase < 0;
+bool pairs_pay(const ucb_engine* e, const ucb_bif1d_request& q, const SystemCode& sys) {
+    return q.n_pts <= 16 * 4 * multiprocessors(e) && q.opt.block_threads <= 64 && sys.trig_phase < 0;
 }
 
-CompileRequest bif_compile_request(const ucb_bif1d_request& q, SystemCode& sys, bool* paired = nullptr) {
+CompileRequest bif_compile_request(const ucb_engine* e, const ucb_bif1d_request& q, SystemCode& sys,
+                                   bool* paired = nullptr) {
     SweepMap m;
     m.dim = 1;
     m.par_or_var = q.sweep_over_var ? 0 : 1;
@@ -64,7 +65,7 @@ CompileRequest bif_compile_request(const ucb_bif1d_request& q, SystemCode& sys, 
     rq.name = "ucb_bif1d.cu";
     std::vector<std::string> defs = clock_defines(sys);
     defs.push_back("UCB_WV " + std::to_string(q.writable_var));
-    const bool two = pairs_pay(q, sys);
+    const bool two = pairs_pay(e, q, sys);
     if (two) defs.push_back("UCB_BIF_PAIRED 1");
     if (paired) *paired = two;
     rq.source = make_prelude(q.opt.precision, q.amount_of_x, q.n_values, m, true, sys, defs) +
@@ -91,7 +92,7 @@ extern "C" int ucb_precompile_bif1d(const ucb_bif1d_request* req, char* err_out,
         return UCB_E_INVALID;
     }
     SystemCode sys;
-    CompileRequest rq = bif_compile_request(*req, sys);
+    CompileRequest rq = bif_compile_request(nullptr, *req, sys);
     TuneConfig shape;
     if (!tune_request(nullptr, req->opt, 32, rq, shape, err)) {
         if (err_out && err_len > 0) std::snprintf(err_out, (size_t)err_len, "%s", err.c_str());
@@ -133,7 +134,7 @@ extern "C" int ucb_run_bif1d(ucb_engine* e, const ucb_bif1d_request* req, ucb_bi
 
     SystemCode sys;
     bool paired = false;
-    CompileRequest rq = bif_compile_request(q, sys, &paired);
+    CompileRequest rq = bif_compile_request(e, q, sys, &paired);
     TuneConfig shape;
     if (!tune_request(e, q.opt, 32, rq, shape, err)) return fail(e, res, UCB_E_INVALID, err);
     auto mod = e->modules.get(rq, err);

@@ -55,7 +55,7 @@ ucb_lle2d_request as_lle(const ucb_ls2d_request& q) {
 // Cells a warp holds at a time when a cell runs on several lanes (ls_groups_dp5,
 // ls_groups_fixed); 0: a cell a lane. Lanes shorten a cell's chain and cost instructions (the
 // transient or the state's step, and the shuffled Gram-Schmidt pass, once a lane), so groups run
-// while the map has few warps for the B200's 592 schedulers.
+// while the map has few warps for the schedulers (592 on the B200).
 // Adaptive method, 4 variables over the wide hyper-chaotic Rossler window (t_end 50, 20,000
 // attempts; a cell a lane / groups): FP64 16^2 65 / 27 ms, 64^2 66 / 37, 96^2 68 / 46, 120^2
 // 69 / 64, 192^2 98 / 130; FP32 64^2 69 / 36, 128^2 71 / 45, 256^2 98 / 82, 384^2 131 / 151.
@@ -65,22 +65,22 @@ ucb_lle2d_request as_lle(const ucb_ls2d_request& q) {
 // 3.28 / 1.18 ms, 96^2 3.30 / 2.06, 128^2 (4.6) 3.29 / 3.17, 192^2 (10) 5.3 / 6.3; FP32 tangents
 // 96^2 (1.9) 1.95 / 1.36, 128^2 (3.5) 1.95 / 2.37; exact FP32 128^2 9.5 / 6.1, 192^2 (10)
 // 11.8 / 12.4, of 3 variables (7.8) 6.0 / 5.4.
-int ls_groups(const ucb_ls2d_request& q, const SweepMap& m, bool tangent, bool exact) {
-    constexpr long long kSchedulers = 4 * 148;
+int ls_groups(const ucb_engine* e, const ucb_ls2d_request& q, const SweepMap& m, bool tangent, bool exact) {
+    const long long schedulers = 4LL * multiprocessors(e);
     const int nx = q.amount_of_x;
     const bool f64 = q.opt.precision == UCB_PREC_F64, dp5 = q.method == UCB_LS_DP5;
     const long long cells = m.dim == 2 ? (long long)q.n_pts * q.n_pts : (long long)q.n_pts;
     if (nx < 2 || nx > 8 || m.h_axis != -1) return 0;
     const int most_groups = 32 / (dp5 || tangent ? nx : nx + 1);
     if (dp5) {
-        if (cells > (f64 ? 24 : 128) * kSchedulers) return 0;
-        return (int)std::min<long long>((cells + kSchedulers - 1) / kSchedulers, most_groups);
+        if (cells > (f64 ? 24 : 128) * schedulers) return 0;
+        return (int)std::min<long long>((cells + schedulers - 1) / schedulers, most_groups);
     }
     const long long most = tangent ? 2 : f64 || !exact ? 5 : 8;
-    return cells <= most * kSchedulers * most_groups ? most_groups : 0;
+    return cells <= most * schedulers * most_groups ? most_groups : 0;
 }
 
-CompileRequest ls_compile_request(const ucb_ls2d_request& q, const SweepMap& m, SystemCode& sys,
+CompileRequest ls_compile_request(const ucb_engine* e, const ucb_ls2d_request& q, const SweepMap& m, SystemCode& sys,
                                   int* groups_out = nullptr) {
     const bool dp5 = q.method == UCB_LS_DP5;
     const int prec = q.opt.precision;
@@ -96,7 +96,7 @@ CompileRequest ls_compile_request(const ucb_ls2d_request& q, const SweepMap& m, 
     std::vector<std::string> defs = dp5 ? clock_defines(sys) : std::vector<std::string>{};
     defs.push_back(dp5 ? "UCB_LS_DP5 1" : "UCB_LS_FIXED 1");
     if (tangent && sys.has_jvp) defs.push_back("UCB_LS_TANGENT 1");
-    const int groups = ls_groups(q, m, tangent && sys.has_jvp, sys.exact);
+    const int groups = ls_groups(e, q, m, tangent && sys.has_jvp, sys.exact);
     if (groups) {
         defs.push_back("UCB_LS_GROUP 1");
         // the fixed method's block length, known at compile time (plan_lle2d's count)
@@ -126,7 +126,7 @@ extern "C" int ucb_precompile_ls2d(const ucb_ls2d_request* req, char* err_out, i
         return UCB_E_INVALID;
     }
     SystemCode sys;
-    CompileRequest rq = ls_compile_request(*req, m, sys);
+    CompileRequest rq = ls_compile_request(nullptr, *req, m, sys);
     if (req->method == UCB_LS_DP5 && !sys.has_jvp) {
         if (err_out && err_len > 0) std::snprintf(err_out, (size_t)err_len, "%s", sys.note.c_str());
         return UCB_E_INVALID;
@@ -165,7 +165,7 @@ int ls_run(ucb_engine* e, const ucb_ls2d_request& q, const SweepMap& m, int n_bl
     const int nx = q.amount_of_x;
     SystemCode sys;
     int groups = 0;
-    CompileRequest rq = ls_compile_request(q, m, sys, &groups);
+    CompileRequest rq = ls_compile_request(e, q, m, sys, &groups);
     if (dp5 && !sys.has_jvp)
         return fail(e, res, UCB_E_INVALID, "the DP5 method needs a recognised RK4 body: " + sys.note);
     TuneConfig shape;
@@ -425,7 +425,7 @@ extern "C" int ucb_autotune_ls2d(ucb_engine* e, const ucb_ls2d_request* req, int
     base.cancel = nullptr;
     base.progress = nullptr;
     SystemCode sys;
-    const std::string key = tune_key(ls_compile_request(base, m, sys));
+    const std::string key = tune_key(ls_compile_request(e, base, m, sys));
     // trial: the same window on at most 384^2 cells, horizon scaled to about 1.2e10 steps
     // (fixed step) or the DP5 interval cut to 50 time units and 20,000 attempts per cell
     // (cells that turn stiff would otherwise run to the full attempt cap in every trial)
@@ -470,7 +470,7 @@ extern "C" int ucb_autotune_ls2d(ucb_engine* e, const ucb_ls2d_request* req, int
     auto build = [&](const TuneConfig& c) {
         ucb_ls2d_request q = with(c);
         SystemCode s2;
-        CompileRequest rq = ls_compile_request(q, tm, s2);
+        CompileRequest rq = ls_compile_request(e, q, tm, s2);
         TuneConfig shape;
         std::string e2;
         tune_request(e, q.opt, 128, rq, shape, e2);
