@@ -17,6 +17,7 @@ constexpr int kMaxSms = 256;    // of ucb_basins.cuh
 constexpr int kMaxK = 8;        // UCB_MAXK of ucb_basins.cuh
 constexpr int kSlices = 8;      // most slices of a map (at most 8: see the workspace)
 constexpr int kMinSlice = 64;   // periods
+constexpr size_t kKeptState = (size_t)256 << 20;  // state between slices that the engine's pool may keep
 
 bool validate(const ucb_basins_request& q, std::string& err) {
     if (!q.krs_body || !*q.krs_body) { err = "krs_body is empty"; return false; }
@@ -182,10 +183,13 @@ extern "C" int ucb_run_basins(ucb_engine* e, const ucb_basins_request* req, ucb_
         (ce = dev_alloc(e, (void**)&d_periods, (size_t)total * 4, st)) != cudaSuccess ||
         (ce = dev_alloc(e, (void**)&d_iters, (size_t)total * 4, st)) != cudaSuccess)
         return fail(e, res, UCB_E_CUDA, std::string("cudaMallocAsync: ") + cudaGetErrorString(ce));
-    // Slices of the cap (ucb_basins_kernel): the cells' state between them has to fit beside
-    // what is in use; a map of at most a warp a scheduler, or of few periods, is one slice.
+    // Slices of the cap (ucb_basins_kernel): the cells' state between them (184 bytes a cell of three
+    // variables with a phase) has to fit beside what is in use; a map of at most a warp a scheduler,
+    // or of few periods, is one slice.
     int slices = 1;
     char* d_state = nullptr;
+    uint64_t pool_bytes = 0;  // reserved without the state
+    if (e->pool) cudaMemPoolGetAttribute(e->pool, cudaMemPoolAttrReservedMemCurrent, &pool_bytes);
     const int ns = q.amount_of_x - (q.phase_var >= 0 ? 1 : 0);
     const size_t state_bytes = (((size_t)total * ns * (1 + kMaxK) * esz + 255) / 256) * 256;
     const size_t runs_bytes = (((size_t)total * kMaxK * 4 + 255) / 256) * 256;
@@ -193,8 +197,8 @@ extern "C" int ucb_run_basins(ucb_engine* e, const ucb_basins_request* req, ucb_
     const size_t slice_bytes = state_bytes + runs_bytes + 2 * list_bytes;
     if (total > 32LL * 4 * e->sm_count && q.max_periods > kMinSlice && !first_come_points(q)) {
         size_t free_b = 0, total_b = 0;
-        if (slice_bytes > ((size_t)256 << 20)) cudaMemGetInfo(&free_b, &total_b);
-        if (slice_bytes <= std::max((size_t)256 << 20, (size_t)(0.4 * (double)free_b)) &&
+        if (slice_bytes > kKeptState) cudaMemGetInfo(&free_b, &total_b);
+        if (slice_bytes <= std::max(kKeptState, (size_t)(0.4 * (double)free_b)) &&
             dev_alloc(e, (void**)&d_state, slice_bytes, st) == cudaSuccess)
             slices = std::min(kSlices, (q.max_periods + kMinSlice - 1) / kMinSlice);
         else
@@ -339,6 +343,8 @@ extern "C" int ucb_run_basins(ucb_engine* e, const ucb_basins_request* req, ucb_
     cudaFreeAsync(d_iters, st);
     if (d_state) cudaFreeAsync(d_state, st);
     cudaStreamSynchronize(st);
+    // a large state goes back to the device, not into the pool that lives as long as the engine
+    if (d_state && slice_bytes > kKeptState && e->pool) cudaMemPoolTrimTo(e->pool, pool_bytes);
     if (rc != UCB_OK) return fail(e, res, rc, err);
     if (overflow) return fail(e, res, UCB_E_INVALID, "attractor table overflow (more than 4096 distinct keys)");
     float ms = 0;
