@@ -202,7 +202,14 @@ __device__ __noinline__ int redo_samples(numb* x, const numb* a, numb h, numb* w
     numb xr[UCB_NX], ar[UCB_NV];
     copy_state<UCB_NX>(x, xr);
     copy_values(a, ar);
-    const int r = sample_chunk(VerbatimStepper(), xr, ar, h, w, m, check, pre, maxv);
+    int r = 1;
+#pragma unroll 1
+    for (int c = 0; c < m && r; ++c) {
+        w[c + 2] = recorded_value(xr);
+#pragma unroll 1
+        for (int j = 0; j < pre; ++j) calculateDiscreteModel(xr, ar, h);
+        if (check && c == 0 && diverged(xr, maxv)) r = 0;
+    }
     copy_state<UCB_NX>(xr, x);
     return r;
 }
@@ -414,7 +421,14 @@ __device__ __noinline__ int redo_strided(numb* x, const numb* a, numb h, numb* o
     numb xr[UCB_NX], ar[UCB_NV];
     copy_state<UCB_NX>(x, xr);
     copy_values(a, ar);
-    const int r = sample_strided(VerbatimStepper(), xr, ar, h, out, m, check, pre, maxv);
+    int r = 1;
+#pragma unroll 1
+    for (int c = 0; c < m && r; ++c) {
+        out[c * 32] = recorded_value(xr);
+#pragma unroll 1
+        for (int j = 0; j < pre; ++j) calculateDiscreteModel(xr, ar, h);
+        if (check && c == 0 && diverged(xr, maxv)) r = 0;
+    }
     copy_state<UCB_NX>(xr, x);
     return r;
 }

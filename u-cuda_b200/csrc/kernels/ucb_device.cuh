@@ -128,7 +128,7 @@ struct VerbatimStepper {
 #ifdef UCB_SIXTH
 // The body with its division by six replaced (ucb_exact.cuh). The bits are the division's
 // while `range` stays within kSixthRange; run_single / run_pair / run_probes and the
-// sampling of ucb_bif.cuh take a block of steps again with VerbatimStepper otherwise, and the
+// sampling of ucb_bif.cuh take a block of steps again with the division otherwise, and the
 // trajectory's later blocks with it from the start, as those of its warp (meet).
 struct Stepper {
     mutable unsigned int range;
@@ -563,29 +563,39 @@ __device__ __forceinline__ void copy_state(const numb* x, numb* out) {
     for (int i = 0; i < N; ++i) out[i] = x[i];
 }
 
-// Blocks taken with the division. The state at the start of the block waits in local memory (the
-// arrays these calls take), not in registers; the steps run on copies of it in registers.
-template <bool Check>
-__device__ __noinline__ int redo_single(numb* x, const numb* a, numb h, int n, numb maxValue) {
+// Blocks taken with the division: block_single and block_pair with few copies of the verbatim step
+// (a form that is seldom run adds little to a build: a diagram's took 0.44 s, 0.33 so). The state at
+// the start of the block waits in local memory (the arrays these calls take), not in registers;
+// the steps run on copies of it in registers.
+#ifdef UCB_NUMB_F32
+#define UCB_REDO_UNROLL 2  // as UCB_NT_UNROLL
+#else
+#define UCB_REDO_UNROLL 1
+#endif
+__device__ __noinline__ int redo_single(numb* x, const numb* a, numb h, int n, numb maxValue, bool check) {
     numb xr[UCB_NX], ar[UCB_NV];
     copy_state<UCB_NX>(x, xr);
     copy_values(a, ar);
-    const int r = block_single<Check>(VerbatimStepper(), xr, ar, h, n, maxValue);
+    calculateDiscreteModel(xr, ar, h);
+    const int r = check && diverged(xr, maxValue) ? 0 : 1;
+    UCB_PRAGMA_(unroll UCB_REDO_UNROLL)
+    for (int i = 1; i < (r ? n : 1); ++i) calculateDiscreteModel(xr, ar, h);
     copy_state<UCB_NX>(xr, x);
     return r;
 }
-__device__ __noinline__ int redo_pair(numb* xy, const numb* a, numb h, int n, numb maxValue, bool whole_nt) {
+__device__ __noinline__ int redo_pair(numb* xy, const numb* a, numb h, int n, numb maxValue) {
     numb xr[UCB_NX], yr[UCB_NX], ar[UCB_NV];
     copy_state<UCB_NX>(xy, xr);
     copy_state<UCB_NX>(xy + UCB_NX, yr);
     copy_values(a, ar);
-    int r;
-#ifdef UCB_NT
-    if (whole_nt)
-        r = block_pair_nt(VerbatimStepper(), xr, yr, ar, h, maxValue);
-    else
-#endif
-        r = block_pair(VerbatimStepper(), xr, yr, ar, h, n, maxValue);
+    calculateDiscreteModel(xr, ar, h);
+    calculateDiscreteModel(yr, ar, h);
+    const int r = diverged(xr, maxValue) || diverged(yr, maxValue) ? 0 : 1;
+    UCB_PRAGMA_(unroll UCB_REDO_UNROLL)
+    for (int i = 1; i < (r ? n : 1); ++i) {
+        calculateDiscreteModel(xr, ar, h);
+        calculateDiscreteModel(yr, ar, h);
+    }
     copy_state<UCB_NX>(xr, xy);
     copy_state<UCB_NX>(yr, xy + UCB_NX);
     return r;
@@ -599,7 +609,7 @@ __device__ __forceinline__ int run_single(const Stepper& s, numb* x, const numb*
     if (s.failed()) {
         numb av[UCB_NV];
         copy_values(a, av);
-        r = redo_single<Check>(keep, av, h, n, maxValue);
+        r = redo_single(keep, av, h, n, maxValue, Check);
         copy_state<UCB_NX>(keep, x);
     }
     return r;
@@ -612,18 +622,18 @@ __device__ __forceinline__ int run_nt(const Stepper& s, numb* x, const numb* a, 
     if (s.failed()) {
         numb av[UCB_NV];
         copy_values(a, av);
-        r = redo_single<true>(keep, av, h, UCB_NT + UCB_EXTRA_STEP, maxValue);
+        r = redo_single(keep, av, h, UCB_NT + UCB_EXTRA_STEP, maxValue, true);
         copy_state<UCB_NX>(keep, x);
     }
     return r;
 }
 #endif
 __device__ __forceinline__ int finish_pair(const Stepper& s, int r, numb* keep, numb* x, numb* y, const numb* a,
-                                           numb h, int n, numb maxValue, bool whole_nt) {
+                                           numb h, int n, numb maxValue) {
     if (s.failed()) {
         numb av[UCB_NV];
         copy_values(a, av);
-        r = redo_pair(keep, av, h, n, maxValue, whole_nt);
+        r = redo_pair(keep, av, h, n, maxValue);
         copy_state<UCB_NX>(keep, x);
         copy_state<UCB_NX>(keep + UCB_NX, y);
     }
@@ -635,7 +645,7 @@ __device__ __forceinline__ int run_pair(const Stepper& s, numb* x, numb* y, cons
     copy_state<UCB_NX>(x, keep);
     copy_state<UCB_NX>(y, keep + UCB_NX);
     const int r = s.verbatim ? 0 : block_pair(s, x, y, a, h, n, maxValue);
-    return finish_pair(s, r, keep, x, y, a, h, n, maxValue, false);
+    return finish_pair(s, r, keep, x, y, a, h, n, maxValue);
 }
 #ifdef UCB_NT
 __device__ __forceinline__ int run_pair_nt(const Stepper& s, numb* x, numb* y, const numb* a, numb h, numb maxValue) {
@@ -643,7 +653,7 @@ __device__ __forceinline__ int run_pair_nt(const Stepper& s, numb* x, numb* y, c
     copy_state<UCB_NX>(x, keep);
     copy_state<UCB_NX>(y, keep + UCB_NX);
     const int r = s.verbatim ? 0 : block_pair_nt(s, x, y, a, h, maxValue);
-    return finish_pair(s, r, keep, x, y, a, h, UCB_NT, maxValue, true);
+    return finish_pair(s, r, keep, x, y, a, h, UCB_NT + UCB_EXTRA_STEP, maxValue);
 }
 #endif
 #else

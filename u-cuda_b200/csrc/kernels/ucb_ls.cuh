@@ -126,14 +126,25 @@ __device__ __forceinline__ int block_probes(const S& s, numb* x, numb (*y)[UCB_N
 }
 
 #ifdef UCB_SIXTH
-template <bool Check>
-__device__ __noinline__ int redo_probes(numb* xy, const numb* a, numb h, int n, numb maxValue) {
+__device__ __noinline__ int redo_probes(numb* xy, const numb* a, numb h, int n, numb maxValue, bool check) {
     numb xr[UCB_NX], yr[UCB_NX][UCB_NX], ar[UCB_NV];
     copy_state<UCB_NX>(xy, xr);
 #pragma unroll
     for (int j = 0; j < UCB_NX; ++j) copy_state<UCB_NX>(xy + UCB_NX + j * UCB_NX, yr[j]);
     copy_values(a, ar);
-    const int r = block_probes<Check>(VerbatimStepper(), xr, yr, ar, h, n, maxValue);
+    int r = 1;
+#pragma unroll 1
+    for (int i = 0; i < n && r; ++i) {
+        calculateDiscreteModel(xr, ar, h);
+#pragma unroll
+        for (int j = 0; j < UCB_NX; ++j) calculateDiscreteModel(yr[j], ar, h);
+        if (check && i == 0) {
+            bool bad = diverged(xr, maxValue);
+#pragma unroll
+            for (int j = 0; j < UCB_NX; ++j) bad = bad || diverged(yr[j], maxValue);
+            if (bad) r = 0;
+        }
+    }
     copy_state<UCB_NX>(xr, xy);
 #pragma unroll
     for (int j = 0; j < UCB_NX; ++j) copy_state<UCB_NX>(yr[j], xy + UCB_NX + j * UCB_NX);
@@ -150,7 +161,7 @@ __device__ __forceinline__ int run_probes(const Stepper& s, numb* x, numb (*y)[U
     if (s.failed()) {
         numb av[UCB_NV];
         copy_values(a, av);
-        r = redo_probes<Check>(keep, av, h, n, maxValue);
+        r = redo_probes(keep, av, h, n, maxValue, Check);
         copy_state<UCB_NX>(keep, x);
 #pragma unroll
         for (int j = 0; j < UCB_NX; ++j) copy_state<UCB_NX>(keep + UCB_NX + j * UCB_NX, y[j]);
