@@ -10,6 +10,7 @@ U-CUDA directory, for the library presets); the committed JSON is what the tests
 import json
 import subprocess
 import sys
+import tempfile
 from pathlib import Path
 
 ROOT = Path(__file__).resolve().parents[2]
@@ -60,13 +61,12 @@ def library_cases():
 
 def run_case(text, alphabet, order, funcs):
     args = [str(REF_BIN), order, alphabet]
-    tmp = None
-    if funcs:
-        tmp = ROOT / "_work" / "funcs.txt"
-        tmp.parent.mkdir(exist_ok=True)
-        tmp.write_text(funcs)
-        args.append(str(tmp))
-    out = subprocess.run(args, input=text.encode(), capture_output=True, check=True).stdout.decode()
+    with tempfile.TemporaryDirectory() as tmp:
+        if funcs:
+            file = Path(tmp) / "funcs.txt"
+            file.write_text(funcs)
+            args.append(str(file))
+        out = subprocess.run(args, input=text.encode(), capture_output=True, check=True).stdout.decode()
     res = {"vars": [], "params": [], "schemes": {}, "error": None}
     cur = None
     buf = []
