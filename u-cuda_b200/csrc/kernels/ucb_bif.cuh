@@ -199,19 +199,7 @@ __device__ __forceinline__ int sample_chunk(const S& st, numb* x, const numb* a,
 #ifdef UCB_SIXTH
 __device__ __noinline__ int redo_samples(numb* x, const numb* a, numb h, numb* w, int m, bool check, int pre,
                                          numb maxv) {
-    numb xr[UCB_NX], ar[UCB_NV];
-    copy_state<UCB_NX>(x, xr);
-    copy_values(a, ar);
-    int r = 1;
-#pragma unroll 1
-    for (int c = 0; c < m && r; ++c) {
-        w[c + 2] = recorded_value(xr);
-#pragma unroll 1
-        for (int j = 0; j < pre; ++j) calculateDiscreteModel(xr, ar, h);
-        if (check && c == 0 && diverged(xr, maxv)) r = 0;
-    }
-    copy_state<UCB_NX>(xr, x);
-    return r;
+    return sample_chunk(VerbatimStepper(), x, a, h, w, m, check, pre, maxv);
 }
 __device__ __forceinline__ int run_samples(const Stepper& st, numb* x, const numb* a, numb h, numb* w, int m,
                                            bool check, int pre, numb maxv) {
@@ -418,19 +406,7 @@ __device__ __forceinline__ int sample_strided(const S& st, numb* x, const numb* 
 #ifdef UCB_SIXTH
 __device__ __noinline__ int redo_strided(numb* x, const numb* a, numb h, numb* out, int m, bool check, int pre,
                                          numb maxv) {
-    numb xr[UCB_NX], ar[UCB_NV];
-    copy_state<UCB_NX>(x, xr);
-    copy_values(a, ar);
-    int r = 1;
-#pragma unroll 1
-    for (int c = 0; c < m && r; ++c) {
-        out[c * 32] = recorded_value(xr);
-#pragma unroll 1
-        for (int j = 0; j < pre; ++j) calculateDiscreteModel(xr, ar, h);
-        if (check && c == 0 && diverged(xr, maxv)) r = 0;
-    }
-    copy_state<UCB_NX>(xr, x);
-    return r;
+    return sample_strided(VerbatimStepper(), x, a, h, out, m, check, pre, maxv);
 }
 __device__ __forceinline__ int run_strided(const Stepper& st, numb* x, const numb* a, numb h, numb* out, int m,
                                            bool check, int pre, numb maxv) {

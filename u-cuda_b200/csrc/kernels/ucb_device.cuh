@@ -147,12 +147,13 @@ struct Stepper {
 // A lane whose blocks are taken with the division has the lanes that step with it take theirs
 // so too (the same bits), or they would wait for its pass after their own: loops ask at intervals of
 // about a hundred steps. Forms with a trajectory a lane do not ask: both passes of one trajectory
-// are still less than the division for several, and the vote costs them up to 4 %.
+// are still less than the division for several, and the vote costs them up to 4 % (others 0-2 %).
 // B200, exact FP32 Lorenz maps some of whose cells settle on the origin, the division everywhere /
-// the settled lanes alone / the warp together: exponent 256^2 (60,000 steps a cell) 51 / 60 / 49 ms,
-// diagram of 1,024 values (30,000) 32.0 / 36.1 / 30.4, spectrum 256^2 (52,000) 45 / 55 / 46.5; no cell
-// settling: exponent 28.4 / 21.0 / 20.3, spectrum 27.2 / 22.3 / 22.3; FP64, none settling: 31.4 / 20.6 /
-// 20.9, 31.8 / 22.7 / 22.7. A trajectory a lane, 64^2: 34.2 / 31.1 / (asking 28.6).
+// the settled lanes alone / the warp together: exponent 256^2 (60,000 steps a cell) 51 / 60 / 50 ms,
+// diagram of 1,024 values (30,000) 32.0 / 36.1 / 31.7, period map 128^2 29.5 / 30.8 / 28.3, spectrum 256^2
+// (52,000) 45 / 53 / 45; no cell settling: 28.4 / 20.9 / 20.9, 9.5 / 4.9 / 4.9, 27.8 / 9.3 / 9.1, 27.2 / 22.3 /
+// 22.2; FP64, none settling: 31.4 / 20.6 / 20.6, 11.0 / 3.42 / 3.45, 29.5 / 5.62 / 5.69, 31.7 / 22.7 / 23.0. A
+// trajectory a lane, 64^2: 34.2 / 31.1 / (not asking).
 __device__ __forceinline__ void meet(const Stepper& s) { s.verbatim = __any_sync(__activemask(), s.verbatim); }
 #else
 struct Stepper : VerbatimStepper {
@@ -553,6 +554,18 @@ __device__ __forceinline__ int block_nt(const S& s, numb* x, const numb* a, numb
 #endif
 
 #ifdef UCB_SIXTH
+// Blocks taken again with the division. The state at the start of the block waits in local
+// memory (the arrays these calls take), not in registers.
+template <bool Check>
+__device__ __noinline__ int redo_single(numb* x, const numb* a, numb h, int n, numb maxValue) {
+    return block_single<Check>(VerbatimStepper(), x, a, h, n, maxValue);
+}
+__device__ __noinline__ int redo_pair(numb* xy, const numb* a, numb h, int n, numb maxValue, bool whole_nt) {
+#ifdef UCB_NT
+    if (whole_nt) return block_pair_nt(VerbatimStepper(), xy, xy + UCB_NX, a, h, maxValue);
+#endif
+    return block_pair(VerbatimStepper(), xy, xy + UCB_NX, a, h, n, maxValue);
+}
 __device__ __forceinline__ void copy_values(const numb* a, numb* out) {
 #pragma unroll
     for (int i = 0; i < UCB_NV; ++i) out[i] = a[i];
@@ -563,44 +576,6 @@ __device__ __forceinline__ void copy_state(const numb* x, numb* out) {
     for (int i = 0; i < N; ++i) out[i] = x[i];
 }
 
-// Blocks taken with the division: block_single and block_pair with few copies of the verbatim step
-// (a form that is seldom run adds little to a build: a diagram's took 0.44 s, 0.33 so). The state at
-// the start of the block waits in local memory (the arrays these calls take), not in registers;
-// the steps run on copies of it in registers.
-#ifdef UCB_NUMB_F32
-#define UCB_REDO_UNROLL 2  // as UCB_NT_UNROLL
-#else
-#define UCB_REDO_UNROLL 1
-#endif
-__device__ __noinline__ int redo_single(numb* x, const numb* a, numb h, int n, numb maxValue, bool check) {
-    numb xr[UCB_NX], ar[UCB_NV];
-    copy_state<UCB_NX>(x, xr);
-    copy_values(a, ar);
-    calculateDiscreteModel(xr, ar, h);
-    const int r = check && diverged(xr, maxValue) ? 0 : 1;
-    UCB_PRAGMA_(unroll UCB_REDO_UNROLL)
-    for (int i = 1; i < (r ? n : 1); ++i) calculateDiscreteModel(xr, ar, h);
-    copy_state<UCB_NX>(xr, x);
-    return r;
-}
-__device__ __noinline__ int redo_pair(numb* xy, const numb* a, numb h, int n, numb maxValue) {
-    numb xr[UCB_NX], yr[UCB_NX], ar[UCB_NV];
-    copy_state<UCB_NX>(xy, xr);
-    copy_state<UCB_NX>(xy + UCB_NX, yr);
-    copy_values(a, ar);
-    calculateDiscreteModel(xr, ar, h);
-    calculateDiscreteModel(yr, ar, h);
-    const int r = diverged(xr, maxValue) || diverged(yr, maxValue) ? 0 : 1;
-    UCB_PRAGMA_(unroll UCB_REDO_UNROLL)
-    for (int i = 1; i < (r ? n : 1); ++i) {
-        calculateDiscreteModel(xr, ar, h);
-        calculateDiscreteModel(yr, ar, h);
-    }
-    copy_state<UCB_NX>(xr, xy);
-    copy_state<UCB_NX>(yr, xy + UCB_NX);
-    return r;
-}
-
 template <bool Check>
 __device__ __forceinline__ int run_single(const Stepper& s, numb* x, const numb* a, numb h, int n, numb maxValue) {
     numb keep[UCB_NX];
@@ -609,7 +584,7 @@ __device__ __forceinline__ int run_single(const Stepper& s, numb* x, const numb*
     if (s.failed()) {
         numb av[UCB_NV];
         copy_values(a, av);
-        r = redo_single(keep, av, h, n, maxValue, Check);
+        r = redo_single<Check>(keep, av, h, n, maxValue);
         copy_state<UCB_NX>(keep, x);
     }
     return r;
@@ -622,18 +597,18 @@ __device__ __forceinline__ int run_nt(const Stepper& s, numb* x, const numb* a, 
     if (s.failed()) {
         numb av[UCB_NV];
         copy_values(a, av);
-        r = redo_single(keep, av, h, UCB_NT + UCB_EXTRA_STEP, maxValue, true);
+        r = redo_single<true>(keep, av, h, UCB_NT + UCB_EXTRA_STEP, maxValue);
         copy_state<UCB_NX>(keep, x);
     }
     return r;
 }
 #endif
 __device__ __forceinline__ int finish_pair(const Stepper& s, int r, numb* keep, numb* x, numb* y, const numb* a,
-                                           numb h, int n, numb maxValue) {
+                                           numb h, int n, numb maxValue, bool whole_nt) {
     if (s.failed()) {
         numb av[UCB_NV];
         copy_values(a, av);
-        r = redo_pair(keep, av, h, n, maxValue);
+        r = redo_pair(keep, av, h, n, maxValue, whole_nt);
         copy_state<UCB_NX>(keep, x);
         copy_state<UCB_NX>(keep + UCB_NX, y);
     }
@@ -645,7 +620,7 @@ __device__ __forceinline__ int run_pair(const Stepper& s, numb* x, numb* y, cons
     copy_state<UCB_NX>(x, keep);
     copy_state<UCB_NX>(y, keep + UCB_NX);
     const int r = s.verbatim ? 0 : block_pair(s, x, y, a, h, n, maxValue);
-    return finish_pair(s, r, keep, x, y, a, h, n, maxValue);
+    return finish_pair(s, r, keep, x, y, a, h, n, maxValue, false);
 }
 #ifdef UCB_NT
 __device__ __forceinline__ int run_pair_nt(const Stepper& s, numb* x, numb* y, const numb* a, numb h, numb maxValue) {
@@ -653,7 +628,7 @@ __device__ __forceinline__ int run_pair_nt(const Stepper& s, numb* x, numb* y, c
     copy_state<UCB_NX>(x, keep);
     copy_state<UCB_NX>(y, keep + UCB_NX);
     const int r = s.verbatim ? 0 : block_pair_nt(s, x, y, a, h, maxValue);
-    return finish_pair(s, r, keep, x, y, a, h, UCB_NT + UCB_EXTRA_STEP, maxValue);
+    return finish_pair(s, r, keep, x, y, a, h, UCB_NT, maxValue, true);
 }
 #endif
 #else
