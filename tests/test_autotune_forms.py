@@ -1,8 +1,8 @@
 """The shape search of a shadow map looks at the kernel that a map of its size runs: a trajectory a
 lane (ucb_lle_split_kernel) while few cells leave schedulers idle, else the pair form; each has
 its own shapes. A build prepared at one size still serves every other."""
+import ctypes as C
 import os
-import re
 import subprocess
 import sys
 from pathlib import Path
@@ -28,14 +28,22 @@ ucb.precompile(engine_request(ucb, lle2d_case(n=8, t_max=1.0, transient=1.0), pr
 
 
 def compiled_registers(rep, cache):
-    """Registers of each kernel of the build in the reported shape, by the compiler's own report."""
+    """Registers of both kernels of the build in the reported shape, of a file compiled for it alone."""
     code = REGISTERS.format(pkg=str(ROOT / "u-cuda_b200"), tests=str(ROOT / "tests"))
-    env = dict(os.environ, UCB_PTXAS_VERBOSE="1", UCB_CUBIN_CACHE=str(cache))
+    env = dict(os.environ, UCB_CUBIN_CACHE=str(cache))
     r = subprocess.run([sys.executable, "-c", code, *(str(rep[k]) for k in ("block_threads", "max_registers", "unroll"))],
                        env=env, capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, r.stderr[-2000:]
-    found = re.findall(r"entry function '(\w+)'.*?Used (\d+) registers", r.stderr, re.S)
-    return {name: int(n) for name, n in found}
+    (cubin,) = cache.iterdir()
+    cuda = C.CDLL("libcuda.so.1")  # (the engine's context is current)
+    module, function, value, out = C.c_void_p(), C.c_void_p(), C.c_int(), {}
+    assert cuda.cuModuleLoad(C.byref(module), str(cubin).encode()) == 0
+    for name in ("ucb_lle_kernel", "ucb_lle_split_kernel"):
+        assert cuda.cuModuleGetFunction(C.byref(function), module, name.encode()) == 0
+        assert cuda.cuFuncGetAttribute(C.byref(value), 4, function) == 0  # CU_FUNC_ATTRIBUTE_NUM_REGS
+        out[name] = value.value
+    assert cuda.cuModuleUnload(module) == 0
+    return out
 
 
 def test_each_form_is_tuned_by_its_own_kernel(tmp_path, monkeypatch):
