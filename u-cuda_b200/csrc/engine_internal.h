@@ -34,7 +34,7 @@ struct TuneConfig {
 struct ucb_run_control {
     volatile int32_t cancel;
     int32_t pad;
-    volatile unsigned long long fetched;  // written by those builds
+    volatile unsigned long long fetched;  // written by those builds; nothing reads it
     unsigned long long position;          // read back from the work counter
 };
 

@@ -878,7 +878,7 @@ __device__ __forceinline__ void warp_add_steps(unsigned long long* counter, long
 struct UcbControl {
     int cancel;
     int pad;
-    unsigned long long fetched;  // (in mapped host memory only)
+    unsigned long long fetched;  // written by UCB_MAPPED_CONTROL builds (warp_fetch), read by nothing
 };
 
 }  // namespace ucbdev

@@ -931,15 +931,6 @@ __device__ __forceinline__ void ls_cell_dp5(const UcbLsParams& p, long long kidx
 }
 
 #if defined(UCB_LS_GROUP)
-// ls_cell_dp5 with a cell on UCB_NX lanes, one tangent vector each (the same values and order of
-// operations): every lane of a group takes the state's step and its own vector's, the error
-// sums and Gram-Schmidt rows are exchanged by shuffles. An attempt is then two chains of
-// stages instead of N + 1 and its registers fall from 254 to 204 (FP64), so a map of few cells,
-// which lasts as long as its slowest ones, ends sooner; a group takes its next cell as soon as
-// it is done. The exchanges are taken by the whole warp; what a group does between them
-// depends on values that all its lanes hold. (The tangent's stages beside the state's, before
-// its step is accepted, gave the same times.) B200, 96^2 hyper-chaotic Rossler, t_end 50, FP64:
-// 68 -> 46 ms; where each form runs and its times: ls_groups of ucb_ls.cpp.
 // mgs() over the group's rows (lane k holds row k), for groups with `act`; the log of the
 // norms added to acc. False if the group's rows are not independent and finite.
 __device__ __forceinline__ bool group_mgs(numb* v, double& acc, bool act, int k, int base, unsigned int group) {
@@ -975,6 +966,15 @@ __device__ __forceinline__ bool group_mgs(numb* v, double& acc, bool act, int k,
     return (ok & group) == group;
 }
 
+// ls_cell_dp5 with a cell on UCB_NX lanes, one tangent vector each (the same values and order of
+// operations): every lane of a group takes the state's step and its own vector's, the error
+// sums and Gram-Schmidt rows are exchanged by shuffles. An attempt is then two chains of
+// stages instead of N + 1 and its registers fall from 254 to 204 (FP64), so a map of few cells,
+// which lasts as long as its slowest ones, ends sooner; a group takes its next cell as soon as
+// it is done. The exchanges are taken by the whole warp; what a group does between them
+// depends on values that all its lanes hold. (The tangent's stages beside the state's, before
+// its step is accepted, gave the same times.) B200, 96^2 hyper-chaotic Rossler, t_end 50, FP64:
+// 68 -> 46 ms; where each form runs and its times: ls_groups of ucb_ls.cpp.
 __device__ __forceinline__ void ls_groups_dp5(const UcbLsParams& p, long long& ns) {
     const unsigned int full = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
