@@ -129,7 +129,7 @@ struct VerbatimStepper {
 // The body with its division by six replaced (ucb_exact.cuh). The bits are the division's
 // while `range` stays within kSixthRange; run_single / run_pair / run_probes and the
 // sampling of ucb_bif.cuh take a block of steps again with the division otherwise, and the
-// trajectory's later blocks with it from the start, as those of its warp (meet).
+// trajectory's later blocks with it from the start, in FP32 as those of its warp (meet).
 struct Stepper {
     mutable unsigned int range;
     mutable bool verbatim;
@@ -146,15 +146,18 @@ struct Stepper {
 };
 // A lane whose blocks are taken with the division has the lanes that step with it take theirs
 // so too (the same bits), or they would wait for its pass after their own: loops ask at intervals of
-// about a hundred steps. Forms with a trajectory a lane do not ask: both passes of one trajectory
-// are still less than the division for several, and the vote costs them up to 4 % (others 0-2 %).
-// B200, exact FP32 Lorenz maps some of whose cells settle on the origin, the division everywhere /
-// the settled lanes alone / the warp together: exponent 256^2 (60,000 steps a cell) 51 / 60 / 50 ms,
-// diagram of 1,024 values (30,000) 32.0 / 36.1 / 31.7, period map 128^2 29.5 / 30.8 / 28.3, spectrum 256^2
-// (52,000) 45 / 53 / 45; no cell settling: 28.4 / 20.9 / 20.9, 9.5 / 4.9 / 4.9, 27.8 / 9.3 / 9.1, 27.2 / 22.3 /
-// 22.2; FP64, none settling: 31.4 / 20.6 / 20.6, 11.0 / 3.42 / 3.45, 29.5 / 5.62 / 5.69, 31.7 / 22.7 / 23.0. A
-// trajectory a lane, 64^2: 34.2 / 31.1 / (not asking).
+// about a hundred steps. B200, exact FP32 Lorenz maps some of whose cells settle on the origin, the
+// division everywhere / the settled lanes alone / the warp together: exponent 256^2 (60,000 steps a
+// cell) 51 / 60 / 50 ms, diagram of 1,024 values (30,000) 32.0 / 36.1 / 31.7, period map 128^2 29.5 / 30.8 /
+// 28.3, spectrum 256^2 (52,000) 45 / 53 / 45; no cell settling: 28.4 / 20.9 / 20.9, 9.5 / 4.9 / 4.9, 27.8 / 9.3 /
+// 9.1, 27.2 / 22.3 / 22.2.
+// Not in FP64, where the block without the division is so much cheaper that both passes take no
+// longer than the division everywhere did (the same maps from 1e-286: 31.8 / 29.4 / 29.5, 15.3 / 13.3 /
+// 13.6, 15.8 / 14.2 / 14.3, 50.5 / 51.2 / 50.8) and the vote costs maps without such cells 1-3 %; nor in the forms
+// with a trajectory a lane, whose both passes are less than the division for several.
+#ifdef UCB_NUMB_F32
 __device__ __forceinline__ void meet(const Stepper& s) { s.verbatim = __any_sync(__activemask(), s.verbatim); }
+#endif
 #else
 struct Stepper : VerbatimStepper {
     __device__ __forceinline__ explicit Stepper(numb) {}
@@ -483,7 +486,7 @@ __device__ __forceinline__ bool diverged2(const float2* x, float maxValue, int c
 // then one extra step and the fixed-point test. 1 ok / -1 fixed point / 0 diverged.
 // ---------------------------------------------------------------------------
 template <class S>
-__device__ __forceinline__ void meet(const S&) {}  // (steps that are never taken again)
+__device__ __forceinline__ void meet(const S&) {}  // (the others)
 
 // `n` steps of x; with Check the divergence test after the first of them. 0: diverged there.
 template <bool Check, class S>
