@@ -160,6 +160,8 @@ bool tune_request(ucb_engine* e, const ucb_options& o, int default_block, Compil
                   std::string& err) {
     if (!resolve_tuning(e, o, tune_key(rq), default_block, out, err)) return false;
     apply_tuning(rq, out);
+    // a caller's one, where the build would unroll by more by itself
+    if (o.unroll == 1) rq.source = "#define UCB_UNROLL_ONE 1\n" + rq.source;
     return true;
 }
 
@@ -194,8 +196,8 @@ int autotune_search(ucb_engine* e, const std::string& key, int default_block, bo
         rep->wall_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
         return UCB_OK;
     }
-    // trials pass every knob explicitly, but a register cap of 0 ("compiler's choice")
-    // would pick a stored cap up again: forget the stored shape while searching
+    // trials pass every knob explicitly, but a register cap of 0 ("compiler's choice") and an unroll of
+    // 1 (the build's own) would pick stored ones up again: forget the stored shape while searching
     e->tuned.erase(key);
     // one run to compile / load, then the better of two
     auto measure = [&](const TuneConfig& c) -> double {

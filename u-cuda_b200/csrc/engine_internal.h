@@ -18,7 +18,8 @@
 
 namespace ucb {
 // Launch shape of a kernel build (see ucb_options): threads per block, registers per
-// thread cap (0 = compiler's choice), steps per unrolled chunk of the step loops.
+// thread cap (0 = compiler's choice), steps per unrolled chunk of the step loops (1: the build's
+// own choice, which for some loops is more).
 struct TuneConfig {
     int block = 128;
     int maxreg = 0;

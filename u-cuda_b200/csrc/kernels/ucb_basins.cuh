@@ -23,7 +23,7 @@
 
 // Steps of the table loop unrolled, so that the next steps' loads run ahead of this one's chain
 // (forced Duffing 512^2, cap 1,000, 1 / 4 / 8 steps: FP64 79.4 / 74.9 / 72.6 ms).
-#if UCB_UNROLL > 1 || defined(UCB_ONE_SLICE)
+#if UCB_UNROLL > 1 || defined(UCB_UNROLL_ONE) || defined(UCB_ONE_SLICE)
 #define UCB_TRIG_UNROLL UCB_UNROLL
 #else
 #define UCB_TRIG_UNROLL 8

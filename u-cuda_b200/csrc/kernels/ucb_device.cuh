@@ -796,7 +796,7 @@ __device__ __forceinline__ void apply_sweep(const CellAxes& c, const numb* ax0, 
 // itself is not advanced (set_phase() gives it), unless the system reads it elsewhere.
 // B200, reference-method Duffing features 256^2, whole calls: FP32 73.1 -> 49.2 ms (350,000
 // steps a cell), FP64 23.9 -> 13.8 ms (47,700 steps a cell); FP64 100^2 14.3 -> 7.7 ms.
-#if UCB_UNROLL > 1
+#if UCB_UNROLL > 1 || defined(UCB_UNROLL_ONE)
 #define UCB_FORCED_UNROLL UCB_UNROLL
 #else
 #define UCB_FORCED_UNROLL 4  // the next steps' loads ahead of this one's chain: 57.2 -> 54.7 ms

@@ -316,7 +316,7 @@ extern "C" int ucb_autotune_bif2d(ucb_engine* e, const ucb_bif2d_request* req, i
         ucb_bif2d_request q = t;
         q.opt.block_threads = c.block;
         q.opt.max_registers = c.maxreg;
-        q.opt.unroll = c.unroll;
+        q.opt.unroll = c.unroll > 1 ? c.unroll : 0;
         return q;
     };
     auto trial = [&](const TuneConfig& c) -> double {

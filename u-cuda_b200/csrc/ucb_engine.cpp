@@ -1217,7 +1217,7 @@ int ucb_autotune_lle2d(ucb_engine* e, const ucb_lle2d_request* req, int32_t forc
         ucb_lle2d_request q = t;
         q.opt.block_threads = c.block;
         q.opt.max_registers = c.maxreg;
-        q.opt.unroll = c.unroll;
+        q.opt.unroll = c.unroll > 1 ? c.unroll : 0;
         return q;
     };
     auto trial = [&](const TuneConfig& c) -> double {
@@ -1259,7 +1259,7 @@ int ucb_autotune_lle2d(ucb_engine* e, const ucb_lle2d_request* req, int32_t forc
         ucb_lle2d_request q = cq;
         q.opt.block_threads = c.block;
         q.opt.max_registers = c.maxreg;
-        q.opt.unroll = c.unroll;
+        q.opt.unroll = c.unroll > 1 ? c.unroll : 0;
         ucb_lle2d_result r{};
         r.values = cvals.data();
         r.flags = cflags.data();

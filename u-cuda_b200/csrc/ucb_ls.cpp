@@ -455,7 +455,7 @@ extern "C" int ucb_autotune_ls2d(ucb_engine* e, const ucb_ls2d_request* req, int
         ucb_ls2d_request q = t;
         q.opt.block_threads = c.block;
         q.opt.max_registers = c.maxreg;
-        q.opt.unroll = c.unroll;
+        q.opt.unroll = c.unroll > 1 ? c.unroll : 0;
         return q;
     };
     auto trial = [&](const TuneConfig& c) -> double {
